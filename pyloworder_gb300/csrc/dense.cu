@@ -19,6 +19,8 @@
 #include <cmath>
 
 #include "plom_common.cuh"
+#include "plom_df.cuh"
+#include "plom_jacobi.cuh"
 #include "plom_kernels.cuh"
 
 namespace cg = cooperative_groups;
@@ -489,18 +491,6 @@ struct JacState {
   const double* V0;  // real, batch 1: starting rotation product (n x n row-major); null = I
 };
 
-__device__ __forceinline__ void rr_pair(int step, int k, int np, int& a, int& b) {
-  // round-robin (circle method) over np (even) players; np-1 steps
-  const int m = np - 1;
-  if (k == 0) {
-    a = 0;
-    b = 1 + (step % m);
-  } else {
-    a = 1 + (step + k) % m;
-    b = 1 + (step - k + m) % m;
-  }
-}
-
 // Rotation of a pair with squared norms al, be and |a_p^H a_q| = gabs.
 // False when the pair is orthogonal to the tolerance (gabs^2 <= tol2 al be).
 __device__ __forceinline__ bool jac_angle(double al, double be, double gabs, double tol2,
@@ -682,39 +672,6 @@ __device__ __forceinline__ int jac_pair(double* x, double* y, double* xv, double
 // error-free transformations (Knuth's two-sum, FMA two-product); the scalar
 // pair parameters stay in FP64.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 df_split(double v) {
-  const float h = (float)v;
-  return make_float2(h, (float)(v - (double)h));
-}
-__device__ __forceinline__ double df_val(float2 a) { return (double)a.x + (double)a.y; }
-__device__ __forceinline__ float2 two_sum(float a, float b) {
-  const float s = a + b;
-  const float bb = s - a;
-  return make_float2(s, (a - (s - bb)) + (b - bb));
-}
-__device__ __forceinline__ float2 fast_two_sum(float a, float b) {
-  const float s = a + b;
-  return make_float2(s, b - (s - a));
-}
-// a - t b
-__device__ __forceinline__ float2 df_fms(float2 a, float2 t, float2 b) {
-  const float ph = t.x * b.x;
-  float pe = fmaf(t.x, b.x, -ph);
-  pe = fmaf(t.x, b.y, pe);
-  pe = fmaf(t.y, b.x, pe);
-  const float2 sm = two_sum(a.x, -ph);
-  return fast_two_sum(sm.x, sm.y + (a.y - pe));
-}
-// acc += x y (acc.y collects the low-order parts)
-__device__ __forceinline__ void df_dot_acc(float2& acc, float2 x, float2 y) {
-  const float ph = x.x * y.x;
-  float pe = fmaf(x.x, y.x, -ph);
-  pe = fmaf(x.x, y.y, pe);
-  pe = fmaf(x.y, y.x, pe);
-  const float2 sm = two_sum(acc.x, ph);
-  acc.x = sm.x;
-  acc.y += sm.y + pe;
-}
 __device__ __forceinline__ double df_warp_sum(float2 v) {
   v = fast_two_sum(v.x, v.y);
 #pragma unroll
@@ -1057,20 +1014,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
-// rounds of the 6 pairs inside a block of 4: (0,1)(2,3) / (0,2)(1,3) / (0,3)(1,2)
-__device__ __forceinline__ void intra_pair(int round, int which, int& a, int& b) {
-  if (round == 0) {
-    a = which ? 2 : 0;
-    b = which ? 3 : 1;
-  } else if (round == 1) {
-    a = which ? 1 : 0;
-    b = which ? 3 : 2;
-  } else {
-    a = which ? 1 : 0;
-    b = which ? 2 : 3;
-  }
-}
-
 constexpr uint64_t JAC_WAIT_NS = 2000000000ull;
 
 template <int CW, bool DF>
@@ -1255,29 +1198,6 @@ __global__ void __launch_bounds__(128) jacobi_block_kernel(const double* __restr
 //   c = (1 + t^2)^-1/2 from an FP32 estimate and one Newton step in
 //   double-float, scales d, 1/d, carried norms and t dq/dp in double-float.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 df_mul(float2 a, float2 b) {
-  const float p = a.x * b.x;
-  float e = fmaf(a.x, b.x, -p);
-  e = fmaf(a.x, b.y, e);
-  e = fmaf(a.y, b.x, e);
-  return fast_two_sum(p, e);
-}
-__device__ __forceinline__ float2 df_add2(float2 a, float2 b) {
-  const float2 s = two_sum(a.x, b.x);
-  return fast_two_sum(s.x, s.y + (a.y + b.y));
-}
-__device__ __forceinline__ float2 df_mulf(float2 a, float t) {
-  const float p = a.x * t;
-  const float e = fmaf(a.x, t, -p);
-  return fast_two_sum(p, fmaf(a.y, t, e));
-}
-// 1 / d in double-float
-__device__ __forceinline__ float2 df_recip(float2 d) {
-  const float h = 1.0f / d.x;
-  const float r = fmaf(-d.x, h, 1.0f) - d.y * h;
-  return fast_two_sum(h, r * h);
-}
-
 struct DfPair {
   float2 tp, tqn;  // x -= tp y ; y -= tqn x
   int rot;
@@ -2731,7 +2651,10 @@ static int jacobi_pre32(const double* A, const double* At, int n, double tol, do
     return PLOM_OK;
   }
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
-  {
+  if (jacobi_cta_f32_usable(n)) {
+    PLOM_TRY(jacobi_cta_f32(A, n, 1, JAC_PRE32_TOL, JAC_PRE32_MAX_SWEEPS, JAC_PRE32_FLOOR,
+                            JAC_PRE32_TSTOP, J32, j32.amax, info, st));
+  } else {
     const void* k = (const void*)jacobi_block_f32_kernel;
     const size_t smem = (size_t)4 * J32B * j32.pitch * sizeof(float);
     PLOM_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2785,7 +2708,9 @@ static int jacobi_svd_transposed(const double* A, int n, double tol, double* S, 
     return pre32 ? jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st) : PLOM_OK;
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
   PLOM_REQUIRE(A && S && U && VH && info, PLOM_ERR_ARG, "jacobi: null pointer");
-  PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
+  if (!pre32 && tol >= JAC_DF_TOL && jacobi_cta_usable(n, 0))
+    return jacobi_cta(A, n, 1, 0, 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U, VH, info, st);
+  if (!pre32 || !jacobi_cta_f32_usable(n)) PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
   if (pre32)
     PLOM_TRY(jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st));
   else
@@ -2805,6 +2730,9 @@ int jacobi_svd(const double* A, int n, int batch, int cplx, double tol, double* 
   if (ws.measuring() || n == 0 || batch == 0) return PLOM_OK;
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
   PLOM_REQUIRE(A && S && U && VH && info, PLOM_ERR_ARG, "jacobi: null pointer");
+  if (tol >= JAC_DF_TOL && jacobi_cta_usable(n, cplx))
+    return jacobi_cta(A, n, batch, cplx, cplx ? 0 : 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U,
+                      VH, info, st);
   return jacobi_launch(A, n, batch, cplx, js, tol, S, U, VH, info, st);
 }
 

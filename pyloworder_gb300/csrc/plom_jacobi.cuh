@@ -1,0 +1,22 @@
+// One-sided Jacobi in shared memory (jacobi_cta.cu): interfaces for dense.cu.
+#pragma once
+#include "plom_common.cuh"
+
+namespace plom {
+
+// Whether n columns (per problem) fit the double-float form and its clusters
+// can be resident on this device.
+bool jacobi_cta_usable(int n, int cplx);
+// SVD of `batch` n x n matrices on double-float rows (tol >= 1e-10): S, U, VH as
+// jacobi_svd gives them.  trans (real): the rows of A are rotated instead of
+// its columns.  At, Vt: batch x n x n (complex: 2n) FP64 scratch, nrm2: batch x n.
+int jacobi_cta(const double* A, int n, int batch, int cplx, int trans, double tol, double* At,
+               double* Vt, double* nrm2, unsigned long long* amax, double* S, double* U,
+               double* VH, int* info, cudaStream_t st);
+// FP32 sweeps of one real matrix: the rotation product J (n x n row-major) and
+// the bits of max |a|.
+bool jacobi_cta_f32_usable(int n);
+int jacobi_cta_f32(const double* A, int n, int trans, float tol, int max_sweeps, float floor_rel,
+                   float tstop, float* J, unsigned long long* amax, int* info, cudaStream_t st);
+
+}  // namespace plom

@@ -1,0 +1,63 @@
+"""The n x n SVD in shared memory at the edges of its plans (lanes per pair,
+columns per CTA, cluster sizes), through the public SVD entry points.
+
+Tolerance 1e-5: the mixed form's stated one for singular values, orthonormality
+and reconstruction (the input's condition number is 100, so every mode is a
+retained one)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def field(m, n, seed, cplx=False):
+    rng = np.random.default_rng(seed)
+    dt = np.complex128 if cplx else np.float64
+    def ortho(r, c):
+        a = rng.standard_normal((r, c)) + (1j * rng.standard_normal((r, c)) if cplx else 0)
+        return np.linalg.qr(a)[0].astype(dt)
+    s = 100.0 ** (-np.arange(n) / max(1, n - 1))
+    return (ortho(m, n) * s) @ ortho(n, n).conj().T
+
+
+def check(A, U, S, V):
+    n = A.shape[1]
+    ex = np.linalg.svd(A, compute_uv=False)
+    assert np.max(np.abs(S - ex) / ex) < TOL
+    eye = np.eye(n)
+    assert np.max(np.abs(V @ V.conj().T - eye)) < TOL
+    assert np.max(np.abs(U.conj().T @ U - eye)) < 2 * TOL
+    assert np.linalg.norm((U * S) @ V - A) < TOL * np.linalg.norm(A)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 16, 17, 32, 33, 48, 49, 64, 65, 96, 97, 128, 129, 192, 193,
+                               255, 256, 257, 384, 385, 512, 513])
+def test_real(n):
+    import pyloworder_gb300 as P
+    A = field(2 * n + 130, n, n).astype(np.float32)
+    U, S, V = P.math.tsqr_svd(A)
+    check(A.astype(np.float64), *(x.astype(np.float64) for x in (U, S, V)))
+
+
+@pytest.mark.parametrize("n", [1, 2, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 80, 81])
+def test_complex_batch(n):
+    import pyloworder_gb300 as P
+    A = np.stack([field(2 * n + 130, n, 1000 + n + b, True) for b in range(3)]).astype(np.complex64)
+    U, S, V = P.vmmath.tsqr_svd_batched_device(torch.from_numpy(A).cuda())
+    for b in range(3):
+        check(A[b].astype(np.complex128), U[b].cpu().numpy().astype(np.complex128),
+              S[b].double().cpu().numpy(), V[b].cpu().numpy().astype(np.complex128))
+
+
+@pytest.mark.parametrize("n", [5, 64, 100, 200])
+def test_real_batch(n):
+    import pyloworder_gb300 as P
+    A = np.stack([field(2 * n + 130, n, 2000 + n + b) for b in range(3)]).astype(np.float32)
+    U, S, V = P.vmmath.tsqr_svd_batched_device(torch.from_numpy(A).cuda())
+    for b in range(3):
+        check(A[b].astype(np.float64), U[b].double().cpu().numpy(), S[b].double().cpu().numpy(),
+              V[b].double().cpu().numpy())
