@@ -243,10 +243,7 @@ static int chol_pass_packed(bool cplx, int n, const Packed& P, PackedCore& b, do
   if (cplx && !ws.measuring()) PLOM_TRY(complexify_gram(b.H, b.G, n, 1, st));
   // the Gram of a factor next to orthonormal is factored in closed form when
   // the implied perturbation of G is below 1e-10 (the operands carry 22 bits)
-  PLOM_TRY(chol_shifted(b.G, R, N, 1, rel0, relfail, info, ws, st, rel0 == 0.0 ? 1e-10 : 0.0));
-  need = std::max(need, ws.off);
-  ws.off = mark;
-  PLOM_TRY(trtri_upper(R, W, N, 1, ws, st));
+  PLOM_TRY(chol_inverse_df(b.G, R, W, N, 1, rel0, relfail, info, ws, st, rel0 == 0.0 ? 1e-10 : 0.0));
   need = std::max(need, ws.off);
   ws.off = need;
   return PLOM_OK;
@@ -376,8 +373,7 @@ static int cholqr3_packed_chunked(const float* X, int64_t m, int n, int64_t ldx,
   PLOM_TRY(sub([&] {
     return gram_packed_chunks(b.P0, C, mc, xscale, b.G, meas ? nullptr : ev.packed, info, ws, st);
   }));
-  PLOM_TRY(sub([&] { return chol_shifted(b.G, b.R1, N, 1, rel1, relfail, info, ws, st); }));
-  PLOM_TRY(sub([&] { return trtri_upper(b.R1, b.W1, N, 1, ws, st); }));
+  PLOM_TRY(sub([&] { return chol_inverse_df(b.G, b.R1, b.W1, N, 1, rel1, relfail, info, ws, st); }));
   Packed P0b = b.P0, P1b = b.P1;
   P0b.batch = P1b.batch = C;
   P0b.m = P1b.m = mc;
@@ -555,8 +551,7 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
   auto pass = [&](const Packed& P, double* R, double* W, double rel0) -> int {
     PLOM_TRY(sub([&] { return gram_packed(P, cplx ? H : G, info, ws, st); }));
     if (cplx && !meas) PLOM_TRY(complexify_gram(H, G, n, bi, st));
-    PLOM_TRY(sub([&] { return chol_shifted(G, R, N, bi, rel0, relfail, info, ws, st); }));
-    return sub([&] { return trtri_upper(R, W, N, bi, ws, st); });
+    return sub([&] { return chol_inverse_df(G, R, W, N, bi, rel0, relfail, info, ws, st); });
   };
   auto rowform_b = [&](const double* W) -> const double* {
     if (!cplx || meas) return W;
@@ -1172,8 +1167,7 @@ static int tsqr_svd_host_mixed(const float* Xh, int64_t m, int n, int64_t ldx, f
     if (!meas) PLOM_CHECK_CUDA(cudaEventRecord(ev.freed[slot], st));
     PLOM_TRY(sub([&] { return gram_packed(v, b.G, info, ws, st, c > 0); }));
   }
-  PLOM_TRY(sub([&] { return chol_shifted(b.G, b.R1, N, 1, rel1, relfail, info, ws, st); }));
-  PLOM_TRY(sub([&] { return trtri_upper(b.R1, b.W1, N, 1, ws, st); }));
+  PLOM_TRY(sub([&] { return chol_inverse_df(b.G, b.R1, b.W1, N, 1, rel1, relfail, info, ws, st); }));
   // Q1 = X R1^-1 with the chunks as a batch: one W, each chunk's input scales
   Packed P0b = b.P0, P1b = b.P1;
   P0b.batch = P1b.batch = pl.C;
