@@ -14,10 +14,12 @@
 //  * the elimination runs on [G + s I | I]: step k's trailing update subtracts
 //    R_ka^T [R_kc | Z_kq], and the right half ends as Z = R^-T, so the inverse
 //    needs no pass and no barrier of its own;
-//  * a diagonal block is eliminated with one CTA barrier per column: every
-//    thread keeps 8 rows of one of the 64 columns of [S | P] in registers, the
-//    pivot row goes round through shared memory unscaled, and each thread derives
-//    the pivot's reciprocal itself.
+//  * a diagonal block is eliminated in panels of 8 rows of [S | P]: one warp takes
+//    a panel through its 8 pivots in registers (shuffles only), then the CTA
+//    subtracts its rank-8 update from the rows below, two barriers a panel
+//    (26,200 cycles a block with a barrier per pivot, 10,000 with panels);
+//  * FP64 <-> double-float conversions and power-of-two scalings are integer
+//    operations on the bits: an FP64 instruction issues at 2 lanes a clock and SM.
 // Blocks are 32 x 32.  One problem of more than 64 columns takes one cooperative
 // launch (two grid barriers a block step: panel, trailing update with the next
 // diagonal block); batches and small problems take one CTA per problem and CTA
@@ -45,15 +47,58 @@ struct CholDf {
   double *R, *W;
   float2 *Rs, *Zs;   // batch x np x np: scaled [R | Z]
   float2* Dt;        // batch x 32 x 32: R_kk^-1 of the current block step
-  float* d;          // batch x np: powers of two
-  double *trace, *shift;
+  int* d;            // batch x np: the scales are 2^-d
+  double *shift, *base;  // of the problem: s, and the least s after a breakdown
   int *status;       // 0 pending, 1 done, 2 failed in this round, 3 bad input
   int *pending, *used;
-  double* colsq;     // near-identity test (batch 1)
+  float* colsq;      // near-identity test (batch 1)
   int* info;
   int n, np, batch, solo;
-  double rel0, relfail, near_tol;
+  double rel0_n, relfail_n;  // shift and breakdown floor relative to the trace
+  float near_tol;
 };
+
+// v 2^s as a double-float number (0 below the FP32 range, inf above), on the
+// integer pipe
+__device__ __forceinline__ float2 cd_split(double v, int s) {
+  const uint64_t b = (uint64_t)__double_as_longlong(v);
+  const int e = (int)(b >> 52) & 0x7ff;
+  const uint32_t sign = (uint32_t)(b >> 32) & 0x80000000u;
+  if (e == 0x7ff) return make_float2((float)v, 0.f);
+  const int ex = e - 896 + s;  // FP32 exponent of the top 24 bits
+  if (e == 0 || ex <= 0) return make_float2(0.f, 0.f);
+  if (ex >= 255) return make_float2(__uint_as_float(0x7f800000u | sign), 0.f);
+  const uint32_t top = (uint32_t)(b >> 29) & 0x7fffffu, low = (uint32_t)b & 0x1fffffffu;
+  const float hi = __uint_as_float(sign | ((uint32_t)ex << 23) | top);
+  const int k = ex - 52;  // biased exponent of the low bits' unit, 2^(ex - 179)
+  const float unit = __uint_as_float(sign | ((uint32_t)(k > 0 ? k : 0) << 23));
+  return fast_two_sum(hi, (float)low * unit);
+}
+// the double-float number v times 2^s in FP64, on the integer pipe
+__device__ __forceinline__ double cd_join(float2 v, int s) {
+  v = fast_two_sum(v.x, v.y);
+  const uint32_t hb = __float_as_uint(v.x);
+  const int eh = (int)(hb >> 23) & 255;
+  if (eh == 255) return (double)v.x;
+  if (eh == 0) return 0.0;
+  // v.y in units of 2^(eh - 179), at most 2^28 of them
+  const int up = 179 - eh, u1 = up / 2, u2 = up - u1;
+  float l = v.y * __uint_as_float((uint32_t)(127 + u1) << 23) * __uint_as_float((uint32_t)(127 + u2) << 23);
+  if (hb & 0x80000000u) l = -l;
+  long long m = ((long long)((hb & 0x7fffffu) | 0x800000u) << 29) + (long long)__float2int_rn(l);
+  int e = eh + 896 + s;
+  if (m < (1ll << 52)) {
+    m <<= 1;
+    e -= 1;
+  } else if (m >= (1ll << 53)) {
+    m >>= 1;
+    e += 1;
+  }
+  const uint64_t sg = (uint64_t)(hb & 0x80000000u) << 32;
+  if (e <= 0) return 0.0;
+  if (e >= 0x7ff) return __longlong_as_double((long long)(sg | 0x7ff0000000000000ull));
+  return __longlong_as_double((long long)(sg | ((uint64_t)e << 52) | ((uint64_t)m & 0xfffffffffffffull)));
+}
 
 // 32 x 32 tile of a float2 matrix (ld np), 2 x 16 bytes a thread
 __device__ __forceinline__ void cd_load(const float2* M, int ld, int bi, int bj, float4 (&v)[2]) {
@@ -92,10 +137,8 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
   cg::grid_group grid = cg::this_grid();
   __shared__ __align__(16) float2 A[CB][CPITCH];
   __shared__ __align__(16) float2 B[CB][CPITCH];
-  __shared__ __align__(16) float2 row_sh[2][2 * CB];
-  __shared__ float2 piv_sh[CB];
   __shared__ double red[8];
-  __shared__ int flag_sh;
+  __shared__ int bad_sh;
   const int tid = threadIdx.x, n = p.n, np = p.np, T = np / CB;
   const int64_t nn = (int64_t)n * n, pp = (int64_t)np * np;
   // problems and tasks of this CTA: in solo mode its own problem's, else all
@@ -118,14 +161,14 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
     if (tid == 0) {
       double t = 0.0;
       for (int w = 0; w < CD_THREADS / 32; ++w) t += red[w];
-      p.trace[b] = t;
-      p.shift[b] = p.rel0 * t / n;
+      p.base[b] = p.relfail_n * t;
+      p.shift[b] = p.rel0_n * t;
       p.status[b] = (isfinite(t) && t > 0.0) ? 0 : 3;
     }
     __syncthreads();
   }
   if (!p.solo && blockIdx.x == 0 && tid < CD_ROUNDS) p.pending[tid] = 0;
-  if (p.near_tol > 0.0 && p.batch == 1 && p.rel0 == 0.0) {
+  if (p.near_tol > 0.f) {
     // G = I + E with X = triu(E, 1) + diag(E) / 2 and every ||X e_j||^2 <= near_tol:
     // R = I + X is the factor of G + X^T X, and R^-1 = I - X + X^2 up to X^3
     const int rows_g = (n + CD_NEAR_GROUPS - 1) / CD_NEAR_GROUPS;
@@ -133,29 +176,30 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
     for (int task = t0; task < cblocks * CD_NEAR_GROUPS; task += ts) {
       const int g = task / cblocks, j = (task % cblocks) * CD_THREADS + tid;
       if (j >= n) continue;
-      float2 acc = make_float2(0.f, 0.f);
+      float acc = 0.f;
       const int i1 = min(min(n, (g + 1) * rows_g), j + 1);
+#pragma unroll 4
       for (int i = g * rows_g; i < i1; ++i) {
         const double e = p.G[(int64_t)i * n + j];
-        const float2 x = df_split(i == j ? 0.5 * (e - 1.0) : e);
-        df_dot_acc(acc, x, x);
+        const float x = i == j ? 0.5f * (float)(e - 1.0) : (float)e;
+        acc = fmaf(x, x, acc);
       }
-      p.colsq[(int64_t)g * n + j] = df_val(acc);
+      p.colsq[(int64_t)g * n + j] = acc;
     }
     barrier();
     int ok = 1;
     for (int j = tid; j < n; j += CD_THREADS) {
-      double c = 0.0;
+      float c = 0.f;
       for (int g = 0; g < CD_NEAR_GROUPS; ++g) c += p.colsq[(int64_t)g * n + j];
       if (!(c <= p.near_tol)) ok = 0;  // (a NaN fails the test)
     }
     if (__syncthreads_and(ok) && p.status[0] == 0) {
       float(*X1)[CB + 1] = reinterpret_cast<float(*)[CB + 1]>(&A[0][0]);
       float(*X2)[CB + 1] = reinterpret_cast<float(*)[CB + 1]>(&B[0][0]);
-      auto xat = [&](int i, int j) -> double {
-        if (i >= n || j >= n || i > j) return 0.0;
+      auto xat = [&](int i, int j) -> float {
+        if (i >= n || j >= n || i > j) return 0.f;
         const double g = p.G[(int64_t)i * n + j];
-        return i == j ? 0.5 * (g - 1.0) : g;
+        return i == j ? 0.5f * (float)(g - 1.0) : (float)g;
       };
       for (int t = t0; t < T * T; t += ts) {
         const int a = t / T, c = t % T;
@@ -163,8 +207,8 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
         for (int k = a; k <= c; ++k) {  // (X^2)_ac
           __syncthreads();
           for (int e = tid; e < CB * CB; e += CD_THREADS) {
-            X1[e >> 5][e & 31] = (float)xat(a * CB + (e >> 5), k * CB + (e & 31));
-            X2[e >> 5][e & 31] = (float)xat(k * CB + (e >> 5), c * CB + (e & 31));
+            X1[e >> 5][e & 31] = xat(a * CB + (e >> 5), k * CB + (e & 31));
+            X2[e >> 5][e & 31] = xat(k * CB + (e >> 5), c * CB + (e & 31));
           }
           __syncthreads();
           for (int q = 0; q < CB; ++q) {
@@ -177,9 +221,18 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
         for (int u = 0; u < 4; ++u) {
           const int i = a * CB + (tid >> 5) + 8 * u, j = c * CB + (tid & 31);
           if (i >= n || j >= n) continue;
-          const double x = xat(i, j), one = i == j ? 1.0 : 0.0;
-          p.R[(int64_t)i * n + j] = one + x;
-          p.W[(int64_t)i * n + j] = i <= j ? one - x + (double)acc[u] : 0.0;
+          const double g = i <= j ? p.G[(int64_t)i * n + j] : 0.0;
+          double r = g, w = 0.0;
+          if (i == j) {
+            const double x = 0.5 * (g - 1.0);
+            r = 1.0 + x;
+            w = 1.0 - x + (double)acc[u];
+          } else if (i < j) {
+            const float2 x = cd_split(g, 0);
+            w = cd_join(df_add2(make_float2(-x.x, -x.y), make_float2(acc[u], 0.f)), 0);
+          }
+          p.R[(int64_t)i * n + j] = r;
+          p.W[(int64_t)i * n + j] = w;
         }
       }
       if (blockIdx.x == 0 && tid == 0) atomicAdd(&p.info[ST_NEAR], 1);
@@ -188,104 +241,126 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
   }
   barrier();
 
-  // ---- diagonal block of step k: [S | P] with S = R_kk (symmetric, upper part
-  // valid) and P = I; eliminated to [R_kk | R_kk^-T]
+  // ---- diagonal block of step k: [S | P] with S = R_kk (symmetric, both
+  // triangles) and P = I; eliminated to [R_kk | R_kk^-T]
   auto diag_block = [&](int b, int k) {
     if (p.status[b] != 0) return;
     float2* Rb = p.Rs + b * pp;
-    const float* db = p.d + (int64_t)b * np;
-    const int c = tid & 63, g = tid >> 6;  // column of [S | P], rows g, g + 4, ...
-    const bool isS = c < CB;
+    float2* Zb = p.Zs + b * pp;
     const int64_t dg = (int64_t)k * CB;
-    float2 v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int a = g + 4 * i;
-      v[i] = isS ? Rb[(dg + a) * np + dg + c] : make_float2(a == c - CB ? 1.f : 0.f, 0.f);
+    {
+      float4 v[2];
+      cd_load(Rb, np, k, k, v);
+      cd_stage(A, v);
+      for (int e = tid; e < CB * CB; e += CD_THREADS)
+        B[e >> 5][e & 31] = make_float2((e >> 5) == (e & 31) ? 1.f : 0.f, 0.f);
+      if (tid == 0) bad_sh = 0;
     }
-    const double floor_piv = p.rel0 == 0.0 ? p.relfail * p.trace[b] / n : 0.0;
-    if (g == 0) row_sh[0][c] = v[0];
     __syncthreads();
-    bool ok = true;
-    for (int j = 0; j < CB; ++j) {
-      const float2* rw = row_sh[j & 1];
-      float2 d = rw[j];
-      bool good = d.x > 0.f && isfinite(d.x);
-      if (!good && p.rel0 == 0.0 && isfinite(d.x)) {
-        // unshifted factorisation (a CholeskyQR pass after the first): a null
-        // direction of G, e.g. an exact zero column of the tall matrix.  This
-        // pivot alone is floored; a shift of the whole diagonal would bias
-        // every other column
-        const float dj = db[dg + j];
-        d = df_split(floor_piv * (double)dj * (double)dj);
-        good = d.x > 0.f;
-      }
-      if (!good) {  // the same value in every thread
-        ok = false;
-        break;
-      }
-      const float2 rp = df_recip(d);
-      if (tid == 0) piv_sh[j] = d;
-      const float2 y = rw[c];
+    constexpr int PB = 8;
+#pragma unroll 1
+    for (int j0 = 0; j0 < CB; j0 += PB) {
+      if (tid < 32) {
+        // the panel's 8 rows in one warp: lane c holds columns c of S and of P
+        const int c = tid;
+        float2 x[PB], y[PB];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int a = g + 4 * i;
-        if (a <= j) continue;  // (warp-uniform)
-        const float2 u = df_mul(rw[a], rp);
-        v[i] = df_fms(v[i], u, y);
-        if (a == j + 1) row_sh[(j + 1) & 1][c] = v[i];
+        for (int i = 0; i < PB; ++i) {
+          x[i] = A[j0 + i][c];
+          y[i] = B[j0 + i][c];
+        }
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+          float2 d = make_float2(__shfl_sync(0xffffffffu, x[i].x, j0 + i),
+                                 __shfl_sync(0xffffffffu, x[i].y, j0 + i));
+          const bool fin = fabsf(d.x) < 3.0e38f;
+          if (!(d.x > 0.f) && fin && p.rel0_n == 0.0) {
+            // unshifted factorisation (a CholeskyQR pass after the first): a null
+            // direction of G, e.g. an exact zero column of the tall matrix.  This
+            // pivot alone is floored; a shift of the whole diagonal would bias
+            // every other column
+            d = cd_split(p.base[b], -2 * p.d[(int64_t)b * np + dg + j0 + i]);
+            if (c == j0 + i) x[i] = d;
+          }
+          ok = ok && fin && d.x > 0.f;  // the same in every lane
+          const float2 rs = df_rsqrt(d);
+          x[i] = df_mul(x[i], rs);  // row j0 + i of R_kk (left of the diagonal: unused)
+          y[i] = df_mul(y[i], rs);
+#pragma unroll
+          for (int a = i + 1; a < PB; ++a) {
+            const float2 f = make_float2(__shfl_sync(0xffffffffu, x[i].x, j0 + a),
+                                         __shfl_sync(0xffffffffu, x[i].y, j0 + a));
+            x[a] = df_fms(x[a], f, x[i]);
+            y[a] = df_fms(y[a], f, y[i]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < PB; ++i) {
+          A[j0 + i][c] = x[i];
+          B[j0 + i][c] = y[i];
+        }
+        if (!ok && c == 0) bad_sh = 1;
+      }
+      __syncthreads();
+      if (bad_sh) break;
+      // rank-8 update of the rows below, columns of S and of P
+      const int c = tid & 63, g = tid >> 6;
+      const bool isS = c < CB;
+      if (j0 + PB < CB && (isS || c - CB < j0 + PB)) {
+        float2 r[PB];
+#pragma unroll
+        for (int i = 0; i < PB; ++i) r[i] = isS ? A[j0 + i][c] : B[j0 + i][c - CB];
+        for (int a = j0 + PB + g; a < CB; a += 4) {
+          float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < PB; ++i) df_dot_acc(acc, A[j0 + i][a], r[i]);
+          float2* dst = isS ? &A[a][c] : &B[a][c - CB];
+          *dst = df_add2(*dst, make_float2(-acc.x, -acc.y));
+        }
       }
       __syncthreads();
     }
-    if (!ok) {
+    if (bad_sh) {
       __syncthreads();
       if (tid == 0) p.status[b] = 2;
       __syncthreads();
       return;
     }
-    // row a scaled by pivot^-1/2: R_ac (c >= a) and Z_aq (q <= a)
-    float2* Zb = p.Zs + b * pp;
     float2* Db = p.Dt + (int64_t)b * CB * CB;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int a = g + 4 * i;
-      const float2 rs = df_rsqrt(piv_sh[a]);
+    for (int e = tid; e < CB * CB; e += CD_THREADS) {
+      const int a = e >> 5, c = e & 31;
       const float2 zero = make_float2(0.f, 0.f);
-      if (isS) {
-        // (a floored pivot's diagonal entry is the pivot, not the stored value)
-        const float2 x = c == a ? df_mul(piv_sh[a], rs) : df_mul(v[i], rs);
-        Rb[(dg + a) * np + dg + c] = c >= a ? x : zero;
-      } else {
-        const int q = c - CB;
-        const float2 x = q <= a ? df_mul(v[i], rs) : zero;
-        Zb[(dg + a) * np + dg + q] = x;
-        Db[q * CB + a] = x;  // R_kk^-1
-      }
+      const float2 z = c <= a ? B[a][c] : zero;
+      Rb[(dg + a) * np + dg + c] = c >= a ? A[a][c] : zero;
+      Zb[(dg + a) * np + dg + c] = z;
+      Db[e] = a <= c ? B[c][a] : zero;  // R_kk^-1
     }
     __syncthreads();
   };
 
   int round = 0;
   for (; round < CD_ROUNDS; ++round) {
-    // ---- scales, then Rs = D (G + s I) D (upper blocks), Zs = 0
+    // ---- scales 2^-d that bring the diagonal into [1/4, 1), then
+    // Rs = D (G + s I) D (upper blocks), Zs = 0
     for (int64_t e = (int64_t)t0 * CD_THREADS + tid; e < (int64_t)b_n * np; e += (int64_t)ts * CD_THREADS) {
       const int64_t b = b_lo + e / np;
       const int j = (int)(e % np);
-      float d = 1.f;
+      int ex = 0;
       if (j < n) {
         const double h = p.G[b * nn + (int64_t)j * n + j] + p.shift[b];
-        int ex = 0;
-        if (h > 0.0 && isfinite(h)) frexp(h, &ex);
-        ex = (ex + ((ex > 0) ? 1 : 0)) / 2;  // ceil(ex / 2)
-        d = ldexpf(1.f, max(-120, min(120, -ex)));
+        const int eb = (int)((uint64_t)__double_as_longlong(h) >> 52);  // sign and exponent
+        if (eb > 0 && eb < 0x7ff) ex = eb - 1022;
+        ex = (ex + (ex > 0 ? 1 : 0)) / 2;  // ceil(ex / 2)
       }
-      p.d[b * np + j] = d;
+      p.d[b * np + j] = ex;
     }
     barrier();
     for (int64_t e = (int64_t)t0 * CD_THREADS + tid; e < (int64_t)b_n * pp; e += (int64_t)ts * CD_THREADS) {
-      const int64_t b = b_lo + e / pp, r = e % pp;
+      const int64_t b = b_lo + e / pp;
+      const int r = (int)(e % pp);
       if (p.status[b] != 0) continue;
-      const int i = (int)(r / np), j = (int)(r % np);
+      const int i = r / np, j = r % np;
       p.Zs[b * pp + r] = make_float2(0.f, 0.f);
       if (i / CB > j / CB) continue;
       float2 v = make_float2(i == j ? 1.f : 0.f, 0.f);
@@ -293,7 +368,7 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
         // the diagonal blocks hold both triangles
         double h = p.G[b * nn + (i <= j ? (int64_t)i * n + j : (int64_t)j * n + i)];
         if (i == j) h += p.shift[b];
-        v = df_split(h * (double)p.d[b * np + i] * (double)p.d[b * np + j]);
+        v = cd_split(h, -p.d[b * np + i] - p.d[b * np + j]);
       }
       p.Rs[b * pp + r] = v;
     }
@@ -396,8 +471,7 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
       __syncthreads();
       if (s == 2) {
         if (tid == 0) {
-          const double base = p.relfail * p.trace[b] / n;
-          p.shift[b] = fmax(p.shift[b] * 100.0, base);
+          p.shift[b] = fmax(p.shift[b] * 100.0, p.base[b]);
           p.status[b] = 0;
           atomicMax(p.used, round + 1);
         }
@@ -413,8 +487,7 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
       if (s == 0) {
         p.status[b] = 1;
       } else if (s == 2) {
-        const double base = p.relfail * p.trace[b] / n;
-        p.shift[b] = fmax(p.shift[b] * 100.0, base);
+        p.shift[b] = fmax(p.shift[b] * 100.0, p.base[b]);
         p.status[b] = 0;
         atomicAdd(&p.pending[round], 1);
         atomicMax(p.used, round + 1);
@@ -425,12 +498,12 @@ __global__ void __launch_bounds__(CD_THREADS) chol_df_kernel(const CholDf p) {
   }
   // ---- out: R = Rs D^-1, W = D Zs^T
   for (int64_t e = (int64_t)t0 * CD_THREADS + tid; e < (int64_t)b_n * nn; e += (int64_t)ts * CD_THREADS) {
-    const int64_t b = b_lo + e / nn, r = e % nn;
-    const int i = (int)(r / n), j = (int)(r % n);
-    const float* db = p.d + b * np;
+    const int64_t b = b_lo + e / nn;
+    const int r = (int)(e % nn), i = r / n, j = r % n;
+    const int* db = p.d + b * np;
     const bool up = i <= j;
-    p.R[b * nn + r] = up ? df_val(p.Rs[b * pp + (int64_t)i * np + j]) * (double)(1.0f / db[j]) : 0.0;
-    p.W[b * nn + r] = up ? df_val(p.Zs[b * pp + (int64_t)j * np + i]) * (double)db[i] : 0.0;
+    p.R[b * nn + r] = up ? cd_join(p.Rs[b * pp + (int64_t)i * np + j], db[j]) : 0.0;
+    p.W[b * nn + r] = up ? cd_join(p.Zs[b * pp + (int64_t)j * np + i], -db[i]) : 0.0;
   }
   for (int bb = t0 * CD_THREADS + tid; bb < b_n; bb += ts * CD_THREADS) {
     const int s = p.status[b_lo + bb];
@@ -449,14 +522,14 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
   p.Rs = ws.take<float2>(pp * batch);
   p.Zs = ws.take<float2>(pp * batch);
   p.Dt = ws.take<float2>((size_t)batch * CB * CB);
-  p.d = ws.take<float>((size_t)batch * p.np);
-  p.trace = ws.take<double>(batch);
+  p.d = ws.take<int>((size_t)batch * p.np);
   p.shift = ws.take<double>(batch);
+  p.base = ws.take<double>(batch);
   p.status = ws.take<int>(batch);
   p.used = ws.take<int>(1);
   p.pending = ws.take<int>(CD_ROUNDS);
   p.colsq = (batch == 1 && rel0 == 0.0 && near_tol > 0.0)
-                ? ws.take<double>((size_t)CD_NEAR_GROUPS * n)
+                ? ws.take<float>((size_t)CD_NEAR_GROUPS * n)
                 : nullptr;
   if (ws.measuring() || n == 0 || batch == 0) return PLOM_OK;
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "chol: workspace too small");
@@ -468,9 +541,9 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
   p.info = info;
   p.n = n;
   p.batch = batch;
-  p.rel0 = rel0;
-  p.relfail = relfail;
-  p.near_tol = p.colsq ? near_tol : 0.0;
+  p.rel0_n = rel0 / n;
+  p.relfail_n = relfail / n;
+  p.near_tol = p.colsq ? (float)near_tol : 0.f;
   // one CTA per problem when the blocks are few (3 tiles a step at 64 columns:
   // 2 us each, no more than a grid barrier) or the problems are many
   p.solo = T <= 2 || batch >= 16;
