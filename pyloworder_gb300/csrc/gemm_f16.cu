@@ -232,51 +232,67 @@ __device__ __forceinline__ float2 ld_shared_h2f(uint32_t addr) {
 // ---------------------------------------------------------------------------
 // column maxima of |Y| (bits of non-negative floats order like unsigned ints);
 // each block takes a contiguous range of rows, threads take 4-column groups
-// (16-byte loads when rows are aligned)
+// (16-byte loads when rows are aligned).  HBM-bound.  The block's maxima meet in
+// shared memory and only one value per column and block goes to the global
+// maxima: with one per thread, narrow matrices were bound by the atomics on
+// their few addresses (2,097,152 x 64: 447 us, 80 us with this).
 __global__ void __launch_bounds__(256) colmax_kernel(const float* __restrict__ Y, int64_t ld,
-                                                     int64_t m, int N, int vec, int64_t bstride,
+                                                     int64_t m, int N, int vec, int sh,
+                                                     int64_t bstride,
                                                      unsigned* __restrict__ cmax) {
+  extern __shared__ unsigned cm_dyn[];  // N (sh; wider matrices go to the global maxima)
   // problem blockIdx.y of a batch (matrices bstride elements apart)
   Y += (int64_t)blockIdx.y * bstride;
   cmax += (int64_t)blockIdx.y * N;
+  unsigned* cm_sh = sh ? cm_dyn : cmax;
+  if (sh) {
+    for (int c = threadIdx.x; c < N; c += blockDim.x) cm_sh[c] = 0u;
+    __syncthreads();
+  }
   const int64_t rows = (m + gridDim.x - 1) / gridDim.x;
   const int64_t r0b = (int64_t)blockIdx.x * rows;
   const int64_t r1 = (r0b + rows < m) ? r0b + rows : m;
   // narrow matrices: the block's threads split into (row lane, column group)
   // so that all of them read; rows r0b + tr, r0b + tr + TR, ...
-  const int groups = vec ? N / 4 : N;
-  const int TR = groups >= (int)blockDim.x ? 1 : (int)blockDim.x / groups;
-  const int tr = (int)threadIdx.x / (groups >= (int)blockDim.x ? (int)blockDim.x : groups);
-  const int tc = (int)threadIdx.x - tr * (groups >= (int)blockDim.x ? (int)blockDim.x : groups);
-  if (tr >= TR) return;
+  const int groups = vec ? (N + 3) / 4 : N;
   const int cstep = groups >= (int)blockDim.x ? (int)blockDim.x : groups;
+  const int TR = (int)blockDim.x / cstep;
+  const int tr = (int)threadIdx.x / cstep;
+  const int tc = (int)threadIdx.x - tr * cstep;
   const int64_t r0 = r0b + tr;
-  if (vec) {
-    for (int c = tc * 4; c < N; c += cstep * 4) {
-      float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float* p = Y + r0 * ld + c;
+  if (tr < TR) {
+    for (int g = tc; g < groups; g += cstep) {
+      const int c = vec ? 4 * g : g;
+      if (vec && c + 4 <= N) {
+        float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* p = Y + r0 * ld + c;
 #pragma unroll 8
-      for (int64_t r = r0; r < r1; r += TR, p += TR * ld) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
-        mx.x = fmaxf(mx.x, fabsf(v.x));
-        mx.y = fmaxf(mx.y, fabsf(v.y));
-        mx.z = fmaxf(mx.z, fabsf(v.z));
-        mx.w = fmaxf(mx.w, fabsf(v.w));
+        for (int64_t r = r0; r < r1; r += TR, p += TR * ld) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+          mx.x = fmaxf(mx.x, fabsf(v.x));
+          mx.y = fmaxf(mx.y, fabsf(v.y));
+          mx.z = fmaxf(mx.z, fabsf(v.z));
+          mx.w = fmaxf(mx.w, fabsf(v.w));
+        }
+        atomicMax(&cm_sh[c], __float_as_uint(mx.x));
+        atomicMax(&cm_sh[c + 1], __float_as_uint(mx.y));
+        atomicMax(&cm_sh[c + 2], __float_as_uint(mx.z));
+        atomicMax(&cm_sh[c + 3], __float_as_uint(mx.w));
+      } else {  // one column, or the last columns of a row
+        for (int q = c; q < (vec ? N : c + 1); ++q) {
+          float mx = 0.f;
+          const float* p = Y + r0 * ld + q;
+#pragma unroll 8
+          for (int64_t r = r0; r < r1; r += TR, p += TR * ld) mx = fmaxf(mx, fabsf(__ldg(p)));
+          atomicMax(&cm_sh[q], __float_as_uint(mx));
+        }
       }
-      if (mx.x > 0.f) atomicMax(&cmax[c], __float_as_uint(mx.x));
-      if (mx.y > 0.f) atomicMax(&cmax[c + 1], __float_as_uint(mx.y));
-      if (mx.z > 0.f) atomicMax(&cmax[c + 2], __float_as_uint(mx.z));
-      if (mx.w > 0.f) atomicMax(&cmax[c + 3], __float_as_uint(mx.w));
-    }
-  } else {
-    for (int c = tc; c < N; c += cstep) {
-      float mx = 0.f;
-      const float* p = Y + r0 * ld + c;
-#pragma unroll 8
-      for (int64_t r = r0; r < r1; r += TR, p += TR * ld) mx = fmaxf(mx, fabsf(__ldg(p)));
-      if (mx > 0.f) atomicMax(&cmax[c], __float_as_uint(mx));
     }
   }
+  if (!sh) return;
+  __syncthreads();
+  for (int c = threadIdx.x; c < N; c += blockDim.x)
+    if (cm_sh[c]) atomicMax(&cmax[c], cm_sh[c]);
 }
 
 // s_j = 2^(14 - e_j) with max_j = f 2^e_j, f in [0.5, 1); 1 for zero or
@@ -738,32 +754,46 @@ __global__ void tn16_reduce_kernel(const double* __restrict__ part, int Na, int 
   }
 }
 
-// G[i][j] = sum over chunks of the tile partials (fixed order) / (s_i s_j), mirrored
-__global__ void gram16_reduce_kernel(const double* __restrict__ part, int N, int tn, int chunks,
-                                     const float* __restrict__ s, double* __restrict__ G,
-                                     int batch, int ld, int accumulate) {
-  const int64_t total = (int64_t)N * N * batch;
+// G[i][j] = sum over chunks of the tile partials (fixed order) / (s_i s_j),
+// mirrored.  A block takes 32 consecutive columns of one row and splits the
+// chunks over its 16 warps (chunk c to warp c mod 16, their sums added in warp
+// order): one thread per element ran 600 dependent loads deep (98 us at
+// 64 columns, 9 us with this).
+constexpr int GR_WARPS = 16;
+__global__ void __launch_bounds__(32 * GR_WARPS) gram16_reduce_kernel(
+    const double* __restrict__ part, int N, int tn, int chunks, const float* __restrict__ s,
+    double* __restrict__ G, int batch, int ld, int accumulate) {
+  __shared__ float2 red[GR_WARPS][32];
   const int ntiles = tn * (tn + 1) / 2;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t pb = e / ((int64_t)N * N);
-    const int64_t r = e - pb * N * N;
-    const int i = (int)(r / N), j = (int)(r % N);
-    int a = i, b = j;
-    if (a / 128 > b / 128) {
-      a = j;
-      b = i;
-    }
-    const int ti = a / 128, tj = b / 128;
+  const int cblk = (N + 31) / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tasks = (int64_t)batch * N * cblk;
+  for (int64_t t = blockIdx.x; t < tasks; t += gridDim.x) {
+    const int64_t pb = t / ((int64_t)N * cblk);
+    const int r = (int)(t - pb * N * cblk);
+    const int i = r / cblk, j0 = (r % cblk) * 32, j = j0 + lane;
+    if (j0 + 31 < i) continue;  // below the diagonal: the mirror writes it (uniform)
+    const int ti = i / 128, tj = j0 / 128;
     const int tile = ti * tn - ti * (ti - 1) / 2 + (tj - ti);
     const float2* p = reinterpret_cast<const float2*>(part) +
-                      ((pb * ntiles + tile) * chunks) * 128 * 128 + (int64_t)(a - ti * 128) * 128 +
-                      (b - tj * 128);
+                      ((pb * ntiles + tile) * chunks) * 128 * 128 + (int64_t)(i - ti * 128) * 128 +
+                      (j - tj * 128);
     float2 acc = make_float2(0.f, 0.f);
-    for (int c = 0; c < chunks; ++c) acc = dw_add(acc, p[(int64_t)c * 128 * 128]);
-    const float* sp = s + pb * ld;
-    const double v = dw_value(acc) / ((double)sp[i] * (double)sp[j]);
-    G[e] = accumulate ? G[e] + v : v;
+#pragma unroll 4
+    for (int c = warp; c < chunks; c += GR_WARPS) acc = dw_add(acc, p[(int64_t)c * 128 * 128]);
+    red[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && j < N && j >= i) {
+#pragma unroll
+      for (int w = 1; w < GR_WARPS; ++w) acc = dw_add(acc, red[w][lane]);
+      const float* sp = s + pb * ld;
+      const double v = dw_value(acc) / ((double)sp[i] * (double)sp[j]);
+      const int64_t up = pb * N * N + (int64_t)i * N + j, lo = pb * N * N + (int64_t)j * N + i;
+      const double g = accumulate ? G[up] + v : v;
+      G[up] = g;
+      G[lo] = g;
+    }
+    __syncthreads();
   }
 }
 
@@ -2208,12 +2238,15 @@ int pack_f32(const float* Y, int64_t ld, int64_t m, int64_t N, Packed& p, Arena&
   const int threads = 256;
   {
     ProfScope prof("colmax", st, 0.0, 4.0 * (double)m * N);
+    // small inputs: 8,192 values a block (32 a thread), few global maxima a column
     const int rblocks = (int)std::max<int64_t>(
-        1, std::min<int64_t>(m, cdiv((int64_t)num_sms() * 8, batch)));
-    const int cvec = ((ld & 3) == 0) && ((N & 3) == 0) && ((bstride & 3) == 0) &&
+        1, std::min<int64_t>(std::min<int64_t>(m, cdiv(m * N, 8192)),
+                             cdiv((int64_t)num_sms() * 8, batch)));
+    const int cvec = ((ld & 3) == 0) && ((bstride & 3) == 0) &&
                      ((reinterpret_cast<uintptr_t>(Y) & 15) == 0);
-    hp::colmax_kernel<<<dim3(rblocks, (unsigned)batch), threads, 0, st>>>(Y, ld, m, (int)N, cvec,
-                                                                         bstride, cmax);
+    const int sh = N <= 8192;
+    hp::colmax_kernel<<<dim3(rblocks, (unsigned)batch), threads, sh ? sizeof(unsigned) * N : 0, st>>>(
+        Y, ld, m, (int)N, cvec, sh, bstride, cmax);
     PLOM_CHECK_LAUNCH();
     hp::colscale_kernel<<<(int)std::min<int64_t>(cdiv(p.ld * batch, 256), 4096), 256, 0, st>>>(
         cmax, (int)N, (int)p.ld, (int)batch, p.scale);
@@ -2391,10 +2424,9 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
   hp::gram16_kernel<true><<<(unsigned)(batch * tiles * chunks_eff), 320, hp::G_SMEM, st>>>(
       tm, tm, m, tn, tn, rpc, chunks_eff, part, err, p.mp);
   PLOM_CHECK_LAUNCH();
-  const int64_t total = N * N * batch;
-  const int blocks = (int)std::min<int64_t>(cdiv(total, 256), (int64_t)num_sms() * 16);
+  const int blocks = (int)std::min<int64_t>(batch * N * cdiv(N, 32), (int64_t)num_sms() * 4);
   ProfScope prof_r("gram_reduce", st, 0.0, 8.0 * (double)batch * tiles * chunks_eff * 128 * 128);
-  hp::gram16_reduce_kernel<<<blocks, 256, 0, st>>>(part, (int)N, tn, chunks_eff, p.scale, G,
+  hp::gram16_reduce_kernel<<<blocks, 32 * hp::GR_WARPS, 0, st>>>(part, (int)N, tn, chunks_eff, p.scale, G,
                                                    (int)batch, (int)p.ld, accumulate ? 1 : 0);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
