@@ -1,9 +1,13 @@
 // Small utility kernels: type conversion, strided 2-D copies and the Philox
 // uniform generator for the randomized range finder's test matrix.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "plom_common.cuh"
 #include "plom_kernels.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace plom {
 
@@ -120,158 +124,128 @@ int fill_uniform_dispatch(int dtype, void* out, int64_t count, uint64_t seed, cu
 // ---------------------------------------------------------------------------
 constexpr int NC_MAX = 8;
 
-__global__ void nc_candidates_kernel(const double* __restrict__ S, int n, int* __restrict__ list,
-                                     int* __restrict__ count) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int c = 0;
-  const double thr = 1e-6 * S[0];
-  for (int j = n - 1; j >= 0 && c < NC_MAX; --j) {
-    if (!(S[j] <= thr)) break;
-    list[c++] = j;
-  }
-  *count = c;
-}
-
-// part[q gn + blockIdx.x] = sum over the 32 rows k of this block of
-// m_c[k] (G m_c)[k] (c = list[q]); the 8 warps' shares summed in a fixed order
-__global__ void __launch_bounds__(256) nc_norms_kernel(const double* __restrict__ G,
-                                                       const double* __restrict__ Mf, int N,
-                                                       const int* __restrict__ list,
-                                                       const int* __restrict__ count,
-                                                       double* __restrict__ part) {
-  const int q = blockIdx.y;
-  if (q >= *count) return;
-  const int c = list[q];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  __shared__ double red[8];
-  double mine = 0.0;
-  for (int k = blockIdx.x * 32 + wib; k < min(N, (int)blockIdx.x * 32 + 32); k += 8) {
-    double acc = 0.0;
-    for (int l = lane; l < N; l += 32) acc = fma(G[(int64_t)k * N + l], Mf[(int64_t)l * N + c], acc);
-    acc = warp_sum(acc);
-    mine = fma(Mf[(int64_t)k * N + c], acc, mine);
-  }
-  if (lane == 0) red[wib] = mine;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < 8; ++w) t += red[w];
-    part[(int64_t)q * gridDim.x + blockIdx.x] = t;
-  }
-}
-
-// out[q] = sum of the g partials of candidate q, in a fixed order (one warp
-// per candidate)
-__global__ void __launch_bounds__(32 * NC_MAX) nc_sum_kernel(const double* __restrict__ part,
-                                                             int g, double* __restrict__ out) {
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double t = 0.0;
-  for (int k = lane; k < g; k += 32) t += part[(int64_t)q * g + k];
-  t = warp_sum(t);
-  if (lane == 0) out[q] = t;
-}
-
 __device__ __forceinline__ int64_t nc_row(int q, int64_t m) {
   return (int64_t)(((uint64_t)(q + 1) * 2654435761ull) % (uint64_t)m);
 }
 
-// u = e_i - U w, w = row i of U without the columns still to be completed
-// (this one included); written into column list[q], the block's share of its
-// squared norm into part[blockIdx.x] (warps summed in a fixed order)
+// All of it in one cooperative launch: without candidates (or with candidates
+// of unit norm, the usual case) every block finds that out by itself and
+// returns; 19 launches cost 55 us a call whether or not there was work.
+//  npart[q gridDim.x + block]: the block's share of candidate q's squared norm,
+//  ppart[block]: its share of a completed column's; all summed in block order.
 template <typename T>
-__global__ void __launch_bounds__(256) nc_project_kernel(T* __restrict__ U, int64_t m, int n,
-                                                         int64_t ldu, const int* __restrict__ list,
-                                                         const int* __restrict__ count,
-                                                         const double* __restrict__ sums, int q,
-                                                         double* __restrict__ part) {
-  if (q >= *count || !(sums[q] < 0.25)) return;
-  extern __shared__ double ncw[];
+__global__ void __launch_bounds__(256) nc_complete_kernel(const double* __restrict__ S, int n,
+                                                          T* U, int64_t m, int64_t ldu,
+                                                          const double* __restrict__ G,
+                                                          const double* __restrict__ Mf,
+                                                          double* npart, double* ppart) {
+  cg::grid_group grid = cg::this_grid();
+  extern __shared__ double ncw[];  // n
   __shared__ double red[8];
-  const int64_t i = nc_row(q, m);
-  const int c = list[q];
-  for (int j = threadIdx.x; j < n; j += blockDim.x) ncw[j] = (double)U[i * ldu + j];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int p = q; p < *count; ++p)
-      if (sums[p] < 0.25) ncw[list[p]] = 0.0;
-  }
-  __syncthreads();
+  __shared__ double sums[NC_MAX];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double mine = 0.0;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + wib; r < m; r += (int64_t)gridDim.x * 8) {
-    const T* row = U + r * ldu;
-    double acc = 0.0;
-    for (int j = lane; j < n; j += 32) acc = fma((double)row[j], ncw[j], acc);
-    acc = warp_sum(acc);
-    const double u = (r == i ? 1.0 : 0.0) - acc;
-    if (lane == 0) {
-      U[r * ldu + c] = (T)u;
-      mine = fma(u, u, mine);
-    }
-  }
-  if (lane == 0) red[wib] = mine;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  // the sum of v over the block, in a fixed order, to every thread
+  auto block_sum = [&](double v) {
+    __syncthreads();
+    if (lane == 0) red[wib] = v;
+    __syncthreads();
     double t = 0.0;
     for (int w = 0; w < 8; ++w) t += red[w];
-    part[blockIdx.x] = t;
+    return t;
+  };
+  // candidates: the smallest singular values <= 1e-6 sigma_1, column n - 1 - q
+  int cnt = 0;
+  {
+    const double thr = 1e-6 * S[0];
+    while (cnt < NC_MAX && cnt < n && S[n - 1 - cnt] <= thr) ++cnt;
   }
-}
-
-// every block sums the gp partials of the projection in a fixed order, then
-// scales its rows of the completed column to unit norm
-template <typename T>
-__global__ void __launch_bounds__(256) nc_scale_kernel(T* __restrict__ U, int64_t m, int64_t ldu,
-                                                       const int* __restrict__ list,
-                                                       const int* __restrict__ count,
-                                                       const double* __restrict__ sums, int q,
-                                                       const double* __restrict__ part, int gp) {
-  if (q >= *count || !(sums[q] < 0.25)) return;
-  __shared__ double red[8];
-  double t = 0.0;
-  for (int k = threadIdx.x; k < gp; k += blockDim.x) t += part[k];
-  t = warp_sum(t);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+  if (cnt == 0) return;
+  // ||U e_c||^2 = m_c^T G m_c: each block takes rows k of it
+  for (int q = 0; q < cnt; ++q) {
+    const int c = n - 1 - q;
+    double mine = 0.0;
+    for (int k = blockIdx.x * 8 + wib; k < n; k += gridDim.x * 8) {
+      double acc = 0.0;
+      for (int l = lane; l < n; l += 32) acc = fma(G[(int64_t)k * n + l], Mf[(int64_t)l * n + c], acc);
+      acc = warp_sum(acc);
+      mine = fma(Mf[(int64_t)k * n + c], acc, mine);
+    }
+    const double t = block_sum(lane == 0 ? mine : 0.0);
+    if (threadIdx.x == 0) npart[(int64_t)q * gridDim.x + blockIdx.x] = t;
+  }
+  grid.sync();
+  bool any = false;
+  for (int q = 0; q < cnt; ++q) {
+    double t = 0.0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) t += npart[(int64_t)q * gridDim.x + k];
+    t = block_sum(warp_sum(t));
+    if (threadIdx.x == 0) sums[q] = t;
+    any = any || t < 0.25;
+  }
   __syncthreads();
-  double nrm2 = 0.0;
-  for (int w = 0; w < 8; ++w) nrm2 += red[w];
-  if (!(nrm2 > 0.0)) return;
-  const int c = list[q];
-  const double f = 1.0 / sqrt(nrm2);
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x)
-    U[r * ldu + c] = (T)((double)U[r * ldu + c] * f);
+  if (!any) return;  // the same in every block
+  for (int q = 0; q < cnt; ++q) {
+    if (!(sums[q] < 0.25)) continue;
+    // u = e_i - U w, w = row i of U without the columns still to be completed
+    const int64_t i = nc_row(q, m);
+    const int c = n - 1 - q;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      const int p = n - 1 - j;
+      ncw[j] = (p >= q && p < cnt && sums[p] < 0.25) ? 0.0 : (double)U[i * ldu + j];
+    }
+    grid.sync();  // row i is read before any block writes its column c
+    double mine = 0.0;
+    for (int64_t r = (int64_t)blockIdx.x * 8 + wib; r < m; r += (int64_t)gridDim.x * 8) {
+      const T* row = U + r * ldu;
+      double acc = 0.0;
+      for (int j = lane; j < n; j += 32) acc = fma((double)row[j], ncw[j], acc);
+      acc = warp_sum(acc);
+      const double u = (r == i ? 1.0 : 0.0) - acc;
+      if (lane == 0) {
+        U[r * ldu + c] = (T)u;
+        mine = fma(u, u, mine);
+      }
+    }
+    const double t = block_sum(lane == 0 ? mine : 0.0);
+    if (threadIdx.x == 0) ppart[blockIdx.x] = t;
+    grid.sync();
+    double nrm2 = 0.0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) nrm2 += ppart[k];
+    nrm2 = block_sum(warp_sum(nrm2));
+    if (nrm2 > 0.0) {
+      const double f = 1.0 / sqrt(nrm2);
+      for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
+           r += (int64_t)gridDim.x * blockDim.x)
+        U[r * ldu + c] = (T)((double)U[r * ldu + c] * f);
+    }
+    grid.sync();
+  }
 }
 
 template <typename T>
 int complete_null_columns(const double* S, int n, T* U, int64_t m, int64_t ldu, const double* G,
                           const double* Mf, Arena& ws, cudaStream_t st) {
-  const unsigned gn = (unsigned)std::max<int64_t>(1, cdiv(n, 32));
-  const unsigned gp = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(m, 8), (int64_t)num_sms() * 8));
-  int* list = ws.take<int>(NC_MAX);
-  int* count = ws.take<int>(1);
-  double* sums = ws.take<double>(NC_MAX);
-  double* npart = ws.take<double>((size_t)NC_MAX * gn);
-  double* ppart = ws.take<double>(gp);
+  const int maxb = 2 * num_sms();  // co-resident: 256 threads, at most 64 KiB shared
+  double* npart = ws.take<double>((size_t)NC_MAX * maxb);
+  double* ppart = ws.take<double>(maxb);
   if (ws.measuring() || n < 1 || m < 1) return PLOM_OK;
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "null-column completion: workspace too small");
   PLOM_REQUIRE(S && U && G && Mf && n <= 8192, PLOM_ERR_ARG,
                "null-column completion: bad arguments");
-  ProfScope prof("null_cols", st, 0.0, (double)sizeof(T) * m, 3 + 2 * NC_MAX);
-  nc_candidates_kernel<<<1, 32, 0, st>>>(S, n, list, count);
-  PLOM_CHECK_LAUNCH();
-  const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(m, 256), (int64_t)num_sms() * 4));
-  nc_norms_kernel<<<dim3(gn, NC_MAX), 256, 0, st>>>(G, Mf, n, list, count, npart);
-  PLOM_CHECK_LAUNCH();
-  nc_sum_kernel<<<1, 32 * NC_MAX, 0, st>>>(npart, (int)gn, sums);
-  PLOM_CHECK_LAUNCH();
-  for (int q = 0; q < NC_MAX; ++q) {
-    nc_project_kernel<T><<<gp, 256, sizeof(double) * n, st>>>(U, m, n, ldu, list, count, sums, q,
-                                                              ppart);
-    PLOM_CHECK_LAUNCH();
-    nc_scale_kernel<T><<<gx, 256, 0, st>>>(U, m, ldu, list, count, sums, q, ppart, (int)gp);
-    PLOM_CHECK_LAUNCH();
-  }
+  ProfScope prof("null_cols", st, 0.0, (double)sizeof(T) * m);
+  const void* k = (const void*)nc_complete_kernel<T>;
+  const size_t smem = sizeof(double) * (size_t)n;
+  if (smem > 48 * 1024)
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  int per_sm = 0;
+  PLOM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, smem));
+  // few blocks for small problems: the candidates' norms are all they compute
+  // unless a column is completed, and that reads U once
+  const int blocks = (int)std::max<int64_t>(
+      1, std::min<int64_t>({(int64_t)maxb, (int64_t)std::max(1, per_sm) * num_sms(), cdiv(m, 64)}));
+  void* args[] = {(void*)&S, (void*)&n, (void*)&U,  (void*)&m,     (void*)&ldu,
+                  (void*)&G, (void*)&Mf, (void*)&npart, (void*)&ppart};
+  PLOM_CHECK_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(256), args, smem, st));
   return PLOM_OK;
 }
 template int complete_null_columns<float>(const double*, int, float*, int64_t, int64_t,
