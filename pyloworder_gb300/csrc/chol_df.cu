@@ -567,4 +567,91 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
   return PLOM_OK;
 }
 
+// ---------------------------------------------------------------------------
+// C = A B for n x n FP64 operands in double-float arithmetic (R3 R2 R1 and
+// R3^-1 Ur of the mixed form): a 32 x 32 tile per CTA, the next pair of blocks
+// in flight while one is multiplied.  tri bit 0: A upper triangular, bit 1: B
+// upper triangular (zero blocks are skipped; B is then scaled by the power of
+// two of its largest diagonal entry, so that a factor of data of any FP32
+// magnitude fits).  An FP64 multiply-add issues at 2 lanes a clock and SM: one
+// 32 x 32 x 32 block took 14 us, here 3.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __restrict__ A,
+                                                             const double* __restrict__ B,
+                                                             double* __restrict__ C, int n,
+                                                             int tri) {
+  __shared__ __align__(16) float2 As[CB][CPITCH];  // [k][row of A]
+  __shared__ __align__(16) float2 Bs[CB][CPITCH];
+  __shared__ int ex_sh;
+  const int tid = threadIdx.x;
+  const int64_t nn = (int64_t)n * n;
+  A += blockIdx.z * nn;
+  B += blockIdx.z * nn;
+  C += blockIdx.z * nn;
+  const int bi = blockIdx.y, bj = blockIdx.x;
+  int sb = 0;
+  if (tri & 2) {
+    if (tid == 0) ex_sh = 0;
+    __syncthreads();
+    int ex = 0;
+    for (int i = tid; i < n; i += CD_THREADS)
+      ex = max(ex, (int)((uint64_t)__double_as_longlong(B[(int64_t)i * n + i]) >> 52) & 0x7ff);
+    ex = warp_max(ex);
+    if ((tid & 31) == 0) atomicMax(&ex_sh, ex);
+    __syncthreads();
+    sb = (ex_sh > 0 && ex_sh < 0x7ff) ? 1023 - ex_sh : 0;
+  }
+  const int T = (n + CB - 1) / CB;
+  const int k0 = (tri & 1) ? bi : 0, k1 = (tri & 2) ? bj : T - 1;
+  const int c = tid & 31, r = tid >> 5;  // rows r, r + 8, ...
+  float2 acc[2][2];
+  acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = make_float2(0.f, 0.f);
+  double va[4], vb[4];
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int ai = bi * CB + r + 8 * u, ak = k * CB + c;
+      const int bk = k * CB + r + 8 * u, bc = bj * CB + c;
+      va[u] = (ai < n && ak < n) ? A[(int64_t)ai * n + ak] : 0.0;
+      vb[u] = (bk < n && bc < n) ? B[(int64_t)bk * n + bc] : 0.0;
+    }
+  };
+  if (k0 <= k1) fetch(k0);
+  for (int k = k0; k <= k1; ++k) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      As[c][r + 8 * u] = cd_split(va[u], 0);
+      Bs[r + 8 * u][c] = cd_split(vb[u], sb);
+    }
+    __syncthreads();
+    if (k < k1) fetch(k + 1);
+    float2 m[2][2];
+    cd_mm(As, Bs, m);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) acc[u][v] = df_add2(acc[u][v], m[u][v]);
+  }
+  const int ty = tid >> 4, tx = tid & 15;
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int i = bi * CB + 2 * ty + u, j = bj * CB + 2 * tx + v;
+      if (i < n && j < n) C[(int64_t)i * n + j] = cd_join(acc[u][v], -sb);
+    }
+}
+
+int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
+               cudaStream_t st) {
+  if (n <= 0 || batch <= 0) return PLOM_OK;
+  PLOM_REQUIRE(A && B && C && batch <= 65535, PLOM_ERR_ARG, "gemm_df: bad arguments");
+  ProfScope prof("gemm_df", st, 2.0 * n * n * n * batch, 24.0 * n * n * batch);
+  const unsigned T = (unsigned)cdiv(n, CB);
+  gemm_df_kernel<<<dim3(T, T, (unsigned)batch), CD_THREADS, 0, st>>>(A, B, C, n, tri);
+  PLOM_CHECK_LAUNCH();
+  return PLOM_OK;
+}
+
 }  // namespace plom

@@ -74,6 +74,10 @@ int chol_shifted(const double* G, double* R, int n, int batch, double shift_rel0
 int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, double shift_rel0,
                     double shift_rel_fail, int* info, Arena& ws, cudaStream_t st,
                     double near_tol = 0.0);
+// C = A B (n x n, batch of problems n*n apart) in double-float arithmetic; tri
+// as in gemm_sq.
+int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
+               cudaStream_t st);
 // W = R^{-1} for upper-triangular R (batch, stride n*n).
 int trtri_upper(const double* R, double* W, int n, int batch, Arena& ws, cudaStream_t st);
 // One-sided Jacobi SVD of `batch` square n x n matrices A (ld n, stride n*n),

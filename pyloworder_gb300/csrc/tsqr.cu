@@ -270,14 +270,15 @@ static int cholqr3_packed_passes23(bool cplx, int n, PackedCore& b, double relfa
   PLOM_TRY(sub([&] { return apply_packed(b.P1, F2, N, N, nullptr, 0, &b.P2, info, ws, st, 0, 0, true); }));
   // pass 3
   PLOM_TRY(sub([&] { return chol_pass_packed(cplx, n, b.P2, b, b.R3, b.W3, 0.0, relfail, info, ws, st); }));
-  // Re = R3 R2 R1: double-float products from n = 256 on (the factors carry
-  // the 22-bit operands' information; FP64 runs at 1/64 of the FP32 rate)
+  // Re = R3 R2 R1 in double-float arithmetic (the factors carry the 22-bit
+  // operands' information; FP64 runs at 1/64 of the FP32 rate): from n = 256 on
+  // as FP32 products with double-float sums
   if (N >= DF_PRODUCT_MIN_N) {
     PLOM_TRY(sub([&] { return gemm_nn_df(b.R3, b.R2, b.Rp, N, ws, st); }));
     PLOM_TRY(sub([&] { return gemm_nn_df(b.Rp, b.R1, b.Re, N, ws, st); }));
   } else if (!ws.measuring()) {
-    PLOM_TRY((gemm_sq_nn(b.R3, b.R2, b.Rp, N, 1, 3, st)));
-    PLOM_TRY((gemm_sq_nn(b.Rp, b.R1, b.Re, N, 1, 3, st)));
+    PLOM_TRY(gemm_df_nn(b.R3, b.R2, b.Rp, N, 1, 3, st));
+    PLOM_TRY(gemm_df_nn(b.Rp, b.R1, b.Re, N, 1, 3, st));
   }
   ws.off = need;
   return PLOM_OK;
@@ -457,10 +458,10 @@ static int svd_tail_packed(bool cplx, int n, PackedCore& b, int64_t m, float* U,
     // M = R3^-1 Ur (embedded for complex), the right operand of Q2 x M
     if (cplx) {
       PLOM_TRY(complex_to_embed(Ur, Ue, n, 1, st));
-      PLOM_TRY((gemm_sq_nn(b.W3, Ue, Me, N, 1, 1, st)));
+      PLOM_TRY(gemm_df_nn(b.W3, Ue, Me, N, 1, 1, st));
       PLOM_TRY(embed_to_rowform(Me, b.F, n, 1, st));
     } else {
-      PLOM_TRY((gemm_sq_nn(b.W3, Ur, Me, N, 1, 1, st)));
+      PLOM_TRY(gemm_df_nn(b.W3, Ur, Me, N, 1, 1, st));
       Mop = Me;
     }
   }
@@ -569,8 +570,8 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
   PLOM_TRY(pass(P2, R3, W3, 0.0));
   const double* Rin = Re;
   if (!meas) {
-    PLOM_TRY((gemm_sq_nn(R3, R2, Rp, N, bi, 3, st)));
-    PLOM_TRY((gemm_sq_nn(Rp, R1, Re, N, bi, 3, st)));
+    PLOM_TRY((gemm_df_nn(R3, R2, Rp, N, bi, 3, st)));
+    PLOM_TRY((gemm_df_nn(Rp, R1, Re, N, bi, 3, st)));
     if (cplx) {
       PLOM_TRY(embed_to_complex(Re, Rc, n, bi, st));
       Rin = Rc;
@@ -582,10 +583,10 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
     // M = R3^-1 Ur (embedded for complex), the right operand of Q2 x M
     if (cplx) {
       PLOM_TRY(complex_to_embed(Ur, Ue, n, bi, st));
-      PLOM_TRY((gemm_sq_nn(W3, Ue, Me, N, bi, 1, st)));
+      PLOM_TRY((gemm_df_nn(W3, Ue, Me, N, bi, 1, st)));
       PLOM_TRY(embed_to_rowform(Me, F, n, bi, st));
     } else {
-      PLOM_TRY((gemm_sq_nn(W3, Ur, Me, N, bi, 1, st)));
+      PLOM_TRY((gemm_df_nn(W3, Ur, Me, N, bi, 1, st)));
       Mop = Me;
     }
   }
