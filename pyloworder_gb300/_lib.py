@@ -223,7 +223,8 @@ def rows_ld(x):
     if x.dim() != 2:
         return None
     if x.shape[1] <= 1:
-        return max(1, x.shape[1]) if x.stride(0) >= x.shape[1] or x.shape[0] <= 1 else None
+        # one column: the row stride is the pitch (a column of a wider matrix)
+        return max(1, x.shape[1], x.stride(0) if x.shape[0] > 1 else 1)
     if x.stride(1) != 1:
         return None
     return x.stride(0)
