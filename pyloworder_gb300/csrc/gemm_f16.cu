@@ -391,22 +391,33 @@ __global__ void __launch_bounds__(256) split_w16_kernel(const double* __restrict
                                                         float out_scale, __half* __restrict__ bhi,
                                                         __half* __restrict__ blo,
                                                         float* __restrict__ f, int64_t wstride,
-                                                        int fstride) {
+                                                        int fstride, int fold) {
+  // fold > 0: two copies of W on the diagonal, column j of copy h in row
+  // h fold + j of Bt at K offset 64 h (ldk = 128, s_in of 64)
   __shared__ double red[8];
   // problem blockIdx.y of a batch: W_p, its input scales, its rows of Bt, its factors
   {
     const int64_t pb = blockIdx.y;
     W += pb * wstride;
-    s_in += pb * ldk;
-    bhi += pb * k * (int64_t)ldk;
-    blo += pb * k * (int64_t)ldk;
+    s_in += pb * (fold ? 64 : ldk);
+    const int64_t rows = fold ? 2 * fold : k;
+    bhi += pb * rows * (int64_t)ldk;
+    blo += pb * rows * (int64_t)ldk;
     f += pb * fstride;
   }
-  const int j = blockIdx.x;
+  const int row = blockIdx.x;
+  const int half = fold && row >= fold ? 1 : 0;
+  const int j = row - half * fold;
   if (j >= k) {
-    if (threadIdx.x == 0) f[j] = 0.f;
+    if (threadIdx.x == 0) f[row] = 0.f;
+    if (fold && row < 2 * fold)  // a padding column of the packed output
+      for (int i = threadIdx.x; i < ldk; i += blockDim.x) {
+        bhi[(int64_t)row * ldk + i] = __float2half_rn(0.f);
+        blo[(int64_t)row * ldk + i] = __float2half_rn(0.f);
+      }
     return;
   }
+  const int koff = 64 * half;
   // 1 / s_in is exact (powers of two)
   double mx = 0.0;
   for (int i = threadIdx.x; i < nin; i += blockDim.x)
@@ -420,14 +431,15 @@ __global__ void __launch_bounds__(256) split_w16_kernel(const double* __restrict
   frexp(mx, &e);
   e = e < -900 ? -900 : (e > 900 ? 900 : e);
   const double t = (mx > 0.0) ? ldexp(1.0, PK_LOG2 - e) : 1.0;
-  for (int i = threadIdx.x; i < ldk; i += blockDim.x) {
-    const float x = (i < nin) ? (float)(W[(int64_t)i * ldw + j] * (double)(1.0f / s_in[i]) * t) : 0.f;
+  for (int kk = threadIdx.x; kk < ldk; kk += blockDim.x) {
+    const int i = kk - koff;
+    const float x = (i >= 0 && i < nin) ? (float)(W[(int64_t)i * ldw + j] * (double)(1.0f / s_in[i]) * t) : 0.f;
     const __half h = __float2half_rn(x);
     const __half l = __float2half_rn(x - __half2float(h));
-    bhi[(int64_t)j * ldk + i] = h;
-    blo[(int64_t)j * ldk + i] = l;
+    bhi[(int64_t)row * ldk + kk] = h;
+    blo[(int64_t)row * ldk + kk] = l;
   }
-  if (threadIdx.x == 0) f[j] = (float)((double)out_scale / t);
+  if (threadIdx.x == 0) f[row] = (float)((double)out_scale / t);
 }
 
 // ---------------------------------------------------------------------------
@@ -762,7 +774,7 @@ __global__ void tn16_reduce_kernel(const double* __restrict__ part, int Na, int 
 constexpr int GR_WARPS = 16;
 __global__ void __launch_bounds__(32 * GR_WARPS) gram16_reduce_kernel(
     const double* __restrict__ part, int N, int tn, int chunks, const float* __restrict__ s,
-    double* __restrict__ G, int batch, int ld, int accumulate) {
+    double* __restrict__ G, int batch, int ld, int accumulate, int fold) {
   __shared__ float2 red[GR_WARPS][32];
   const int ntiles = tn * (tn + 1) / 2;
   const int cblk = (N + 31) / 32;
@@ -779,8 +791,16 @@ __global__ void __launch_bounds__(32 * GR_WARPS) gram16_reduce_kernel(
                       ((pb * ntiles + tile) * chunks) * 128 * 128 + (int64_t)(i - ti * 128) * 128 +
                       (j - tj * 128);
     float2 acc = make_float2(0.f, 0.f);
+    if (fold) {  // the diagonal blocks of the even and of the odd rows
+#pragma unroll 2
+      for (int c = warp; c < chunks; c += GR_WARPS) {
+        const float2* q = p + (int64_t)c * 128 * 128;
+        acc = dw_add(dw_add(acc, q[0]), q[64 * 128 + 64]);
+      }
+    } else {
 #pragma unroll 4
-    for (int c = warp; c < chunks; c += GR_WARPS) acc = dw_add(acc, p[(int64_t)c * 128 * 128]);
+      for (int c = warp; c < chunks; c += GR_WARPS) acc = dw_add(acc, p[(int64_t)c * 128 * 128]);
+    }
     red[warp][lane] = acc;
     __syncthreads();
     if (warp == 0 && j < N && j >= i) {
@@ -1288,6 +1308,7 @@ struct ApplyOut {
   __half* ohi;     // packed output planes (m x ldo) or nullptr
   __half* olo;
   int ldo;
+  int klast;       // columns of the last row (folded rows of an odd m: one half)
 };
 
 // one 32-column group of an apply tile (FP32 or packed output) through the
@@ -1330,16 +1351,17 @@ __device__ __forceinline__ void apply_store_chunk(const float (&v)[32], int col0
     const int64_t r = row0 + rr;
     if (out.C) {
       const int c = col0 + 4 * q;
-      if (r < m && c < k) {
+      const int kr = r == m - 1 ? out.klast : k;
+      if (r < m && c < kr) {
         float* dst = out.C + pb * out.cstride + r * out.ldc + c;
-        if (c_vec && c + 4 <= k) {
+        if (c_vec && c + 4 <= kr) {
           *reinterpret_cast<uint4*>(dst) = val;
         } else {
           const float w4[4] = {__uint_as_float(val.x), __uint_as_float(val.y),
                                __uint_as_float(val.z), __uint_as_float(val.w)};
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            if (c + e < k) dst[e] = w4[e];
+            if (c + e < kr) dst[e] = w4[e];
         }
       }
     } else if (r < mp) {
@@ -2187,16 +2209,28 @@ static int pair_clusters() {
   return n;
 }
 
-// rows per problem in the planes: m for one problem; for a batch, m rounded
+// rows per problem in the planes: m for one problem (even when ld = 64, so
+// that two rows can be read as one of 128, see fold2); for a batch, m rounded
 // up to 128 so that no stage or output tile of one problem reaches the next
-int64_t packed_rows(int64_t m, int64_t batch) { return batch > 1 ? cdiv(m, 128) * 128 : m; }
+int64_t packed_rows(int64_t m, int64_t batch, int64_t ld) {
+  return batch > 1 ? cdiv(m, 128) * 128 : ld == 64 ? m + (m & 1) : m;
+}
+
+// Operands of at most 64 columns (ld = 64) fill half of a 128-column tile.
+// Their planes, row-major m x 64, are read as (m / 2) x 128: rows 2 r and
+// 2 r + 1 side by side.  A Gram then is the sum of the two 64 x 64 diagonal
+// blocks of the 128 x 128 product, and Y W is the product with diag(W, W).
+// Stages, tensor products, TMEM drains and epilogue warps all carry twice the
+// rows at the same cost.
+static bool fold2(const Packed& p) { return p.ld == 64 && (p.mp & 1) == 0; }
 
 void packed_carve(Arena& ws, Packed& p, int64_t m, int64_t N, int64_t batch) {
   p.m = m;
   p.N = N;
   p.ld = packed_ld(N);
   p.batch = batch;
-  p.mp = packed_rows(m, batch);
+  p.mp = packed_rows(m, batch, p.ld);
+  p.pstride = batch * p.mp * p.ld;
   p.hi = ws.take<__half>((size_t)(2 * batch * p.mp * p.ld));
   p.lo = p.hi ? p.hi + batch * p.mp * p.ld : nullptr;
   p.scale = ws.take<float>((size_t)(batch * p.ld));
@@ -2219,7 +2253,8 @@ void packed_view(Packed& p, void* storage, int64_t m, int64_t N, float* scale, i
   p.N = N;
   p.ld = packed_ld(N);
   p.batch = batch;
-  p.mp = packed_rows(m, batch);
+  p.mp = packed_rows(m, batch, p.ld);
+  p.pstride = batch * p.mp * p.ld;
   p.hi = static_cast<__half*>(storage);
   p.lo = p.hi ? p.hi + batch * p.mp * p.ld : nullptr;
   p.scale = scale;
@@ -2393,7 +2428,10 @@ int gram_packed_chunks(const Packed& p, int C, int64_t mc, const float* scales, 
 int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st,
                 bool accumulate) {
   if (p.ld > 128) return gram_packed_wide(p, G, err, ws, st, accumulate);
-  const int64_t m = p.m, N = p.N, batch = p.batch;
+  const int64_t N = p.N, batch = p.batch;
+  const bool fold = fold2(p);
+  const int64_t m = fold ? cdiv(p.m, 2) : p.m;  // (folded) rows
+  const int64_t mp = fold ? p.mp / 2 : p.mp, ld = fold ? 128 : p.ld;
   const int tn = (int)cdiv(p.ld, 128);
   const int tiles = tn * (tn + 1) / 2;
   const int chunks = gram16_chunks(m, (int)std::min<int64_t>(tiles * batch, 1 << 20));
@@ -2417,17 +2455,17 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
     attr = true;
   }
   CUtensorMap tm;
-  PLOM_REQUIRE(make_map_planes(&tm, p.hi, (uint64_t)p.ld, (uint64_t)(batch * p.mp),
-                               (uint64_t)p.ld, 64, hp::G_BK, (uint64_t)p.pstride),
+  PLOM_REQUIRE(make_map_planes(&tm, p.hi, (uint64_t)ld, (uint64_t)(batch * mp), (uint64_t)ld, 64,
+                               hp::G_BK, (uint64_t)p.pstride),
                PLOM_ERR_CUDA, "gram16: tensor map encoding failed");
-  ProfScope prof_g("tc_gram_f16x3", st, (double)m * N * N * batch, 4.0 * (double)m * p.ld * batch);
+  ProfScope prof_g("tc_gram_f16x3", st, (double)p.m * N * N * batch, 4.0 * (double)p.m * p.ld * batch);
   hp::gram16_kernel<true><<<(unsigned)(batch * tiles * chunks_eff), 320, hp::G_SMEM, st>>>(
-      tm, tm, m, tn, tn, rpc, chunks_eff, part, err, p.mp);
+      tm, tm, m, tn, tn, rpc, chunks_eff, part, err, mp);
   PLOM_CHECK_LAUNCH();
   const int blocks = (int)std::min<int64_t>(batch * N * cdiv(N, 32), (int64_t)num_sms() * 4);
   ProfScope prof_r("gram_reduce", st, 0.0, 8.0 * (double)batch * tiles * chunks_eff * 128 * 128);
   hp::gram16_reduce_kernel<<<blocks, 32 * hp::GR_WARPS, 0, st>>>(part, (int)N, tn, chunks_eff, p.scale, G,
-                                                   (int)batch, (int)p.ld, accumulate ? 1 : 0);
+                                                   (int)batch, (int)p.ld, accumulate ? 1 : 0, fold ? 1 : 0);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
 }
@@ -2523,8 +2561,15 @@ int tn_packed(const Packed& a, const Packed& b, double* C, int64_t ldc, int* err
 int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float* C, int64_t ldc,
                  Packed* out, int* err, Arena& ws, cudaStream_t st, int64_t wstride,
                  int64_t cstride, bool upper) {
-  const int64_t m = p.m, batch = p.batch;
-  const int64_t ldk = p.ld;  // K extent of the W copies (= packed pitch of the input)
+  const int64_t batch = p.batch;
+  // two rows per 128-column tile row (see fold2) when the output folds too:
+  // packed planes of 64 columns, or dense FP32 rows
+  const bool fold = fold2(p) && k <= 64 && (out ? out->ld == 64 : ldc == k);
+  const int64_t kh = out ? 64 : k;             // (folded) output columns of one row
+  const int64_t m = fold ? cdiv(p.m, 2) : p.m; // (folded) rows
+  const int64_t mp = fold ? p.mp / 2 : p.mp, lda = fold ? 128 : p.ld;
+  const int64_t ldk = lda;  // K extent of the W copies (= packed pitch of the input)
+  const int64_t kf = fold ? 2 * kh : k;        // columns of the product
   // output tile width (see ApplyCfg): 256 for dense W wider than 128 columns.
   // An upper-triangular W keeps 128-wide tiles: its short column tiles (the
   // first K blocks only) finish their products faster than the single
@@ -2542,19 +2587,22 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
                                                                                       : 0;
   const bool pair = pair_tn != 0;
   const int TN = pair ? pair_tn : (k > 128 && !tri_w) ? tuning().apply_dense_tn : 128;
-  const int64_t col_tiles = cdiv(k, TN);
+  const int64_t col_tiles = cdiv(kf, TN);
   const int fstride = (int)(col_tiles * TN);
-  __half* bhi = ws.take<__half>((size_t)(2 * batch * k * ldk));
-  __half* blo = bhi ? bhi + batch * k * ldk : nullptr;
+  // (what folds is decided by the strides of the call too: room for both)
+  const bool may_fold = p.ld == 64 && k <= 64;
+  const int64_t wk = may_fold ? 128 * 128 : kf * ldk;
+  __half* bhi = ws.take<__half>((size_t)(2 * batch * wk));
+  __half* blo = bhi ? bhi + batch * kf * ldk : nullptr;
   float* f = ws.take<float>((size_t)(batch * fstride));
   if (ws.measuring()) return PLOM_OK;
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "apply16: workspace too small");
   PLOM_REQUIRE(p.hi && W && (C || out) && m >= 1 && batch * p.mp < (1ll << 31) && k >= 1 &&
                    batch * k < (1ll << 31),
                PLOM_ERR_ARG, "apply16: bad arguments");
-  PLOM_REQUIRE(batch == 1 || ((wstride == 0 || wstride >= p.N * ldw) && (out || cstride >= m * ldc)),
+  PLOM_REQUIRE(batch == 1 || ((wstride == 0 || wstride >= p.N * ldw) && (out || cstride >= p.m * ldc)),
                PLOM_ERR_ARG, "apply16: batch strides too small");
-  if (out) PLOM_REQUIRE(out->hi && out->scale && out->m == m && out->N == k && out->batch == batch &&
+  if (out) PLOM_REQUIRE(out->hi && out->scale && out->m == p.m && out->N == k && out->batch == batch &&
                             out->mp == p.mp,
                         PLOM_ERR_ARG, "apply16: bad packed output");
   static bool attr = false;
@@ -2569,7 +2617,8 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   }
   const float out_scale = out ? (float)(1 << hp::PK_LOG2) : 1.0f;
   hp::split_w16_kernel<<<dim3((unsigned)fstride, (unsigned)batch), 256, 0, st>>>(
-      W, ldw, (int)p.N, (int)k, (int)ldk, p.scale, out_scale, bhi, blo, f, wstride, fstride);
+      W, ldw, (int)p.N, (int)k, (int)ldk, p.scale, out_scale, bhi, blo, f, wstride, fstride,
+      fold ? (int)kh : 0);
   PLOM_CHECK_LAUNCH();
   if (out) {
     // packed output columns carry the fixed scale 2^14
@@ -2584,12 +2633,12 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
                 "pair tiles use the single-SM kernels' K depth");
   // B boxes: TN rows of W (single SM, in boxes of 128) or the CTA's half (pair)
   const uint32_t b_rows = pair ? (uint32_t)(TN / 2) : 128u;
-  PLOM_REQUIRE(make_map_planes(&tmA, p.hi, (uint64_t)p.ld, (uint64_t)(batch * p.mp),
-                               (uint64_t)p.ld, bk, 128, (uint64_t)p.pstride, bk == 32) &&
-                   make_map_planes(&tmB, bhi, (uint64_t)ldk, (uint64_t)(batch * k), (uint64_t)ldk,
+  PLOM_REQUIRE(make_map_planes(&tmA, p.hi, (uint64_t)lda, (uint64_t)(batch * mp), (uint64_t)lda,
+                               bk, 128, (uint64_t)p.pstride, bk == 32) &&
+                   make_map_planes(&tmB, bhi, (uint64_t)ldk, (uint64_t)(batch * kf), (uint64_t)ldk,
                                    bk, b_rows, 0, bk == 32),
                PLOM_ERR_CUDA, "apply16: tensor map encoding failed");
-  const int64_t row_tiles = cdiv(p.mp, 128);
+  const int64_t row_tiles = cdiv(mp, 128);
   const int64_t tiles = batch * row_tiles * col_tiles;
   // whole row blocks per CTA pay for the triangular case (column tiles of very
   // different lengths; interleaved single tiles measured 10 % slower there);
@@ -2602,17 +2651,18 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   const int grid = (int)std::min<int64_t>(by_rows ? batch * row_tiles : tiles, num_sms());
   hp::ApplyOut o;
   o.C = out ? nullptr : C;
-  o.ldc = ldc;
+  o.ldc = fold ? 2 * ldc : ldc;
   o.cstride = cstride;
+  o.klast = (int)(fold && (p.m & 1) ? k : kf);
   o.ohi = out ? out->hi : nullptr;
   o.olo = out ? out->lo : nullptr;
-  o.ldo = out ? (int)out->ld : 0;
+  o.ldo = out ? (int)(fold ? 128 : out->ld) : 0;
   // an upper-triangular W (k = N) needs m N (N + 1) flops: row i of W meets
   // columns j >= i only
   const bool tri = tri_w;
-  const double flops = tri ? (double)m * p.N * (p.N + 1) * batch : 2.0 * m * p.N * k * batch;
+  const double flops = tri ? (double)p.m * p.N * (p.N + 1) * batch : 2.0 * p.m * p.N * k * batch;
   ProfScope prof(pair ? "tc_apply_f16x3_pair" : "tc_apply_f16x3", st, flops,
-                 4.0 * ((double)m * p.ld + (double)m * k) * batch);
+                 4.0 * ((double)p.m * p.ld + (double)p.m * k) * batch);
   if (pair) {
     const int clusters_max = TN == 256 ? pair_clusters<256>() : pair_clusters<128>();
     const int64_t pairs = cdiv(p.mp, 256), ptiles = pairs * col_tiles;
@@ -2648,7 +2698,7 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
         row_tiles, fstride, tri ? 1 : 0, by_rows);
   else
     hp::apply16_kernel<128><<<grid, hp::ApplyWarps<128>::THREADS, hp::apply_smem<128>(), st>>>(
-        tmA, tmB, m, (int)(ldk / 64), (int)k, col_tiles, tiles, f, o, err, p.mp, row_tiles,
+        tmA, tmB, m, (int)(ldk / 64), (int)kf, col_tiles, tiles, f, o, err, mp, row_tiles,
         fstride, tri ? 1 : 0, by_rows);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;

@@ -12,8 +12,8 @@ namespace plom {
 //   hi + lo = Y diag(scale), hi and lo row-major (batch x mp) x ld (ld = N
 //   rounded up to 64, padding columns zero; lo right after hi), scale[p][j]
 //   a power of two per problem and column.  A batch holds `batch` problems
-//   of m rows each, mp rows apart (mp = m for one problem, else m rounded up
-//   to 128 with zero padding rows).
+//   of m rows each, mp rows apart (one problem: mp = m, rounded up to even when
+//   ld = 64; else m rounded up to 128; the padding rows are zero).
 struct Packed {
   __half* hi;
   __half* lo;
@@ -26,7 +26,7 @@ struct Packed {
 // (planes and plane stride of the parent; scales as given)
 Packed packed_rows_view(const Packed& p, int64_t r0, int64_t rows, int64_t mp, float* scale);
 int64_t packed_ld(int64_t N);
-int64_t packed_rows(int64_t m, int64_t batch);
+int64_t packed_rows(int64_t m, int64_t batch, int64_t ld);
 // carve planes and scales from the workspace
 void packed_carve(Arena& ws, Packed& p, int64_t m, int64_t N, int64_t batch = 1);
 // planes in caller storage of 4 batch packed_rows(m) packed_ld(N) bytes, scales in `scale`

@@ -416,9 +416,12 @@ static int cholqr3_packed(bool cplx, const float* X, int64_t m, int n, int64_t l
   return PLOM_OK;
 }
 
-// P1 may live in a float output buffer of m rows x ld floats when ld covers
-// the packed pitch (4 m packed_ld(N) bytes)
-static bool p1_fits(int64_t ld_floats, int N) { return ld_floats >= packed_ld(N); }
+// P1 may live in a float output buffer of m rows x ld floats when that covers
+// its planes (4 packed_rows(m) packed_ld(N) bytes)
+static bool p1_fits(int64_t m, int64_t ld_floats, int N) {
+  const int64_t ld = packed_ld(N);
+  return ld_floats >= ld && m * ld_floats >= packed_rows(m, 1, ld) * ld;
+}
 
 // svd(Re) = Ur S V^T and U = Q2 (R3^-1 Ur) into the first m rows of U (ldu),
 // S, VT, after the CholeskyQR3 passes (b.P2, b.W3, b.Re)
@@ -483,7 +486,7 @@ static int tsqr_svd_packed(bool cplx, const float* X, int64_t m, int n, int64_t 
                            cudaStream_t st) {
   const int N = cplx ? 2 * n : n;
   PackedCore b;
-  carve_packed_core(ws, b, m, N, p1_fits(ldu, N), U);
+  carve_packed_core(ws, b, m, N, p1_fits(m, ldu, N), U);
   if (!ws.measuring())
     PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "tsqr_svd: workspace too small (%zu > %zu)",
                  ws.off, ws.cap);
@@ -609,7 +612,7 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
 static int tsqr_packed(const float* X, int64_t m, int n, int64_t ldx, float* Q, int64_t ldq,
                        float* R, int* info, Arena& ws, cudaStream_t st, bool hh = false) {
   PackedCore b;
-  carve_packed_core(ws, b, m, n, p1_fits(ldq, n), Q);
+  carve_packed_core(ws, b, m, n, p1_fits(m, ldq, n), Q);
   if (!ws.measuring()) PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "tsqr: workspace too small");
   const size_t mark = ws.off;
   PLOM_TRY(cholqr3_packed(false, X, m, n, ldx, b, info, ws, st));
