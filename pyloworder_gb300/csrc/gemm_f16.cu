@@ -2314,6 +2314,21 @@ static int gram16_chunks(int64_t m, int tiles, int bk = hp::G_BK, int wave_mult 
   return (int)std::max<int64_t>(1, std::min<int64_t>(maxc, cdiv(2 * sms, tiles)));
 }
 
+// row chunks of the narrow kernel (tiles: of all problems): whole waves of
+// CTAs, gram_wave_mult of them while a chunk keeps 16 stages or more, else
+// fewer.  A CTA costs ~5 us besides its stages (barriers, TMEM, the drain of
+// its slab), so 17 problems of 10,006 folded rows in 1,343 chunks of two
+// stages took 135 us, in 136 of twenty 40 us.
+static int gram16_narrow_chunks(int64_t m, int64_t tiles) {
+  const int64_t sms = num_sms();
+  int64_t c = 1;
+  for (int64_t mult = std::max(1, tuning().gram_wave_mult);; mult /= 2) {
+    c = std::max<int64_t>(1, sms * mult / tiles);
+    if (mult <= 1 || m / c >= 16 * hp::G_BK) break;
+  }
+  return (int)std::min<int64_t>(c, std::max<int64_t>(1, cdiv(m, 4 * hp::G_BK)));
+}
+
 // Gram of operands wider than 128 columns: 128 x 256 tiles (gram16w_kernel);
 // row chunks are whole 4,096-row sub-chunks, each with its own FP32 slab.
 // Short chunks keep the tiles of one chunk that run at the same time close
@@ -2434,7 +2449,7 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
   const int64_t mp = fold ? p.mp / 2 : p.mp, ld = fold ? 128 : p.ld;
   const int tn = (int)cdiv(p.ld, 128);
   const int tiles = tn * (tn + 1) / 2;
-  const int chunks = gram16_chunks(m, (int)std::min<int64_t>(tiles * batch, 1 << 20));
+  const int chunks = gram16_narrow_chunks(m, tiles * batch);
   int64_t rpc = cdiv(m, chunks);
   rpc = cdiv(rpc, hp::G_BK) * hp::G_BK;  // chunk boundaries on stage boundaries
   const int chunks_eff = (int)std::max<int64_t>(1, cdiv(m, rpc));
@@ -2520,7 +2535,7 @@ int tn_packed(const Packed& a, const Packed& b, double* C, int64_t ldc, int* err
   const int64_t m = a.m;
   const int tna = (int)cdiv(a.ld, 128), tnb = (int)cdiv(b.ld, 128);
   const int tiles = tna * tnb;
-  const int chunks = gram16_chunks(m, tiles);
+  const int chunks = gram16_narrow_chunks(m, tiles);
   int64_t rpc = cdiv(m, chunks);
   rpc = cdiv(rpc, hp::G_BK) * hp::G_BK;
   const int chunks_eff = (int)std::max<int64_t>(1, cdiv(m, rpc));
