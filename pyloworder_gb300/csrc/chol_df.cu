@@ -568,42 +568,50 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
 }
 
 // ---------------------------------------------------------------------------
-// C = A B for n x n FP64 operands in double-float arithmetic (R3 R2 R1 and
-// R3^-1 Ur of the mixed form): a 32 x 32 tile per CTA, the next pair of blocks
-// in flight while one is multiplied.  tri bit 0: A upper triangular, bit 1: B
-// upper triangular (zero blocks are skipped; B is then scaled by the power of
-// two of its largest diagonal entry, so that a factor of data of any FP32
-// magnitude fits).  An FP64 multiply-add issues at 2 lanes a clock and SM: one
-// 32 x 32 x 32 block took 14 us, here 3.
+// n x n products of the mixed form, FP64 operands, a 32 x 32 tile per CTA, the
+// next pair of blocks in flight while one is multiplied.  F32 = false: C = A B in
+// double-float arithmetic (R3 R2 R1, R3^-1 Ur); F32 = true: C = A B or Cin - A B
+// with FP32 products (corrections at the 1e-7 level of C).  tri bit 0: A upper
+// triangular, bit 1: B upper triangular (zero blocks are skipped).  D (or null):
+// s is the power of two that brings D's largest diagonal entry next to 1; A is
+// scaled by s^ea and B by s^eb, so that factors of data of any FP32 magnitude
+// fit.  An FP64 multiply-add issues at 2 lanes a clock and SM: one 32 x 32 x 32
+// block took 14 us on the FP64 pipe, 3 us in double-float arithmetic.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ int cd_diag_exponent(const double* D, int n, int* sh) {
+  if (threadIdx.x == 0) *sh = 0;
+  __syncthreads();
+  int ex = 0;
+  for (int i = threadIdx.x; i < n; i += CD_THREADS)
+    ex = max(ex, (int)((uint64_t)__double_as_longlong(D[(int64_t)i * n + i]) >> 52) & 0x7ff);
+  ex = warp_max(ex);
+  if ((threadIdx.x & 31) == 0) atomicMax(sh, ex);
+  __syncthreads();
+  const int e = *sh;
+  return (e > 0 && e < 0x7ff) ? 1023 - e : 0;
+}
+
+template <bool F32>
 __global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __restrict__ A,
                                                              const double* __restrict__ B,
-                                                             double* __restrict__ C, int n,
-                                                             int tri) {
+                                                             const double* __restrict__ Cin,
+                                                             double* __restrict__ C, int n, int tri,
+                                                             const double* __restrict__ D, int ea,
+                                                             int eb) {
   __shared__ __align__(16) float2 As[CB][CPITCH];  // [k][row of A]
   __shared__ __align__(16) float2 Bs[CB][CPITCH];
   __shared__ int ex_sh;
   const int tid = threadIdx.x;
-  const int64_t nn = (int64_t)n * n;
-  A += blockIdx.z * nn;
-  B += blockIdx.z * nn;
-  C += blockIdx.z * nn;
+  const int64_t off = (int64_t)blockIdx.z * n * n;
+  A += off;
+  B += off;
+  C += off;
   const int bi = blockIdx.y, bj = blockIdx.x;
-  int sb = 0;
-  if (tri & 2) {
-    if (tid == 0) ex_sh = 0;
-    __syncthreads();
-    int ex = 0;
-    for (int i = tid; i < n; i += CD_THREADS)
-      ex = max(ex, (int)((uint64_t)__double_as_longlong(B[(int64_t)i * n + i]) >> 52) & 0x7ff);
-    ex = warp_max(ex);
-    if ((tid & 31) == 0) atomicMax(&ex_sh, ex);
-    __syncthreads();
-    sb = (ex_sh > 0 && ex_sh < 0x7ff) ? 1023 - ex_sh : 0;
-  }
+  const int s = D ? cd_diag_exponent(D + off, n, &ex_sh) : 0;
   const int T = (n + CB - 1) / CB;
   const int k0 = (tri & 1) ? bi : 0, k1 = (tri & 2) ? bj : T - 1;
   const int c = tid & 31, r = tid >> 5;  // rows r, r + 8, ...
+  const int ty = tid >> 4, tx = tid & 15;
   float2 acc[2][2];
   acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = make_float2(0.f, 0.f);
   double va[4], vb[4];
@@ -621,36 +629,192 @@ __global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __res
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      As[c][r + 8 * u] = cd_split(va[u], 0);
-      Bs[r + 8 * u][c] = cd_split(vb[u], sb);
+      As[c][r + 8 * u] = cd_split(va[u], ea * s);
+      Bs[r + 8 * u][c] = cd_split(vb[u], eb * s);
     }
     __syncthreads();
     if (k < k1) fetch(k + 1);
-    float2 m[2][2];
-    cd_mm(As, Bs, m);
+    if constexpr (F32) {
+#pragma unroll 8
+      for (int q = 0; q < CB; ++q) {
+        const float4 a = *reinterpret_cast<const float4*>(&As[q][2 * ty]);
+        const float4 b = *reinterpret_cast<const float4*>(&Bs[q][2 * tx]);
+        acc[0][0].x = fmaf(a.x, b.x, acc[0][0].x);
+        acc[0][1].x = fmaf(a.x, b.z, acc[0][1].x);
+        acc[1][0].x = fmaf(a.z, b.x, acc[1][0].x);
+        acc[1][1].x = fmaf(a.z, b.z, acc[1][1].x);
+      }
+    } else {
+      float2 m[2][2];
+      cd_mm(As, Bs, m);
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int v = 0; v < 2; ++v) acc[u][v] = df_add2(acc[u][v], m[u][v]);
+        for (int v = 0; v < 2; ++v) acc[u][v] = df_add2(acc[u][v], m[u][v]);
+    }
   }
-  const int ty = tid >> 4, tx = tid & 15;
 #pragma unroll
   for (int u = 0; u < 2; ++u)
 #pragma unroll
     for (int v = 0; v < 2; ++v) {
       const int i = bi * CB + 2 * ty + u, j = bj * CB + 2 * tx + v;
-      if (i < n && j < n) C[(int64_t)i * n + j] = cd_join(acc[u][v], -sb);
+      if (i >= n || j >= n) continue;
+      double x = cd_join(acc[u][v], -(ea + eb) * s);
+      if (Cin) x = Cin[off + (int64_t)i * n + j] - x;
+      C[(int64_t)i * n + j] = x;
     }
 }
 
-int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
-               cudaStream_t st) {
+static int gemm_df_launch(bool f32, const double* A, const double* B, const double* Cin, double* C,
+                          int n, int batch, int tri, const double* D, int ea, int eb,
+                          cudaStream_t st) {
   if (n <= 0 || batch <= 0) return PLOM_OK;
   PLOM_REQUIRE(A && B && C && batch <= 65535, PLOM_ERR_ARG, "gemm_df: bad arguments");
   ProfScope prof("gemm_df", st, 2.0 * n * n * n * batch, 24.0 * n * n * batch);
   const unsigned T = (unsigned)cdiv(n, CB);
-  gemm_df_kernel<<<dim3(T, T, (unsigned)batch), CD_THREADS, 0, st>>>(A, B, C, n, tri);
+  const dim3 grid(T, T, (unsigned)batch);
+  if (f32)
+    gemm_df_kernel<true><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb);
+  else
+    gemm_df_kernel<false><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb);
   PLOM_CHECK_LAUNCH();
+  return PLOM_OK;
+}
+
+int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
+               cudaStream_t st) {
+  return gemm_df_launch(false, A, B, nullptr, C, n, batch, tri, (tri & 2) ? B : nullptr, 0, 1, st);
+}
+
+// Re = R3 R2' R1' for at most 64 columns in one launch, one CTA per problem:
+// R' = R - R (dW R) with FP32 products, then two double-float products.  Five
+// launches of the tile kernel cost 25 us there.
+__global__ void __launch_bounds__(CD_THREADS) re_chain_kernel(const double* __restrict__ R1,
+                                                              const double* __restrict__ dW1,
+                                                              const double* __restrict__ R2,
+                                                              const double* __restrict__ dW2,
+                                                              const double* __restrict__ R3,
+                                                              double* __restrict__ Re, int n) {
+  constexpr int MP = 2 * CB + 2;  // pitch of a 64 x 64 float2 matrix (16-byte aligned rows)
+  extern __shared__ __align__(16) float2 rc_sh[];
+  __shared__ int ex_sh;
+  float2(*X)[MP] = reinterpret_cast<float2(*)[MP]>(rc_sh);                // a factor
+  float2(*Y)[MP] = reinterpret_cast<float2(*)[MP]>(rc_sh + 2 * CB * MP);  // the running product
+  float2(*E)[MP] = reinterpret_cast<float2(*)[MP]>(rc_sh + 4 * CB * MP);  // scratch
+  const int tid = threadIdx.x, T = (n + CB - 1) / CB, np = T * CB;
+  const int64_t off = (int64_t)blockIdx.x * n * n;
+  const int ty = tid >> 4, tx = tid & 15;
+  auto load = [&](float2(*M)[MP], const double* src, int s) {
+    for (int e = tid; e < np * np; e += CD_THREADS) {
+      const int i = e / np, j = e % np;
+      M[i][j] = (i < n && j < n && i <= j) ? cd_split(src[off + (int64_t)i * n + j], s)
+                                           : make_float2(0.f, 0.f);
+    }
+  };
+  // the elements of a tile of this thread: rows 2 ty + u, columns 2 tx + v
+  auto mul32 = [&](float2(*A)[MP], float2(*B)[MP], int a, int c, float (&m)[2][2]) {
+    m[0][0] = m[0][1] = m[1][0] = m[1][1] = 0.f;
+    for (int k = a * CB; k < (c + 1) * CB; ++k) {
+      const float a0 = A[a * CB + 2 * ty][k].x, a1 = A[a * CB + 2 * ty + 1][k].x;
+      const float b0 = B[k][c * CB + 2 * tx].x, b1 = B[k][c * CB + 2 * tx + 1].x;
+      m[0][0] = fmaf(a0, b0, m[0][0]);
+      m[0][1] = fmaf(a0, b1, m[0][1]);
+      m[1][0] = fmaf(a1, b0, m[1][0]);
+      m[1][1] = fmaf(a1, b1, m[1][1]);
+    }
+  };
+  // X <- X - X (dW X) for the factor R with rounding dW (through E); X scaled by
+  // 2^s, dW by 2^-s
+  auto corrected = [&](const double* R, const double* dW, int s) {
+    load(X, R, s);
+    load(E, dW, -s);
+    __syncthreads();
+    float m[3][2][2];
+    int t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c) mul32(E, X, a, c, m[t++]);
+    __syncthreads();
+    t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c, ++t)
+        for (int u = 0; u < 2; ++u)
+          for (int v = 0; v < 2; ++v)
+            E[a * CB + 2 * ty + u][c * CB + 2 * tx + v] = make_float2(m[t][u][v], 0.f);
+    __syncthreads();
+    t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c) mul32(X, E, a, c, m[t++]);
+    __syncthreads();
+    t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c, ++t)
+        for (int u = 0; u < 2; ++u)
+          for (int v = 0; v < 2; ++v) {
+            float2& x = X[a * CB + 2 * ty + u][c * CB + 2 * tx + v];
+            x = df_add2(x, make_float2(-m[t][u][v], 0.f));
+          }
+    __syncthreads();
+  };
+  // Y <- Y X
+  auto times = [&]() {
+    float2 m[3][2][2];
+    int t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c, ++t) {
+        for (int u = 0; u < 2; ++u)
+          for (int v = 0; v < 2; ++v) m[t][u][v] = make_float2(0.f, 0.f);
+        for (int k = a * CB; k < (c + 1) * CB; ++k) {
+          const float2 a0 = Y[a * CB + 2 * ty][k], a1 = Y[a * CB + 2 * ty + 1][k];
+          const float4 b = *reinterpret_cast<const float4*>(&X[k][c * CB + 2 * tx]);
+          const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+          df_dot_acc(m[t][0][0], a0, b0);
+          df_dot_acc(m[t][0][1], a0, b1);
+          df_dot_acc(m[t][1][0], a1, b0);
+          df_dot_acc(m[t][1][1], a1, b1);
+        }
+      }
+    __syncthreads();
+    t = 0;
+    for (int a = 0; a < T; ++a)
+      for (int c = a; c < T; ++c, ++t)
+        for (int u = 0; u < 2; ++u)
+          for (int v = 0; v < 2; ++v)
+            Y[a * CB + 2 * ty + u][c * CB + 2 * tx + v] = fast_two_sum(m[t][u][v].x, m[t][u][v].y);
+    __syncthreads();
+  };
+  const int s1 = cd_diag_exponent(R1 + off, n, &ex_sh);
+  load(Y, R3, 0);
+  corrected(R2, dW2, 0);
+  times();
+  corrected(R1, dW1, s1);
+  times();
+  for (int e = tid; e < n * n; e += CD_THREADS) {
+    const int i = e / n, j = e % n;
+    Re[off + e] = i <= j ? cd_join(Y[i][j], -s1) : 0.0;
+  }
+}
+
+int re_chain(const double* R1, const double* dW1, const double* R2, const double* dW2,
+             const double* R3, double* Re, double* T1, double* T2, int n, int batch,
+             cudaStream_t st) {
+  PLOM_REQUIRE(R1 && dW1 && R2 && dW2 && R3 && Re && T1 && T2, PLOM_ERR_ARG, "re_chain: null pointer");
+  if (n <= 2 * CB) {
+    const size_t smem = (size_t)3 * 2 * CB * (2 * CB + 2) * sizeof(float2);
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(re_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem));
+    ProfScope prof("gemm_df", st, 4.0 * n * n * n * batch, 48.0 * n * n * batch);
+    re_chain_kernel<<<batch, CD_THREADS, smem, st>>>(R1, dW1, R2, dW2, R3, Re, n);
+    PLOM_CHECK_LAUNCH();
+    return PLOM_OK;
+  }
+  // (all upper triangular)  T2 = R2' = R2 - R2 (dW2 R2), T1 = R3 R2'
+  PLOM_TRY(gemm_df_launch(true, dW2, R2, nullptr, T1, n, batch, 3, nullptr, 0, 0, st));
+  PLOM_TRY(gemm_df_launch(true, R2, T1, R2, T2, n, batch, 3, nullptr, 0, 0, st));
+  PLOM_TRY(gemm_df_launch(false, R3, T2, nullptr, T1, n, batch, 3, nullptr, 0, 0, st));
+  // T2 = R1' = R1 - R1 (dW1 R1), Re = T1 R1'
+  PLOM_TRY(gemm_df_launch(true, dW1, R1, nullptr, Re, n, batch, 3, R1, -1, 1, st));
+  PLOM_TRY(gemm_df_launch(true, R1, Re, R1, T2, n, batch, 3, R1, 1, 0, st));
+  PLOM_TRY(gemm_df_launch(false, T1, T2, nullptr, Re, n, batch, 3, T2, 0, 1, st));
   return PLOM_OK;
 }
 

@@ -2464,21 +2464,6 @@ static int rf_graded(double* X, int n, RefineBufs& b, Arena& ws, cudaStream_t st
   return PLOM_OK;
 }
 
-// C = A B (n x n FP64): [Ah^T; Ah^T; Al^T]^T [Bh; Bl; Bh] by gemm_tn_df
-int gemm_nn_df(const double* A, const double* B, double* C, int n, Arena& ws, cudaStream_t st) {
-  const int64_t nn = (int64_t)n * n;
-  float* at = ws.take<float>((size_t)(3 * nn));
-  float* b3 = ws.take<float>((size_t)(3 * nn));
-  if (ws.measuring()) return gemm_tn_df(nullptr, n, nullptr, n, nullptr, n, n, n, 3 * (int64_t)n, ws, st);
-  PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "gemm_nn_df: workspace too small");
-  PLOM_REQUIRE(A && B && C && n >= 1, PLOM_ERR_ARG, "gemm_nn_df: bad arguments");
-  const int eg = rf_grid(nn);
-  rf_tsplit_kernel<<<eg, 256, 0, st>>>(A, n, 3, at);
-  PLOM_CHECK_LAUNCH();
-  rf_split3_kernel<<<eg, 256, 0, st>>>(B, nn, nullptr, b3);
-  PLOM_CHECK_LAUNCH();
-  return gemm_tn_df(at, n, b3, n, C, n, n, n, 3 * (int64_t)n, ws, st);
-}
 
 // SVD of the scaled B (Rcat = [Ah; Ah; Al], A = B^T) from the orthonormal
 // starting product Jo: S (scaled), Ut (columns = left vectors), VHt (rows =

@@ -8,7 +8,7 @@
 // tensor pipe (kind::f16, FP32 accumulation in TMEM) as hi*hi + hi*lo + lo*hi
 // (the dropped lo*lo term is below 2^-22 |x y|), at twice the rate of TF32
 // and with half the operand bytes.  Both planes are row-major m x ldp
-// (ldp = N rounded up to 64; padding columns are zero), which serves both
+// (ldp = packed_ld(N); padding columns are zero), which serves both
 // products without a transpose:
 //
 //  gram_packed  G (N x N, FP64) = Y^T Y over the m rows.  Upper 128 x 128
@@ -391,33 +391,36 @@ __global__ void __launch_bounds__(256) split_w16_kernel(const double* __restrict
                                                         float out_scale, __half* __restrict__ bhi,
                                                         __half* __restrict__ blo,
                                                         float* __restrict__ f, int64_t wstride,
-                                                        int fstride, int fold) {
-  // fold > 0: two copies of W on the diagonal, column j of copy h in row
-  // h fold + j of Bt at K offset 64 h (ldk = 128, s_in of 64)
+                                                        int fstride, int fold, int ldp,
+                                                        double* __restrict__ dW) {
+  // fold > 0: ldk / ldp copies of W on the diagonal, column j of copy h in row
+  // h fold + j of Bt at K offset h ldp (s_in of ldp).  dW (nin x k, or null;
+  // a batch with one W writes it once): the copies' rounding, W' - W
   __shared__ double red[8];
   // problem blockIdx.y of a batch: W_p, its input scales, its rows of Bt, its factors
   {
     const int64_t pb = blockIdx.y;
     W += pb * wstride;
-    s_in += pb * (fold ? 64 : ldk);
-    const int64_t rows = fold ? 2 * fold : k;
+    s_in += pb * ldp;
+    const int64_t rows = fold ? (int64_t)(ldk / ldp) * fold : k;
     bhi += pb * rows * (int64_t)ldk;
     blo += pb * rows * (int64_t)ldk;
     f += pb * fstride;
   }
   const int row = blockIdx.x;
-  const int half = fold && row >= fold ? 1 : 0;
-  const int j = row - half * fold;
+  const int copies = fold ? ldk / ldp : 1;
+  const int copy = fold ? min(row / fold, copies - 1) : 0;
+  const int j = row - copy * fold;
   if (j >= k) {
     if (threadIdx.x == 0) f[row] = 0.f;
-    if (fold && row < 2 * fold)  // a padding column of the packed output
+    if (fold && row < copies * fold)  // a padding column of the packed output
       for (int i = threadIdx.x; i < ldk; i += blockDim.x) {
         bhi[(int64_t)row * ldk + i] = __float2half_rn(0.f);
         blo[(int64_t)row * ldk + i] = __float2half_rn(0.f);
       }
     return;
   }
-  const int koff = 64 * half;
+  const int koff = copy * ldp;
   // 1 / s_in is exact (powers of two)
   double mx = 0.0;
   for (int i = threadIdx.x; i < nin; i += blockDim.x)
@@ -438,6 +441,10 @@ __global__ void __launch_bounds__(256) split_w16_kernel(const double* __restrict
     const __half l = __float2half_rn(x - __half2float(h));
     bhi[(int64_t)row * ldk + kk] = h;
     blo[(int64_t)row * ldk + kk] = l;
+    if (dW && copy == 0 && i < nin && (wstride != 0 || blockIdx.y == 0)) {
+      const double w = (double)(__half2float(h) + __half2float(l)) / t * (double)s_in[i];
+      dW[blockIdx.y * wstride + (int64_t)i * k + j] = w - W[(int64_t)i * ldw + j];
+    }
   }
   if (threadIdx.x == 0) f[row] = (float)((double)out_scale / t);
 }
@@ -791,12 +798,12 @@ __global__ void __launch_bounds__(32 * GR_WARPS) gram16_reduce_kernel(
                       ((pb * ntiles + tile) * chunks) * 128 * 128 + (int64_t)(i - ti * 128) * 128 +
                       (j - tj * 128);
     float2 acc = make_float2(0.f, 0.f);
-    if (fold) {  // the diagonal blocks of the even and of the odd rows
+    if (fold > 1) {  // the diagonal blocks of the rows side by side
+      if (j < N)
+        for (int c = warp; c < chunks; c += GR_WARPS)
 #pragma unroll 2
-      for (int c = warp; c < chunks; c += GR_WARPS) {
-        const float2* q = p + (int64_t)c * 128 * 128;
-        acc = dw_add(dw_add(acc, q[0]), q[64 * 128 + 64]);
-      }
+          for (int h = 0; h < fold; ++h)
+            acc = dw_add(acc, p[(int64_t)c * 128 * 128 + (int64_t)h * ld * 129]);
     } else {
 #pragma unroll 4
       for (int c = warp; c < chunks; c += GR_WARPS) acc = dw_add(acc, p[(int64_t)c * 128 * 128]);
@@ -1366,7 +1373,8 @@ __device__ __forceinline__ void apply_store_chunk(const float (&v)[32], int col0
       }
     } else if (r < mp) {
       __half* plane = q < 4 ? out.ohi : out.olo;
-      *reinterpret_cast<uint4*>(plane + (pb * mp + r) * out.ldo + col0 + 8 * (q & 3)) = val;
+      if (col0 + 8 * (q & 3) < out.ldo)
+        *reinterpret_cast<uint4*>(plane + (pb * mp + r) * out.ldo + col0 + 8 * (q & 3)) = val;
     }
   }
 }
@@ -2172,7 +2180,11 @@ static bool make_map_planes(CUtensorMap* map, const __half* base, uint64_t inner
   return r == CUDA_SUCCESS;
 }
 
-int64_t packed_ld(int64_t N) { return cdiv(N, 64) * 64; }
+// pitch of the planes.  Up to 128 columns the products are DRAM-bound, so the
+// pitch is padded to 16 columns only (TMA boxes past it read zeros): 80 columns
+// in 160 bytes a row instead of 256.  Wider operands are bound by the tensor
+// pipe and the L2; their rows keep to whole 128-byte lines.
+int64_t packed_ld(int64_t N) { return N <= 128 ? cdiv(N, 16) * 16 : cdiv(N, 64) * 64; }
 
 static void pair_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned grid,
                                unsigned threads, size_t smem, cudaStream_t st) {
@@ -2209,20 +2221,27 @@ static int pair_clusters() {
   return n;
 }
 
-// rows per problem in the planes: m for one problem (even when ld = 64, so
-// that two rows can be read as one of 128, see fold2); for a batch, m rounded
-// up to 128 so that no stage or output tile of one problem reaches the next
+// Operands of at most 64 columns fill a part of a 128-column tile.  Their
+// planes, row-major m x ld, are read as (m / F) x (F ld): F = 2, 4 or 8 rows side
+// by side (F ld <= 128).  A Gram then is the sum of the F diagonal blocks of the
+// product, and Y W the product with diag(W, ..., W).  Stages, tensor products,
+// TMEM drains and epilogue warps all carry F times the rows at the same cost.
+static int64_t fold_of(int64_t ld) { return ld <= 16 ? 8 : ld <= 32 ? 4 : ld <= 64 ? 2 : 1; }
+
+// rows per problem in the planes: m rounded up to whole folded rows; for a
+// batch, to 128 rows and 64 folded rows, so that no stage or output tile of one
+// problem reaches the next
 int64_t packed_rows(int64_t m, int64_t batch, int64_t ld) {
-  return batch > 1 ? cdiv(m, 128) * 128 : ld == 64 ? m + (m & 1) : m;
+  const int64_t F = fold_of(ld), u = batch > 1 ? std::max<int64_t>(128, 64 * F) : F;
+  return cdiv(m, u) * u;
 }
 
-// Operands of at most 64 columns (ld = 64) fill half of a 128-column tile.
-// Their planes, row-major m x 64, are read as (m / 2) x 128: rows 2 r and
-// 2 r + 1 side by side.  A Gram then is the sum of the two 64 x 64 diagonal
-// blocks of the 128 x 128 product, and Y W is the product with diag(W, W).
-// Stages, tensor products, TMEM drains and epilogue warps all carry twice the
-// rows at the same cost.
-static bool fold2(const Packed& p) { return p.ld == 64 && (p.mp & 1) == 0; }
+// the rows that can be folded (a view may hold a row count that F does not divide)
+static int64_t fold_rows(const Packed& p, int64_t unit = 1) {
+  int64_t F = fold_of(p.ld);
+  while (F > 1 && p.mp % (F * unit)) F /= 2;
+  return F;
+}
 
 void packed_carve(Arena& ws, Packed& p, int64_t m, int64_t N, int64_t batch) {
   p.m = m;
@@ -2444,9 +2463,8 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
                 bool accumulate) {
   if (p.ld > 128) return gram_packed_wide(p, G, err, ws, st, accumulate);
   const int64_t N = p.N, batch = p.batch;
-  const bool fold = fold2(p);
-  const int64_t m = fold ? cdiv(p.m, 2) : p.m;  // (folded) rows
-  const int64_t mp = fold ? p.mp / 2 : p.mp, ld = fold ? 128 : p.ld;
+  const int64_t F = fold_rows(p, batch > 1 ? hp::G_BK : 1);
+  const int64_t m = cdiv(p.m, F), mp = p.mp / F, ld = F * p.ld;  // folded
   const int tn = (int)cdiv(p.ld, 128);
   const int tiles = tn * (tn + 1) / 2;
   const int chunks = gram16_narrow_chunks(m, tiles * batch);
@@ -2480,7 +2498,7 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
   const int blocks = (int)std::min<int64_t>(batch * N * cdiv(N, 32), (int64_t)num_sms() * 4);
   ProfScope prof_r("gram_reduce", st, 0.0, 8.0 * (double)batch * tiles * chunks_eff * 128 * 128);
   hp::gram16_reduce_kernel<<<blocks, 32 * hp::GR_WARPS, 0, st>>>(part, (int)N, tn, chunks_eff, p.scale, G,
-                                                   (int)batch, (int)p.ld, accumulate ? 1 : 0, fold ? 1 : 0);
+                                                   (int)batch, (int)p.ld, accumulate ? 1 : 0, (int)F);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
 }
@@ -2575,16 +2593,16 @@ int tn_packed(const Packed& a, const Packed& b, double* C, int64_t ldc, int* err
 
 int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float* C, int64_t ldc,
                  Packed* out, int* err, Arena& ws, cudaStream_t st, int64_t wstride,
-                 int64_t cstride, bool upper) {
+                 int64_t cstride, bool upper, double* dW) {
   const int64_t batch = p.batch;
-  // two rows per 128-column tile row (see fold2) when the output folds too:
-  // packed planes of 64 columns, or dense FP32 rows
-  const bool fold = fold2(p) && k <= 64 && (out ? out->ld == 64 : ldc == k);
-  const int64_t kh = out ? 64 : k;             // (folded) output columns of one row
-  const int64_t m = fold ? cdiv(p.m, 2) : p.m; // (folded) rows
-  const int64_t mp = fold ? p.mp / 2 : p.mp, lda = fold ? 128 : p.ld;
-  const int64_t ldk = lda;  // K extent of the W copies (= packed pitch of the input)
-  const int64_t kf = fold ? 2 * kh : k;        // columns of the product
+  // rows side by side (see fold_of) when the output folds too: packed planes
+  // of the same pitch, or dense FP32 rows
+  const int64_t kh = out ? out->ld : k;  // output columns of one row
+  int64_t F = (out ? out->ld == p.ld : ldc == k) ? fold_rows(p) : 1;
+  while (F > 1 && F * kh > 128) F /= 2;
+  const int64_t m = cdiv(p.m, F), mp = p.mp / F, lda = F * p.ld;  // folded
+  const int64_t ldk = lda;  // K extent of the W copies (= pitch of the input)
+  const int64_t kf = F > 1 ? F * kh : k;  // columns of the product
   // output tile width (see ApplyCfg): 256 for dense W wider than 128 columns.
   // An upper-triangular W keeps 128-wide tiles: its short column tiles (the
   // first K blocks only) finish their products faster than the single
@@ -2605,8 +2623,7 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   const int64_t col_tiles = cdiv(kf, TN);
   const int fstride = (int)(col_tiles * TN);
   // (what folds is decided by the strides of the call too: room for both)
-  const bool may_fold = p.ld == 64 && k <= 64;
-  const int64_t wk = may_fold ? 128 * 128 : kf * ldk;
+  const int64_t wk = p.ld <= 64 && k <= 64 ? 128 * 128 : kf * ldk;
   __half* bhi = ws.take<__half>((size_t)(2 * batch * wk));
   __half* blo = bhi ? bhi + batch * kf * ldk : nullptr;
   float* f = ws.take<float>((size_t)(batch * fstride));
@@ -2633,7 +2650,7 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   const float out_scale = out ? (float)(1 << hp::PK_LOG2) : 1.0f;
   hp::split_w16_kernel<<<dim3((unsigned)fstride, (unsigned)batch), 256, 0, st>>>(
       W, ldw, (int)p.N, (int)k, (int)ldk, p.scale, out_scale, bhi, blo, f, wstride, fstride,
-      fold ? (int)kh : 0);
+      F > 1 ? (int)kh : 0, (int)p.ld, dW);
   PLOM_CHECK_LAUNCH();
   if (out) {
     // packed output columns carry the fixed scale 2^14
@@ -2666,12 +2683,12 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   const int grid = (int)std::min<int64_t>(by_rows ? batch * row_tiles : tiles, num_sms());
   hp::ApplyOut o;
   o.C = out ? nullptr : C;
-  o.ldc = fold ? 2 * ldc : ldc;
+  o.ldc = F * ldc;
   o.cstride = cstride;
-  o.klast = (int)(fold && (p.m & 1) ? k : kf);
+  o.klast = (int)(F > 1 && p.m % F ? (p.m % F) * k : kf);
   o.ohi = out ? out->hi : nullptr;
   o.olo = out ? out->lo : nullptr;
-  o.ldo = out ? (int)(fold ? 128 : out->ld) : 0;
+  o.ldo = out ? (int)(F * out->ld) : 0;
   // an upper-triangular W (k = N) needs m N (N + 1) flops: row i of W meets
   // columns j >= i only
   const bool tri = tri_w;
@@ -2693,14 +2710,14 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
       pair_launch_config(cfg, at, (unsigned)(2 * clusters), hp::PairCfg<256>::THREADS,
                          hp::pair_smem<256>(), st);
       PLOM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hp::apply16p_kernel<256>, tmA, tmB, m,
-                                         (int)(ldk / hp::PairCfg<256>::BK), (int)k, col_tiles,
+                                         (int)cdiv(ldk, hp::PairCfg<256>::BK), (int)k, col_tiles,
                                          ptiles, (const float*)f, o, err, p.mp, tri ? 1 : 0,
                                          pby_rows));
     } else {
       pair_launch_config(cfg, at, (unsigned)(2 * clusters), hp::PairCfg<128>::THREADS,
                          hp::pair_smem<128>(), st);
       PLOM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hp::apply16p_kernel<128>, tmA, tmB, m,
-                                         (int)(ldk / hp::PairCfg<128>::BK), (int)k, col_tiles,
+                                         (int)cdiv(ldk, hp::PairCfg<128>::BK), (int)k, col_tiles,
                                          ptiles, (const float*)f, o, err, p.mp, tri ? 1 : 0,
                                          pby_rows));
     }
@@ -2709,11 +2726,11 @@ int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float
   }
   if (TN == 256)
     hp::apply16_kernel<256><<<grid, hp::ApplyWarps<256>::THREADS, hp::apply_smem<256>(), st>>>(
-        tmA, tmB, m, (int)(ldk / hp::ApplyCfg<256>::BK), (int)k, col_tiles, tiles, f, o, err, p.mp,
+        tmA, tmB, m, (int)cdiv(ldk, hp::ApplyCfg<256>::BK), (int)k, col_tiles, tiles, f, o, err, p.mp,
         row_tiles, fstride, tri ? 1 : 0, by_rows);
   else
     hp::apply16_kernel<128><<<grid, hp::ApplyWarps<128>::THREADS, hp::apply_smem<128>(), st>>>(
-        tmA, tmB, m, (int)(ldk / 64), (int)kf, col_tiles, tiles, f, o, err, mp, row_tiles,
+        tmA, tmB, m, (int)cdiv(ldk, 64), (int)kf, col_tiles, tiles, f, o, err, mp, row_tiles,
         fstride, tri ? 1 : 0, by_rows);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;

@@ -48,10 +48,6 @@ size_t gemm_tn_workspace_batched(int64_t M, int64_t N, int64_t K, bool sym, size
 // C (M x N, FP64, ld ldc) = A^T B for FP32 A (K x M), B (K x N): exact products,
 // compensated double-float sums over row chunks, FP64 chunk reduction.
 // ---- dense.cu ----
-// C = A B for n x n FP64 operands as double-float sums of exact FP32 products
-// (~1e-9 relative to sum |a_ik b_kj|; the mixed form's n x n products, whose
-// factors carry FP32-level information), on the CUDA cores' FP32 pipe
-int gemm_nn_df(const double* A, const double* B, double* C, int n, Arena& ws, cudaStream_t st);
 int gemm_tn_df(const float* A, int64_t lda, const float* B, int64_t ldb, double* C, int64_t ldc,
                int64_t M, int64_t N, int64_t K, Arena& ws, cudaStream_t st);
 
@@ -78,6 +74,12 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
 // as in gemm_sq.
 int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
                cudaStream_t st);
+// Re = R3 R2' R1' with R' = R - R dW R, the factor of X Q W' = Q for the rounded
+// W' = W + dW that the tall product used in the place of W = R^-1: R' is the
+// inverse of W' up to (dW R)^2.  T1, T2: n x n scratch per problem.
+int re_chain(const double* R1, const double* dW1, const double* R2, const double* dW2,
+             const double* R3, double* Re, double* T1, double* T2, int n, int batch,
+             cudaStream_t st);
 // W = R^{-1} for upper-triangular R (batch, stride n*n).
 int trtri_upper(const double* R, double* W, int n, int batch, Arena& ws, cudaStream_t st);
 // One-sided Jacobi SVD of `batch` square n x n matrices A (ld n, stride n*n),

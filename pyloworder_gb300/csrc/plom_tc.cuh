@@ -9,11 +9,10 @@
 namespace plom {
 
 // Tall FP32 operand packed as two fp16 planes (gemm_f16.cu):
-//   hi + lo = Y diag(scale), hi and lo row-major (batch x mp) x ld (ld = N
-//   rounded up to 64, padding columns zero; lo right after hi), scale[p][j]
-//   a power of two per problem and column.  A batch holds `batch` problems
-//   of m rows each, mp rows apart (one problem: mp = m, rounded up to even when
-//   ld = 64; else m rounded up to 128; the padding rows are zero).
+//   hi + lo = Y diag(scale), hi and lo row-major (batch x mp) x ld (ld =
+//   packed_ld(N), padding columns zero; lo right after hi), scale[p][j] a power
+//   of two per problem and column.  A batch holds `batch` problems of m rows
+//   each, mp = packed_rows(m) rows apart (the padding rows are zero).
 struct Packed {
   __half* hi;
   __half* lo;
@@ -48,10 +47,13 @@ int tn_packed(const Packed& a, const Packed& b, double* C, int64_t ldc, int* err
 // Y W for W (N x k, FP64, ldw; a batch: W_p wstride apart): FP32 into C
 // (ldc; C_p cstride apart) when out == nullptr, else packed into *out
 // (planes like the input, scale 2^14).  upper: W (k = N) is upper triangular,
-// and the zero blocks below its diagonal are skipped
+// and the zero blocks below its diagonal are skipped.  dW (N x k, FP64, problems
+// wstride apart, or null): the rounding of W to its 22-bit copies, W' - W (the
+// product is exact for W' up to the operand's own rounding and the accumulation)
 int apply_packed(const Packed& p, const double* W, int64_t ldw, int64_t k, float* C, int64_t ldc,
                  Packed* out, int* err, Arena& ws, cudaStream_t st, int64_t wstride = 0,
-                 int64_t cstride = 0, bool upper = false);
+                 int64_t cstride = 0, bool upper = false,
+                 double* dW = nullptr);
 
 // U = Q2 M (m x cw*n FP32, ldu; a batch: U_p ustride, M_p mstride apart):
 // renormalise the columns whose M column (N x N, real or embedded complex)

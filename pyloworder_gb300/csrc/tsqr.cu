@@ -35,8 +35,6 @@ namespace plom {
 
 static const double U64 = 1.1102230246251565e-16;  // 2^-53
 static const double U32 = 5.9604644775390625e-08;  // 2^-24 (the fp16-pair products are FP32-accurate)
-// n x n products of the mixed form in double-float sums from this size on
-static const int DF_PRODUCT_MIN_N = 256;
 
 // ---------------------------------------------------------------------------
 // tall operations, dispatched on precision
@@ -203,6 +201,7 @@ static int cholqr3(int prec, bool cplx, const TI* X, int64_t m, int n, int64_t l
 struct PackedCore {
   Packed P0, P1, P2;
   double *G, *H, *R1, *R2, *R3, *W1, *W2, *W3, *Rp, *Re, *F;
+  double *dW1, *dW2;  // rounding of the W1 and W2 that the tall products used
 };
 
 static void carve_packed_core(Arena& ws, PackedCore& b, int64_t m, int N, bool p1_external,
@@ -219,6 +218,8 @@ static void carve_packed_core(Arena& ws, PackedCore& b, int64_t m, int N, bool p
   b.Rp = ws.take<double>(nn);
   b.Re = ws.take<double>(nn);
   b.F = ws.take<double>(nn);
+  b.dW1 = ws.take<double>(nn);
+  b.dW2 = ws.take<double>(nn);
   packed_carve(ws, b.P0, m, N);
   b.P2 = b.P0;
   b.P2.scale = ws.take<float>((size_t)b.P0.ld);
@@ -249,7 +250,24 @@ static int chol_pass_packed(bool cplx, int n, const Packed& P, PackedCore& b, do
   return PLOM_OK;
 }
 
-// passes 2 and 3 from Q1 (packed in b.P1; R1 in b.R1) and Re = R3 R2 R1
+// Q (packed in out) = P W with the rounding of W recorded in dW.  W's copies
+// carry 22 bits, and W = R^-1 of an ill-conditioned factor is large: through
+// |W| |R| its rounding, the same for every row, was the largest error of the
+// mixed form (1e-6 of a POD's reconstruction, 1e-7 without it), so R is later
+// replaced by the inverse of the W that was used (re_chain).
+static int apply_recorded(bool cplx, int n, const Packed& P, const double* W, double* F, double* dF,
+                          double* dW, Packed& out, int* info, Arena& ws, cudaStream_t st) {
+  const int N = cplx ? 2 * n : n;
+  int s = PLOM_OK;
+  const double* Wf = ws.measuring() ? W : rowform(cplx, W, F, n, st, s);
+  PLOM_TRY(s);
+  PLOM_TRY(apply_packed(P, Wf, N, N, nullptr, 0, &out, info, ws, st, 0, 0, true, cplx ? dF : dW));
+  // (the row form is a block transpose: applied again, it goes back)
+  if (cplx && !ws.measuring()) PLOM_TRY(embed_to_rowform(dF, dW, n, 1, st));
+  return PLOM_OK;
+}
+
+// passes 2 and 3 from Q1 (packed in b.P1; R1, dW1 in b) and Re = R3 R2' R1'
 static int cholqr3_packed_passes23(bool cplx, int n, PackedCore& b, double relfail, int* info,
                                    Arena& ws, cudaStream_t st) {
   const int N = cplx ? 2 * n : n;
@@ -262,24 +280,15 @@ static int cholqr3_packed_passes23(bool cplx, int n, PackedCore& b, double relfa
     ws.off = mark;
     return s;
   };
-  int s = PLOM_OK;
   // pass 2
   PLOM_TRY(sub([&] { return chol_pass_packed(cplx, n, b.P1, b, b.R2, b.W2, 0.0, relfail, info, ws, st); }));
-  const double* F2 = ws.measuring() ? b.W2 : rowform(cplx, b.W2, b.F, n, st, s);
-  PLOM_TRY(s);
-  PLOM_TRY(sub([&] { return apply_packed(b.P1, F2, N, N, nullptr, 0, &b.P2, info, ws, st, 0, 0, true); }));
+  PLOM_TRY(sub([&] {
+    return apply_recorded(cplx, n, b.P1, b.W2, b.F, b.Rp, b.dW2, b.P2, info, ws, st);
+  }));
   // pass 3
   PLOM_TRY(sub([&] { return chol_pass_packed(cplx, n, b.P2, b, b.R3, b.W3, 0.0, relfail, info, ws, st); }));
-  // Re = R3 R2 R1 in double-float arithmetic (the factors carry the 22-bit
-  // operands' information; FP64 runs at 1/64 of the FP32 rate): from n = 256 on
-  // as FP32 products with double-float sums
-  if (N >= DF_PRODUCT_MIN_N) {
-    PLOM_TRY(sub([&] { return gemm_nn_df(b.R3, b.R2, b.Rp, N, ws, st); }));
-    PLOM_TRY(sub([&] { return gemm_nn_df(b.Rp, b.R1, b.Re, N, ws, st); }));
-  } else if (!ws.measuring()) {
-    PLOM_TRY(gemm_df_nn(b.R3, b.R2, b.Rp, N, 1, 3, st));
-    PLOM_TRY(gemm_df_nn(b.Rp, b.R1, b.Re, N, 1, 3, st));
-  }
+  if (!ws.measuring())
+    PLOM_TRY(re_chain(b.R1, b.dW1, b.R2, b.dW2, b.R3, b.Re, b.Rp, b.H, N, 1, st));
   ws.off = need;
   return PLOM_OK;
 }
@@ -381,7 +390,9 @@ static int cholqr3_packed_chunked(const float* X, int64_t m, int n, int64_t ldx,
   P0b.mp = P1b.mp = mc;
   P0b.scale = xscale;
   P1b.scale = qscale;
-  PLOM_TRY(sub([&] { return apply_packed(P0b, b.W1, N, N, nullptr, 0, &P1b, info, ws, st, 0, 0, true); }));
+  PLOM_TRY(sub([&] {
+    return apply_recorded(false, n, P0b, b.W1, b.F, b.Rp, b.dW1, P1b, info, ws, st);
+  }));
   PLOM_TRY(sub([&] { return cholqr3_packed_passes23(false, n, b, relfail, info, ws, st); }));
   ws.off = need;
   return PLOM_OK;
@@ -404,13 +415,12 @@ static int cholqr3_packed(bool cplx, const float* X, int64_t m, int n, int64_t l
     ws.off = mark;
     return s;
   };
-  int s = PLOM_OK;
   PLOM_TRY(sub([&] { return pack_f32(X, ldx, m, N, b.P0, ws, st); }));
   // pass 1
   PLOM_TRY(sub([&] { return chol_pass_packed(cplx, n, b.P0, b, b.R1, b.W1, rel1, relfail, info, ws, st); }));
-  const double* F1 = ws.measuring() ? b.W1 : rowform(cplx, b.W1, b.F, n, st, s);
-  PLOM_TRY(s);
-  PLOM_TRY(sub([&] { return apply_packed(b.P0, F1, N, N, nullptr, 0, &b.P1, info, ws, st, 0, 0, true); }));
+  PLOM_TRY(sub([&] {
+    return apply_recorded(cplx, n, b.P0, b.W1, b.F, b.Rp, b.dW1, b.P1, info, ws, st);
+  }));
   PLOM_TRY(sub([&] { return cholqr3_packed_passes23(cplx, n, b, relfail, info, ws, st); }));
   ws.off = need;
   return PLOM_OK;
@@ -451,13 +461,7 @@ static int svd_tail_packed(bool cplx, int n, PackedCore& b, int64_t m, float* U,
   need = std::max(need, ws.off);
   ws.off = mark;
   const double* Mop = b.F;
-  if (!cplx && N >= DF_PRODUCT_MIN_N) {
-    // M = R3^-1 Ur, the right operand of Q2 x M (double-float products)
-    PLOM_TRY(gemm_nn_df(b.W3, Ur, Me, N, ws, st));
-    need = std::max(need, ws.off);
-    ws.off = mark;
-    Mop = Me;
-  } else if (!ws.measuring()) {
+  if (!ws.measuring()) {
     // M = R3^-1 Ur (embedded for complex), the right operand of Q2 x M
     if (cplx) {
       PLOM_TRY(complex_to_embed(Ur, Ue, n, 1, st));
@@ -528,6 +532,8 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
   double* F = ws.take<double>(nnb);
   double* Me = ws.take<double>(nnb);
   double* Ue = ws.take<double>(nnb);
+  double* dW1 = ws.take<double>(nnb);
+  double* dW2 = ws.take<double>(nnb);
   const size_t cnb = (size_t)n * n * cw * batch;
   double* Rc = ws.take<double>(cnb);
   double* Ur = ws.take<double>(cnb);
@@ -557,24 +563,28 @@ static int tsqr_svd_batched_packed(bool cplx, const float* X, int64_t batch, int
     if (cplx && !meas) PLOM_TRY(complexify_gram(H, G, n, bi, st));
     return sub([&] { return chol_inverse_df(G, R, W, N, bi, rel0, relfail, info, ws, st); });
   };
-  auto rowform_b = [&](const double* W) -> const double* {
-    if (!cplx || meas) return W;
-    return embed_to_rowform(W, F, n, bi, st) == PLOM_OK ? F : nullptr;
+  // out = P W, the rounding of W in dW (see apply_recorded)
+  auto apply_rec = [&](const Packed& P, const double* W, double* dW, Packed& out) -> int {
+    const double* Wf = W;
+    if (cplx && !meas) {
+      PLOM_TRY(embed_to_rowform(W, F, n, bi, st));
+      Wf = F;
+    }
+    PLOM_TRY(sub([&] {
+      return apply_packed(P, Wf, N, N, nullptr, 0, &out, info, ws, st, NN, 0, true, cplx ? Rp : dW);
+    }));
+    if (cplx && !meas) PLOM_TRY(embed_to_rowform(Rp, dW, n, bi, st));
+    return PLOM_OK;
   };
   PLOM_TRY(sub([&] { return pack_f32(X, ldx, m, N, P0, ws, st, xstride); }));
   PLOM_TRY(pass(P0, R1, W1, rel1));
-  const double* F1 = rowform_b(W1);
-  PLOM_REQUIRE(meas || F1, PLOM_ERR_CUDA, "tsqr_svd_batched: embedding failed");
-  PLOM_TRY(sub([&] { return apply_packed(P0, F1, N, N, nullptr, 0, &P1, info, ws, st, NN, 0, true); }));
+  PLOM_TRY(apply_rec(P0, W1, dW1, P1));
   PLOM_TRY(pass(P1, R2, W2, 0.0));
-  const double* F2 = rowform_b(W2);
-  PLOM_REQUIRE(meas || F2, PLOM_ERR_CUDA, "tsqr_svd_batched: embedding failed");
-  PLOM_TRY(sub([&] { return apply_packed(P1, F2, N, N, nullptr, 0, &P2, info, ws, st, NN, 0, true); }));
+  PLOM_TRY(apply_rec(P1, W2, dW2, P2));
   PLOM_TRY(pass(P2, R3, W3, 0.0));
   const double* Rin = Re;
   if (!meas) {
-    PLOM_TRY((gemm_df_nn(R3, R2, Rp, N, bi, 3, st)));
-    PLOM_TRY((gemm_df_nn(Rp, R1, Re, N, bi, 3, st)));
+    PLOM_TRY(re_chain(R1, dW1, R2, dW2, R3, Re, Rp, H, N, bi, st));
     if (cplx) {
       PLOM_TRY(embed_to_complex(Re, Rc, n, bi, st));
       Rin = Rc;
@@ -1179,7 +1189,9 @@ static int tsqr_svd_host_mixed(const float* Xh, int64_t m, int n, int64_t ldx, f
   P0b.mp = P1b.mp = pl.mc;
   P0b.scale = xscale;
   P1b.scale = qscale;
-  PLOM_TRY(sub([&] { return apply_packed(P0b, b.W1, N, N, nullptr, 0, &P1b, info, ws, st, 0, 0, true); }));
+  PLOM_TRY(sub([&] {
+    return apply_recorded(false, n, P0b, b.W1, b.F, b.Rp, b.dW1, P1b, info, ws, st);
+  }));
   PLOM_TRY(sub([&] { return cholqr3_packed_passes23(false, n, b, relfail, info, ws, st); }));
   // U straight into page-locked host memory when the caller's U is mapped
   // (the final product's stores cross the host link while it computes);

@@ -1,6 +1,6 @@
-"""Tall operands of at most 64 columns, whose packed rows the tensor products
-read in pairs: odd and even row counts around the tiles, dense and strided
-rows, narrow and full outputs.
+"""Tall operands of at most 128 columns: packed rows padded to 16 columns, read
+2, 4 or 8 side by side up to 64 columns.  Row counts around the tiles and the
+folds, dense and strided rows, narrow and full outputs.
 
 Tolerances: a product of 22-bit operands errs by at most 2^-21 of |A| |B| per
 element, its FP32 accumulation by the K = 64 terms' rounding: 1e-6 (|A| |B|).
@@ -16,7 +16,8 @@ ROWS = [1, 2, 3, 127, 128, 129, 255, 256, 257, 511, 4097, 40001]
 
 
 @pytest.mark.parametrize("m", ROWS)
-@pytest.mark.parametrize("n,k", [(1, 1), (7, 64), (32, 5), (63, 63), (64, 64), (64, 65), (65, 64)])
+@pytest.mark.parametrize("n,k", [(1, 1), (7, 64), (16, 16), (17, 8), (32, 5), (32, 33), (33, 32), (48, 48),
+                                 (63, 63), (64, 64), (64, 65), (65, 64), (80, 81), (97, 128), (129, 16)])
 def test_products(m, n, k):
     import pyloworder_gb300 as P
     rng = np.random.default_rng(m * 100 + n + k)
@@ -28,7 +29,7 @@ def test_products(m, n, k):
 
 
 @pytest.mark.parametrize("m", [64, 65, 127, 128, 129, 255, 256, 257, 4097, 40001])
-@pytest.mark.parametrize("n", [1, 33, 62, 64])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 32, 33, 48, 49, 62, 64, 65, 80, 97, 113])
 @pytest.mark.parametrize("ld", [0, 5])
 def test_factors(m, n, ld):
     import pyloworder_gb300 as P
@@ -42,3 +43,19 @@ def test_factors(m, n, ld):
     assert np.max(np.abs(Q.T @ Q - np.eye(n))) < 1e-5
     assert np.linalg.norm(Q @ R - A64) < 1e-5 * np.linalg.norm(A64)
     assert np.linalg.norm(R - np.linalg.qr(A64)[1]) < 1e-4 * np.linalg.norm(R)
+
+
+@pytest.mark.parametrize("m", [64, 65, 129, 511, 513])
+@pytest.mark.parametrize("n", [5, 16, 24, 31])
+def test_batch(m, n):
+    # complex problems side by side (2 n real columns): no row of one reaches another
+    import pyloworder_gb300 as P
+    rng = np.random.default_rng(m * n)
+    A = (rng.standard_normal((5, m, n)) + 1j * rng.standard_normal((5, m, n))).astype(np.complex64)
+    A *= np.array([1.0, 1e3, 1e-3, 1.0, 1e6])[:, None, None]
+    U, S, V = P.vmmath.tsqr_svd_batched_device(torch.from_numpy(A).cuda())
+    U, S, V = (x.cpu().numpy() for x in (U, S, V))
+    for b in range(5):
+        ex = np.linalg.svd(A[b].astype(np.complex128), compute_uv=False)
+        assert np.max(np.abs(S[b] - ex)) < 1e-5 * ex[0]
+        assert np.linalg.norm((U[b] * S[b]) @ V[b] - A[b]) < 1e-5 * np.linalg.norm(A[b])
