@@ -2578,18 +2578,23 @@ static int jacobi_pre32(const double* A, const double* At, int n, double tol, do
   double* Jo = ws.take<double>(nn);
   float* Rcat = ws.take<float>(3 * nn);
   const size_t mark = ws.off;
-  if (ws.measuring()) {  // the partials of G's product, then the refinement's needs
-    PLOM_TRY(gemm_tn_df(nullptr, n, nullptr, n, nullptr, n, n, n, n, ws, st));
+  if (ws.measuring()) {  // the sweeps', the partials of G's product, then the refinement's needs
+    if (jacobi_gram_plan_ok(n))
+      PLOM_TRY(jacobi_gram_f32(nullptr, n, 0.f, 0.f, 0.f, nullptr, nullptr, nullptr, ws, st));
     size_t need = ws.off;
+    ws.off = mark;
+    PLOM_TRY(gemm_tn_df(nullptr, n, nullptr, n, nullptr, n, n, n, n, ws, st));
+    need = std::max(need, ws.off);
     ws.off = mark;
     PLOM_TRY(jacobi_refine(nullptr, nullptr, n, nullptr, nullptr, nullptr, nullptr, ws, st));
     ws.off = std::max(need, ws.off);
     return PLOM_OK;
   }
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
-  if (jacobi_cta_f32_usable(n)) {
-    PLOM_TRY(jacobi_cta_f32(A, n, 1, JAC_PRE32_TOL, JAC_PRE32_MAX_SWEEPS, JAC_PRE32_FLOOR,
-                            JAC_PRE32_TSTOP, J32, j32.amax, info, st));
+  if (jacobi_gram_usable(n)) {
+    PLOM_TRY(jacobi_gram_f32(A, n, JAC_PRE32_TOL, JAC_PRE32_FLOOR, JAC_PRE32_TSTOP, J32, j32.amax,
+                             info, ws, st));
+    ws.off = mark;
   } else {
     const void* k = (const void*)jacobi_block_f32_kernel;
     const size_t smem = (size_t)4 * J32B * j32.pitch * sizeof(float);
@@ -2646,7 +2651,7 @@ static int jacobi_svd_transposed(const double* A, int n, double tol, double* S, 
   PLOM_REQUIRE(A && S && U && VH && info, PLOM_ERR_ARG, "jacobi: null pointer");
   if (!pre32 && tol >= JAC_DF_TOL && jacobi_cta_usable(n, 0))
     return jacobi_cta(A, n, 1, 0, 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U, VH, info, st);
-  if (!pre32 || !jacobi_cta_f32_usable(n)) PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
+  if (!pre32 || !jacobi_gram_usable(n)) PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
   if (pre32)
     PLOM_TRY(jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st));
   else

@@ -803,15 +803,6 @@ static bool jc_plan(JcPlan& pl, int n, int cplx) {
   return true;
 }
 
-static bool jc_plan_f32(JcPlan& pl, int n) {
-  if (n > 512) return false;
-  jc_blocks(pl, n, 16);
-  if (n <= 256) jc_set<ArF32, 32, 2, 256>(pl);
-  else if (n <= 384) jc_set<ArF32, 32, 3, 384>(pl);
-  else jc_set<ArF32, 32, 4, 512>(pl);
-  return true;
-}
-
 // kernel attributes, and whether clusters of the plan's size can be resident
 // (asked once per kernel and device)
 static bool jc_ready(const JcPlan& pl) {
@@ -906,34 +897,6 @@ int jacobi_cta(const double* A, int n, int batch, int cplx, int trans, double to
       At, Vt, nrm2, n, cplx ? 2 : 1, trans, amax, S, U, VH);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
-}
-
-bool jacobi_cta_f32_usable(int n) {
-  JcPlan pl;
-  return jc_plan_f32(pl, n) && jc_ready(pl);
-}
-
-int jacobi_cta_f32(const double* A, int n, int trans, float tol, int max_sweeps, float floor_rel,
-                   float tstop, float* J, unsigned long long* amax, int* info, cudaStream_t st) {
-  JcPlan pl;
-  PLOM_REQUIRE(jc_plan_f32(pl, n), PLOM_ERR_UNSUPPORTED, "jacobi: %d columns", n);
-  JacCtaArgs a = {};
-  a.A = A;
-  a.n = n;
-  a.C = pl.C;
-  a.bs = pl.bs;
-  a.nblk = pl.nblk;
-  a.rows = pl.rows;
-  a.tol = tol;
-  a.trans = trans;
-  a.J = J;
-  a.floor = floor_rel;
-  a.tstop = tstop;
-  a.amax = amax;
-  a.info = info;
-  a.max_sweeps = max_sweeps;
-  ProfScope prof("jacobi_svd_f32", st, 0.0, 4.0 * 3.0 * n * n);
-  return jc_launch(pl, a, 1, st);
 }
 
 }  // namespace plom

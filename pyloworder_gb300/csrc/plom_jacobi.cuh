@@ -13,10 +13,13 @@ bool jacobi_cta_usable(int n, int cplx);
 int jacobi_cta(const double* A, int n, int batch, int cplx, int trans, double tol, double* At,
                double* Vt, double* nrm2, unsigned long long* amax, double* S, double* U,
                double* VH, int* info, cudaStream_t st);
-// FP32 sweeps of one real matrix: the rotation product J (n x n row-major) and
-// the bits of max |a|.
-bool jacobi_cta_f32_usable(int n);
-int jacobi_cta_f32(const double* A, int n, int trans, float tol, int max_sweeps, float floor_rel,
-                   float tstop, float* J, unsigned long long* amax, int* info, cudaStream_t st);
+// FP32 sweeps over the rows of one real n x n matrix (jacobi_gram.cu): the
+// rotation product V (n x n row-major, FP32) and the bits of max |a|.  plan_ok:
+// by the size alone (workspace queries); usable: its CTAs can also be resident
+// together on this device.
+bool jacobi_gram_plan_ok(int n);
+bool jacobi_gram_usable(int n);
+int jacobi_gram_f32(const double* A, int n, float tol, float floor_rel, float tstop, float* V,
+                    unsigned long long* amax, int* info, Arena& ws, cudaStream_t st);
 
 }  // namespace plom
