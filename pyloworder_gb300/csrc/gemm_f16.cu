@@ -2553,7 +2553,11 @@ int tn_packed(const Packed& a, const Packed& b, double* C, int64_t ldc, int* err
   const int64_t m = a.m;
   const int tna = (int)cdiv(a.ld, 128), tnb = (int)cdiv(b.ld, 128);
   const int tiles = tna * tnb;
-  const int chunks = gram16_narrow_chunks(m, tiles);
+  // gram16_chunks, not the Gram's fewer and longer chunks: these products are
+  // results, not Grams that later passes correct, and the FP32 sums of a chunk
+  // lose by their length (7 x 1 tiles of 82,127 rows, 256 rows a chunk: 1.6e-6;
+  // 4,096 rows: 8.7e-6)
+  const int chunks = gram16_chunks(m, tiles);
   int64_t rpc = cdiv(m, chunks);
   rpc = cdiv(rpc, hp::G_BK) * hp::G_BK;
   const int chunks_eff = (int)std::max<int64_t>(1, cdiv(m, rpc));

@@ -59,3 +59,21 @@ def test_batch(m, n):
         ex = np.linalg.svd(A[b].astype(np.complex128), compute_uv=False)
         assert np.max(np.abs(S[b] - ex)) < 1e-5 * ex[0]
         assert np.linalg.norm((U[b] * S[b]) @ V[b] - A[b]) < 1e-5 * np.linalg.norm(A[b])
+
+
+@pytest.mark.parametrize("m,n,r", [(40001, 830, 20), (82127, 799, 30), (40001, 650, 16)])
+def test_long_products(m, n, r):
+    # the products over the rows (A^T Q) are results: with 6 or 7 tiles a row chunk's
+    # FP32 sums run over 256 rows (tiles that divide the SMs have longer chunks).  3 products of 16 rows
+    # a step: 48 sums, each cut by at most 2^-23 of the running sum: 2.9e-6 on
+    # average, one unit of the factors' rounding besides
+    import pyloworder_gb300 as P
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n)
+    U = torch.linalg.qr(torch.randn(m, r, generator=g, device="cuda", dtype=torch.float64))[0]
+    V = torch.linalg.qr(torch.randn(n, r, generator=g, device="cuda", dtype=torch.float64))[0]
+    S = 0.8 ** torch.arange(r, device="cuda", dtype=torch.float64)
+    A = ((U * S) @ V.T).float()
+    s = P.vmmath.randomized_svd(A, r + 4, 1, seed=1)[1]
+    s = torch.as_tensor(np.asarray(s.cpu() if hasattr(s, "cpu") else s)).double()[:r]
+    assert float((s - S.cpu()).norm() / S.cpu().norm()) < 4e-6
