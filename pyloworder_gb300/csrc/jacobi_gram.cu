@@ -4,13 +4,13 @@
 // Rotating column pairs one by one costs a dot product over the whole column, a
 // warp reduction and a barrier per round (1,900 to 2,800 cycles at 301 to 512
 // columns), and moves every column of V along.  Here a block step
-//   1. forms the Gram matrix of its 2 b columns (2 b <= 32) once,
+//   1. forms the Gram matrix of its 2 b columns (2 b <= 32) once (after a sweep's
+//      first step only the cross part: the blocks bring their own along),
 //   2. runs the step's rounds of rotations on that matrix alone: one thread per
 //      pair derives (c, s), then one thread per 2 x 2 block updates it (two CTA
 //      barriers, ~400 cycles a round, whatever the column length), while the
 //      other threads accumulate the 2 b x 2 b rotation product J,
-//   3. multiplies the columns by J, storing them straight where the next step
-//      needs them, and writes J to memory.
+//   3. multiplies the columns by J and writes J to memory.
 // V = product of all J is formed afterwards by a kernel whose CTAs own rows of V:
 // a row passes through every step's J without any exchange.
 // The dot products are those of the columns themselves at every step, so small
@@ -20,8 +20,8 @@
 // sweep's first) is that of the column-by-column kernels.
 //
 //  cluster form: 16 CTAs, two blocks of b columns each (up to 512 columns);
-//    step 3 stores into the next owners' shared memory (two buffers, one cluster
-//    barrier a step).
+//    the blocks go to their next owners by bulk copies through distributed
+//    shared memory (two buffers).
 //  grid form: one CTA per pair of 8-column blocks, through L2, with a release
 //    flag per block (larger problems).
 #include <cooperative_groups.h>
@@ -58,10 +58,41 @@ struct JgArgs {
   unsigned *cmax, *tmax;
 };
 
-// Gram matrix of TB columns of `len` (a multiple of 128) values: warps take 4 x 4
+__device__ __forceinline__ float jg_rsqrt(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float jg_sqrt(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// sums 16 values over the warp, halving the values held at each of 4 steps: lanes
+// 2 q and 2 q + 1 return value q'
+__device__ __forceinline__ float jg_sum16(float (&acc)[16], int lane, int& q) {
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int o = 16 >> s, h = 8 >> s;  // lane distance, values kept
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k >= h) continue;
+      const float send = up ? acc[k] : acc[k + h];
+      const float keep = up ? acc[k + h] : acc[k];
+      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  q = lane >> 1;  // lane bits 4, 3, 2, 1 are the bits 3, 2, 1, 0 of the value's index
+  return acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+}
+
+// Gram matrix of TB columns of `pitch` values: warps take 4 x 4
 // blocks of it, lanes 16-byte vectors of the columns
 template <int TB>
-__device__ __forceinline__ void jg_gram(const float* X, int pitch, float (*G)[TB + 1]) {
+__device__ __forceinline__ void jg_gram(const float* X0, const float* X1, int pitch,
+                                        float (*G)[TB + 1]) {
   constexpr int NB = TB / 4, NT = NB * (NB + 1) / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t = warp; t < NT; t += JG_THREADS / 32) {
@@ -78,8 +109,9 @@ __device__ __forceinline__ void jg_gram(const float* X, int pitch, float (*G)[TB
       float4 x[4], y[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        x[q] = reinterpret_cast<const float4*>(X + (size_t)(4 * bi + q) * pitch)[v];
-        y[q] = reinterpret_cast<const float4*>(X + (size_t)(4 * bj + q) * pitch)[v];
+        const int ci = 4 * bi + q, cj = 4 * bj + q;
+        x[q] = reinterpret_cast<const float4*>(ci < TB / 2 ? X0 + (size_t)ci * pitch : X1 + (size_t)(ci - TB / 2) * pitch)[v];
+        y[q] = reinterpret_cast<const float4*>(cj < TB / 2 ? X0 + (size_t)cj * pitch : X1 + (size_t)(cj - TB / 2) * pitch)[v];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -87,24 +119,9 @@ __device__ __forceinline__ void jg_gram(const float* X, int pitch, float (*G)[TB
         for (int j = 0; j < 4; ++j)
           acc[4 * i + j] = fmaf(x[i].x, y[j].x, fmaf(x[i].y, y[j].y, fmaf(x[i].z, y[j].z, fmaf(x[i].w, y[j].w, acc[4 * i + j]))));
     }
-    // sum 16 values over the warp: halve the values held at each of 4 steps,
-    // then add the two half-warps
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int o = 16 >> s, h = 8 >> s;  // lane distance, values kept
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        if (q >= h) continue;
-        const float send = up ? acc[q] : acc[q + h];
-        const float keep = up ? acc[q + h] : acc[q];
-        acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    }
-    const float g = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    int q;
+    const float g = jg_sum16(acc, lane, q);
     if ((lane & 1) == 0) {
-      // lane bits 4, 3, 2, 1 select value bits 3, 2, 1, 0
-      const int q = (((lane >> 4) & 1) << 3) | (((lane >> 3) & 1) << 2) | (((lane >> 2) & 1) << 1) | ((lane >> 1) & 1);
       const int i = 4 * bi + (q >> 2), j = 4 * bj + (q & 3);
       G[i][j] = g;
       G[j][i] = g;
@@ -112,94 +129,276 @@ __device__ __forceinline__ void jg_gram(const float* X, int pitch, float (*G)[TB
   }
 }
 
-// the rounds of one block step on G (TB x TB), accumulating Jt (row = new
-// column); returns in thread k < b its rotations and largest |t| above the floor
-template <int TB>
-__device__ __forceinline__ void jg_rounds(float (*G)[TB + 1], float (*Jt)[TB], float2* cs, int2* pq,
-                                          bool first, float tol, float floor2, int& rot,
-                                          float& tmax) {
-  constexpr int B = TB / 2;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < TB * TB; e += JG_THREADS) Jt[e / TB][e % TB] = (e / TB == e % TB) ? 1.f : 0.f;
-  const int nintra = first ? B - 1 : 0;
-  for (int rd = 0; rd < nintra + B; ++rd) {
-    if (tid < B) {
-      int p, q;
-      if (rd < nintra) {
-        const int h = tid >= B / 2 ? B : 0;
-        rr_pair(rd, tid % (B / 2), B, p, q);
-        p += h;
-        q += h;
+// the cross part X0^T X1 of two blocks of B columns into G (rows 0 .. B - 1,
+// columns B .. 2 B - 1, and mirrored): 4 x 4 tiles, and where these are fewer than
+// the warps, each in S row ranges whose sums meet in `part`
+template <int B>
+__device__ __forceinline__ void jg_cross(const float* X0, const float* X1, int pitch,
+                                         float (*G)[2 * B + 1], float* part) {
+  constexpr int NT = (B + 3) / 4, W = JG_THREADS / 32;
+  constexpr int S = W / (NT * NT) >= 1 ? W / (NT * NT) : 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < NT * NT * S) {
+    const int t = warp / S, sp = warp % S;
+    const int i0 = 4 * (t / NT), j0 = 4 * (t % NT);
+    float acc[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) acc[q] = 0.f;
+    for (int v = lane + 32 * sp; v < pitch / 4; v += 32 * S) {
+      float4 x[4], y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {  // (columns past the block repeat its last one)
+        x[q] = reinterpret_cast<const float4*>(X0 + (size_t)min(i0 + q, B - 1) * pitch)[v];
+        y[q] = reinterpret_cast<const float4*>(X1 + (size_t)min(j0 + q, B - 1) * pitch)[v];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[4 * i + j] = fmaf(x[i].x, y[j].x, fmaf(x[i].y, y[j].y, fmaf(x[i].z, y[j].z, fmaf(x[i].w, y[j].w, acc[4 * i + j]))));
+    }
+    int q;
+    const float g = jg_sum16(acc, lane, q);
+    const int i = i0 + (q >> 2), j = j0 + (q & 3);
+    if ((lane & 1) == 0 && i < B && j < B) {
+      if (S == 1) {
+        G[i][B + j] = g;
+        G[B + j][i] = g;
       } else {
-        p = tid;
-        q = tid + rd - nintra;
-        q = B + (q >= B ? q - B : q);
-      }
-      const float al = G[p][p], be = G[q][q], g = G[p][q];
-      float c = 1.f, s = 0.f, t = 0.f;
-      if (al > 0.f && be > 0.f && fabsf(g) > tol * (al * rsqrtf(al)) * (be * rsqrtf(be))) {
-        const float z = __fdividef(be - al, 2.0f * g);
-        const float az = fabsf(z), w = fmaf(z, z, 1.0f);
-        t = az > 1e18f ? __fdividef(0.5f, z) : copysignf(__fdividef(1.0f, az + w * rsqrtf(w)), z);
-        const float w1 = fmaf(t, t, 1.0f), c0 = rsqrtf(w1);
-        c = fmaf(0.5f * c0, fmaf(-w1 * c0, c0, 1.0f), c0);
-        s = c * t;
-        ++rot;
-        if (fmaxf(al, be) > floor2) tmax = fmaxf(tmax, fabsf(t));
-      }
-      cs[tid] = make_float2(c, s);
-      pq[tid] = make_int2(p, q);
-    }
-    __syncthreads();
-    if (tid < 256) {
-      if (tid < B * B) {
-        const int k = tid / B, l = tid % B;
-        const float2 rk = cs[k], rl = cs[l];
-        const int2 a = pq[k], c = pq[l];
-        const float g00 = G[a.x][c.x], g01 = G[a.x][c.y], g10 = G[a.y][c.x], g11 = G[a.y][c.y];
-        // columns, then rows: x' = c x - s y, y' = s x + c y
-        const float h00 = fmaf(rl.x, g00, -rl.y * g01), h01 = fmaf(rl.y, g00, rl.x * g01);
-        const float h10 = fmaf(rl.x, g10, -rl.y * g11), h11 = fmaf(rl.y, g10, rl.x * g11);
-        float f00 = fmaf(rk.x, h00, -rk.y * h10), f10 = fmaf(rk.y, h00, rk.x * h10);
-        float f01 = fmaf(rk.x, h01, -rk.y * h11), f11 = fmaf(rk.y, h01, rk.x * h11);
-        if (k == l && rk.y != 0.f) f01 = f10 = 0.f;
-        G[a.x][c.x] = f00;
-        G[a.x][c.y] = f01;
-        G[a.y][c.x] = f10;
-        G[a.y][c.y] = f11;
-      }
-    } else {
-      for (int e = tid - 256; e < TB * B; e += 256) {
-        const int l = e / TB, i = e % TB;
-        const float2 r = cs[l];
-        const int2 c = pq[l];
-        const float x = Jt[c.x][i], y = Jt[c.y][i];
-        Jt[c.x][i] = fmaf(r.x, x, -r.y * y);
-        Jt[c.y][i] = fmaf(r.y, x, r.x * y);
+        part[(sp * B + i) * B + j] = g;
       }
     }
+  }
+  if (S > 1) {
     __syncthreads();
+    for (int e = threadIdx.x; e < B * B; e += JG_THREADS) {
+      float g = part[e];
+#pragma unroll
+      for (int k = 1; k < S; ++k) g += part[k * B * B + e];
+      const int i = e / B, j = e % B;
+      G[i][B + j] = g;
+      G[B + j][i] = g;
+    }
   }
 }
 
-// X J for the rows of X (TB columns of `len` values): put(j, r, value)
-template <int TB, typename Put>
-__device__ __forceinline__ void jg_apply(const float* X, int pitch, int len, const float (*Jt)[TB],
-                                         Put&& put) {
-  for (int r = threadIdx.x; r < len; r += JG_THREADS) {
-    float x[TB];
+// one round: the pairs (pt, qt) of thread t < b, (pk, qk) and (pl, ql) of the
+// thread's 2 x 2 block of G, (pj, qj)[u] of its columns of J.  One chain: the
+// diagonal entries, two reciprocal square roots, a barrier, the 2 x 2 blocks (read
+// before the barrier), a barrier.
+template <int TB, int JN>
+__device__ __forceinline__ void jg_round(float (*G)[TB + 1], float (*Jt)[TB], float2* cs, int k,
+                                         int l, int pt, int qt, int pk, int qk, int pl, int ql,
+                                         const int (&pj)[JN], const int (&qj)[JN], float tol,
+                                         float floor2, int& rot, float& tmax) {
+  constexpr int B = TB / 2;
+  const int tid = threadIdx.x;
+  // threads < 256: block (k, l) of G; threads 256 + t: entries of J's columns of pair l
+  const bool gth = tid < B * B, jth = tid >= 256;
+  float g00 = 0.f, g01 = 0.f, g10 = 0.f, g11 = 0.f;
+  float vx[JN], vy[JN];
+  if (gth) {
+    g00 = G[pk][pl];
+    g01 = G[pk][ql];
+    g10 = G[qk][pl];
+    g11 = G[qk][ql];
+  } else if (jth) {
 #pragma unroll
-    for (int i = 0; i < TB; ++i) x[i] = X[(size_t)i * pitch + r];
-#pragma unroll 4
-    for (int j = 0; j < TB; ++j) {
-      float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-      for (int i = 0; i < TB; i += 4) {
-        const float4 c = *reinterpret_cast<const float4*>(&Jt[j][i]);
-        a0 = fmaf(x[i], c.x, fmaf(x[i + 2], c.z, a0));
-        a1 = fmaf(x[i + 1], c.y, fmaf(x[i + 3], c.w, a1));
+    for (int u = 0; u < JN; ++u) {
+      const int e = tid - 256 + 256 * u;
+      vx[u] = vy[u] = 0.f;
+      if (e < TB * B) {
+        vx[u] = Jt[pj[u]][e % TB];
+        vy[u] = Jt[qj[u]][e % TB];
       }
-      put(j, r, a0 + a1);
+    }
+  }
+  if (tid < B) {
+    const float al = G[pt][pt], be = G[qt][qt], g = G[pt][qt];
+    float c = 1.f, s = 0.f;
+    // half angles: with h = sqrt((be - al)^2 + 4 g^2), cos^2 = (1 + |be - al| / h) / 2
+    // and sin = g / (h cos), two reciprocal square roots deep; scaled by the
+    // power of two of the larger norm
+    const uint32_t eb = __float_as_uint(fmaxf(al, be)) & 0x7f800000u;
+    const float sc = __uint_as_float(0x7f000000u - eb);
+    const float d = (be - al) * sc, g2 = 2.f * g * sc;
+    const float w = fmaf(d, d, g2 * g2);
+    const float rs = jg_rsqrt(w);
+    const float c2 = fmaf(0.5f * fabsf(d), rs, 0.5f);
+    const float rc = jg_rsqrt(c2);
+    const float thr = tol * jg_sqrt(al * be);
+    if (al > 0.f && be > 0.f && fabsf(g) > thr && w > 1e-35f) {
+      c = c2 * rc;
+      s = copysignf(0.5f, d) * g2 * (rs * rc);
+      const float t = fabsf(s * rc);
+      // c^2 + s^2 = 1 to FP32: the products of thousands of rotations stay orthogonal
+      const float h = 0.5f * (fmaf(-c, c, 1.f) - s * s);
+      c = fmaf(c, h, c);
+      s = fmaf(s, h, s);
+      ++rot;
+      if (fmaxf(al, be) > floor2) tmax = fmaxf(tmax, t);
+    }
+    cs[tid] = make_float2(c, s);
+  }
+  __syncthreads();
+  if (gth) {
+    const float2 rk = cs[k], rl = cs[l];
+    // columns, then rows: x' = c x - s y, y' = s x + c y
+    const float h00 = fmaf(rl.x, g00, -rl.y * g01), h01 = fmaf(rl.y, g00, rl.x * g01);
+    const float h10 = fmaf(rl.x, g10, -rl.y * g11), h11 = fmaf(rl.y, g10, rl.x * g11);
+    const bool dg = k == l && rk.y != 0.f;
+    G[pk][pl] = fmaf(rk.x, h00, -rk.y * h10);
+    G[qk][pl] = dg ? 0.f : fmaf(rk.y, h00, rk.x * h10);
+    G[pk][ql] = dg ? 0.f : fmaf(rk.x, h01, -rk.y * h11);
+    G[qk][ql] = fmaf(rk.y, h01, rk.x * h11);
+  } else if (jth) {
+#pragma unroll
+    for (int u = 0; u < JN; ++u) {
+      const int e = tid - 256 + 256 * u;
+      if (e < TB * B) {
+        const float2 r = cs[e / TB];
+        Jt[pj[u]][e % TB] = fmaf(r.x, vx[u], -r.y * vy[u]);
+        Jt[qj[u]][e % TB] = fmaf(r.y, vx[u], r.x * vy[u]);
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// the rounds of one block step on G (TB x TB), accumulating Jt (row = new
+// column); adds to rot and tmax in thread t < b
+template <int TB>
+__device__ __forceinline__ void jg_rounds(float (*G)[TB + 1], float (*Jt)[TB], float2* cs,
+                                          bool first, float tol, float floor2, int& rot,
+                                          float& tmax) {
+  constexpr int B = TB / 2, JN = (TB * B + 255) / 256;
+  const int tid = threadIdx.x;
+  for (int e = tid; e < TB * TB; e += JG_THREADS) Jt[e / TB][e % TB] = (e / TB == e % TB) ? 1.f : 0.f;
+  __syncthreads();
+  const int t = tid < B ? tid : 0;
+  const int k = tid < B * B ? tid / B : 0, l = tid < B * B ? tid % B : 0;
+  int lj[JN], pj[JN], qj[JN];
+#pragma unroll
+  for (int u = 0; u < JN; ++u) lj[u] = tid >= 256 ? min((tid - 256 + 256 * u) / TB, B - 1) : 0;
+  int pt, qt, pk, qk, pl, ql;
+  if (first) {  // inside the two blocks
+    auto pair = [&](int rd, int x, int& p, int& q) {
+      const int h = x >= B / 2 ? B : 0;
+      rr_pair(rd, h ? x - B / 2 : x, B, p, q);
+      p += h;
+      q += h;
+    };
+    for (int rd = 0; rd < B - 1; ++rd) {
+      pair(rd, t, pt, qt);
+      pair(rd, k, pk, qk);
+      pair(rd, l, pl, ql);
+#pragma unroll
+      for (int u = 0; u < JN; ++u) pair(rd, lj[u], pj[u], qj[u]);
+      jg_round<TB, JN>(G, Jt, cs, k, l, pt, qt, pk, qk, pl, ql, pj, qj, tol, floor2, rot, tmax);
+    }
+  }
+  // across: column x of the first block with column (x + round) mod b of the second
+  qt = B + t;
+  qk = B + k;
+  ql = B + l;
+#pragma unroll
+  for (int u = 0; u < JN; ++u) {
+    pj[u] = lj[u];
+    qj[u] = B + lj[u];
+  }
+  auto next = [](int& q) { q = q + 1 == 2 * B ? B : q + 1; };
+#pragma unroll 1
+  for (int rd = 0; rd < B; ++rd) {
+    jg_round<TB, JN>(G, Jt, cs, k, l, t, qt, k, qk, l, ql, pj, qj, tol, floor2, rot, tmax);
+    next(qt);
+    next(qk);
+    next(ql);
+#pragma unroll
+    for (int u = 0; u < JN; ++u) next(qj[u]);
+  }
+}
+
+// J out: transposed to global memory (row = new column, for the rows of V) and as
+// it is to Jn (row = old column, for jg_apply)
+template <int TB>
+__device__ __forceinline__ void jg_out(const float (*Jt)[TB], float (*Jn)[TB], float* Jo) {
+  for (int e = threadIdx.x; e < TB * TB; e += JG_THREADS) {
+    const float v = Jt[e / TB][e % TB];
+    Jo[e] = v;
+    Jn[e % TB][e / TB] = v;
+  }
+}
+
+// X <- X J in place: a thread takes RT rows of CT new columns.  A 16-byte shared read
+// costs four cycles of the SM's return path even when all lanes read the same
+// address, so the tile, not the FMA count, sets the pace: 8 x 8 reads 4 vectors for
+// 64 FMAs (8 x 4: 3 for 32; one row a thread: 8 for 32).  8 x 8 at blocks of 16
+// columns (10.2k cycles a step at n = 512, 12.1k with 8 x 4), 8 x 4 where 8 x 8 leaves
+// more than half of the threads idle (n = 256: 2.0k, 2.4k).  Column i + 1 is read
+// before column i is used.
+template <int TB, int RT, int CT>
+__device__ __forceinline__ void jg_apply(float* X0, float* X1, int pitch, const float (*Jn)[TB]) {
+  constexpr int B = TB / 2, NG = TB / CT, RV = RT / 4, CV = CT / 4;
+  const int groups = pitch / RT * NG;
+  const int rounds = (groups + JG_THREADS - 1) / JG_THREADS;
+  for (int rd = 0; rd < rounds; ++rd) {  // (rows of different rounds are apart)
+    const int t = threadIdx.x + rd * JG_THREADS;
+    const bool live = t < groups;
+    const int j0 = (t % NG) * CT, r = (t / NG) * RT;
+    float4 y[CT][RV];
+#pragma unroll
+    for (int c = 0; c < CT; ++c)
+#pragma unroll
+      for (int v = 0; v < RV; ++v) y[c][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) {
+      const float* src = X0 + r;
+      const float* jn = &Jn[0][j0];
+      float4 xn[RV], jv[CV];
+#pragma unroll
+      for (int v = 0; v < CV; ++v) jv[v] = *reinterpret_cast<const float4*>(jn + 4 * v);
+#pragma unroll
+      for (int v = 0; v < RV; ++v) xn[v] = *reinterpret_cast<const float4*>(src + 4 * v);
+#pragma unroll 2
+      for (int i = 0; i < TB; ++i) {
+        float cj[CT];
+        float4 x[RV];
+#pragma unroll
+        for (int v = 0; v < CV; ++v) {
+          cj[4 * v] = jv[v].x;
+          cj[4 * v + 1] = jv[v].y;
+          cj[4 * v + 2] = jv[v].z;
+          cj[4 * v + 3] = jv[v].w;
+        }
+#pragma unroll
+        for (int v = 0; v < RV; ++v) x[v] = xn[v];
+        if (i + 1 < TB) {
+          src = i + 1 == B ? X1 + r : src + pitch;
+          jn += TB;
+#pragma unroll
+          for (int v = 0; v < CV; ++v) jv[v] = *reinterpret_cast<const float4*>(jn + 4 * v);
+#pragma unroll
+          for (int v = 0; v < RV; ++v) xn[v] = *reinterpret_cast<const float4*>(src + 4 * v);
+        }
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+#pragma unroll
+          for (int v = 0; v < RV; ++v) {
+            y[c][v].x = fmaf(x[v].x, cj[c], y[c][v].x);
+            y[c][v].y = fmaf(x[v].y, cj[c], y[c][v].y);
+            y[c][v].z = fmaf(x[v].z, cj[c], y[c][v].z);
+            y[c][v].w = fmaf(x[v].w, cj[c], y[c][v].w);
+          }
+      }
+    }
+    __syncthreads();  // the rows' other column groups have read them
+    if (live) {
+#pragma unroll
+      for (int c = 0; c < CT; ++c) {
+        const int j = j0 + c;
+        float* dst = (j < B ? X0 + (size_t)j * pitch : X1 + (size_t)(j - B) * pitch) + r;
+#pragma unroll
+        for (int v = 0; v < RV; ++v) reinterpret_cast<float4*>(dst)[v] = y[c][v];
+      }
     }
   }
 }
@@ -225,29 +424,59 @@ __device__ __forceinline__ double jg_scale(unsigned long long mx) {
   return ldexp(1.0, -ex);
 }
 
+// bounded wait for a phase of an mbarrier
+__device__ __forceinline__ bool jg_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok = 0;
+  uint64_t t0 = 0;
+  while (true) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    uint64_t t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    if (t0 == 0) t0 = t1;
+    if (t1 - t0 > JG_WAIT_NS) return false;
+  }
+}
+
+// A block is a region of shared memory: B columns of `pitch` values, then the B x B
+// Gram matrix of the block as its rotations left it.  Between steps whole regions
+// go to their next owners by bulk copies (thread stores to distributed shared
+// memory move 6 bytes a clock), into the other of two buffers; the receiver's
+// barrier counts their bytes.  A cluster barrier, arrived at once a CTA has
+// its regions and waited for before it sends, says that every copy of the step
+// before has landed, so the buffers sent from may be written again.
 template <int TB>
 __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_cluster_kernel(const JgArgs p) {
   constexpr int B = TB / 2, C = JG_CLUSTER, steps = 2 * C - 1;
-  extern __shared__ __align__(16) float jg_sm[];  // two buffers of TB x pitch
+  extern __shared__ __align__(128) float jg_sm[];  // two buffers of two regions
   __shared__ __align__(16) float Jt[TB][TB];
+  __shared__ __align__(16) float Jn[TB][TB];
   __shared__ float G[TB][TB + 1];
+  __shared__ float part[JG_THREADS / 32 * 16];
   __shared__ float2 cs[B];
-  __shared__ int2 pq[B];
   __shared__ unsigned long long mx_sh[C];
   __shared__ int cnt_sh[2][C];
   __shared__ float tm_sh[2][C], cm_sh[2][C];
-  __shared__ int dst_sh[2], rot_sh;
-  __shared__ float tmax_sh;
+  __shared__ int dst_sh[2], abort_sh;
+  __shared__ __align__(8) uint64_t bar;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), tid = threadIdx.x;
   const int n = p.n, pitch = p.pitch;
-  const size_t half = (size_t)TB * pitch;
+  const int region = B * pitch + B * B;  // floats
+  const uint32_t bar_s = (uint32_t)__cvta_generic_to_shared(&bar);
 
   // power-of-two scale: max |a| < 1
   if (tid < C) mx_sh[tid] = 0ull;
   if (tid == 0) {
-    rot_sh = 0;
-    tmax_sh = 0.f;
+    abort_sh = 0;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_s));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   {
@@ -268,19 +497,32 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_cluster_kernel(cons
     for (int e = tid; e < TB * pitch; e += JG_THREADS) {
       const int j = e / pitch, i = e % pitch;
       const int col = (j < B ? b0 : b1) * B + j % B;
-      jg_sm[e] = (col < n && i < n) ? (float)(p.A[(int64_t)col * n + i] * sc) : 0.f;
+      jg_sm[(j / B) * region + (j % B) * pitch + i] =
+          (col < n && i < n) ? (float)(p.A[(int64_t)col * n + i] * sc) : 0.f;
     }
   }
   __syncthreads();
 
   float cmax_prev = 0.f;
   int sweep = 0, cur = 0;
+  uint32_t phase = 0;
   for (; sweep < p.max_sweeps; ++sweep) {
     int rot = 0;
     float tmax = 0.f, cmax = 0.f;
     const float floor2 = sweep > 0 ? p.floor * p.floor * cmax_prev : 3.0e38f;
     for (int step = 0; step < steps; ++step) {
-      const float* X = jg_sm + (size_t)cur * half;
+      float* X0 = jg_sm + (size_t)cur * 2 * region;
+      float* X1 = X0 + region;
+      if (sweep > 0 || step > 0) {  // this step's regions
+        if (!abort_sh && !jg_wait(bar_s, phase)) abort_sh = 1;
+        phase ^= 1u;
+        __syncthreads();
+      }
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      if (tid == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_s),
+                     "r"((uint32_t)(2 * region * sizeof(float)))
+                     : "memory");
       // where this CTA's blocks go next
       if (tid < 32) {
         int b0, b1, a = -1, b = -1;
@@ -294,23 +536,44 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_cluster_kernel(cons
           if (tid == 0) dst_sh[side] = ma ? 2 * (__ffs(ma) - 1) : 2 * (__ffs(mb) - 1) + 1;
         }
       }
-      jg_gram<TB>(X, pitch, G);
+      // the Gram matrix: all of it at a sweep's first step, else the cross part
+      // beside the blocks' own
+      if (step == 0) {
+        jg_gram<TB>(X0, X1, pitch, G);
+      } else {
+        for (int e = tid; e < 2 * B * B; e += JG_THREADS) {
+          const int side = e / (B * B), r = e % (B * B);
+          G[side * B + r / B][side * B + r % B] = (side ? X1 : X0)[B * pitch + r];
+        }
+        jg_cross<B>(X0, X1, pitch, G, part);
+      }
       __syncthreads();
       if (step == 0 && tid < TB) cmax = fmaxf(cmax, G[tid][tid]);
-      jg_rounds<TB>(G, Jt, cs, pq, step == 0, p.tol, floor2, rot, tmax);
+      jg_rounds<TB>(G, Jt, cs, step == 0, p.tol, floor2, rot, tmax);
       float* Jo = p.J + (((int64_t)sweep * steps + step) * C + rank) * TB * TB;
-      for (int e = tid; e < TB * TB / 4; e += JG_THREADS)
-        reinterpret_cast<float4*>(Jo)[e] = reinterpret_cast<const float4*>(&Jt[0][0])[e];
-      float* dst[2];
-#pragma unroll
-      for (int side = 0; side < 2; ++side)
-        dst[side] = cl.map_shared_rank(jg_sm, dst_sh[side] >> 1) + (size_t)(cur ^ 1) * half +
-                    (size_t)(dst_sh[side] & 1) * B * pitch;
-      jg_apply<TB>(X, pitch, pitch, Jt, [&](int j, int r, float v) {
-        (j < B ? dst[0] + (size_t)j * pitch : dst[1] + (size_t)(j - B) * pitch)[r] = v;
-      });
+      jg_out<TB>(Jt, Jn, Jo);
+      __syncthreads();
+      jg_apply<TB, 8, (TB == 32 ? 8 : 4)>(X0, X1, pitch, Jn);
+      for (int e = tid; e < 2 * B * B; e += JG_THREADS) {
+        const int side = e / (B * B), r = e % (B * B);
+        (side ? X1 : X0)[B * pitch + r] = G[side * B + r / B][side * B + r % B];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
       cur ^= 1;
-      cl.sync();
+      if (tid < 2) {
+        const int d = dst_sh[tid];
+        uint32_t dst, rbar;
+        const uint32_t ldst = (uint32_t)__cvta_generic_to_shared(jg_sm + (size_t)(2 * cur + (d & 1)) * region);
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(ldst), "r"(d >> 1));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(bar_s), "r"(d >> 1));
+        asm volatile(
+            "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+            "r"((uint32_t)__cvta_generic_to_shared(tid ? X1 : X0)),
+            "r"((uint32_t)(region * sizeof(float))), "r"(rbar)
+            : "memory");
+      }
     }
     // rotations, angles and norms of the sweep over the cluster
     if (tid < 32) {
@@ -338,26 +601,35 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_cluster_kernel(cons
     if (total == 0) break;
     if (sweep > 0 && tall <= p.tstop) break;
   }
+  // the last step's regions land before any CTA leaves
+  if (!abort_sh && !jg_wait(bar_s, phase)) abort_sh = 1;
+  __syncthreads();
+  if (tid == 0 && abort_sh) atomicMax(&p.info[ST_FAIL], PLOM_NUM_TIMEOUT);
   if (rank == 0 && tid == 0) {
     const int done = sweep < p.max_sweeps ? sweep + 1 : sweep;
     p.info[ST_SWEEPS32] = done;
     *p.nsteps = done * steps;
   }
+  cl.sync();
 }
 
 // the grid form: CTA k takes block pair k of every step
 template <int TB>
 __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_grid_kernel(const JgArgs p) {
   constexpr int B = TB / 2;
-  extern __shared__ __align__(16) float jg_sm[];  // TB x pitch
+  extern __shared__ __align__(128) float jg_sm[];  // two regions
   __shared__ __align__(16) float Jt[TB][TB];
+  __shared__ __align__(16) float Jn[TB][TB];
   __shared__ float G[TB][TB + 1];
+  __shared__ float part[JG_THREADS / 32 * 16];
   __shared__ float2 cs[B];
-  __shared__ int2 pq[B];
   __shared__ int abort_sh;
   cg::grid_group grid = cg::this_grid();
   const int n = p.n, pitch = p.pitch, nblk = p.nblk, steps = nblk - 1;
   const int tid = threadIdx.x, rank = blockIdx.x;
+  const int region = B * pitch + B * B;  // floats; block k's region at At + k region
+  float* X0 = jg_sm;
+  float* X1 = jg_sm + region;
   const int64_t gtid = (int64_t)blockIdx.x * JG_THREADS + tid, gth = (int64_t)gridDim.x * JG_THREADS;
   if (tid == 0) abort_sh = 0;
   if (gtid == 0) {
@@ -383,7 +655,8 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_grid_kernel(const J
     for (int e = tid; e < TB * pitch; e += JG_THREADS) {
       const int j = e / pitch, i = e % pitch;
       const int col = (j < B ? b0 : b1) * B + j % B;
-      jg_sm[e] = (col < n && i < n) ? (float)(p.A[(int64_t)col * n + i] * sc) : 0.f;
+      jg_sm[(j / B) * region + (j % B) * pitch + i] =
+          (col < n && i < n) ? (float)(p.A[(int64_t)col * n + i] * sc) : 0.f;
     }
   }
   __syncthreads();
@@ -424,25 +697,39 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_grid_kernel(const J
           __syncthreads();
           continue;
         }
-        const int pv = pitch / 4;
-        for (int e = tid; e < TB * pv; e += JG_THREADS) {
-          const int j = e / pv, v = e % pv;
-          const int col = (j < B ? b0 : b1) * B + j % B;
-          reinterpret_cast<float4*>(jg_sm)[e] =
-              __ldcg(reinterpret_cast<const float4*>(p.At + (int64_t)col * pitch) + v);
-        }
+        const int rv = region / 4;
+#pragma unroll 4
+        for (int e = tid; e < 2 * rv; e += JG_THREADS)
+          reinterpret_cast<float4*>(jg_sm)[e] = __ldcg(
+              reinterpret_cast<const float4*>(p.At + (int64_t)(e < rv ? b0 : b1) * region) + (e < rv ? e : e - rv));
         __syncthreads();
       }
-      jg_gram<TB>(jg_sm, pitch, G);
+      if (step == 0) {
+        jg_gram<TB>(X0, X1, pitch, G);
+      } else {
+        for (int e = tid; e < 2 * B * B; e += JG_THREADS) {
+          const int side = e / (B * B), r = e % (B * B);
+          G[side * B + r / B][side * B + r % B] = (side ? X1 : X0)[B * pitch + r];
+        }
+        jg_cross<B>(X0, X1, pitch, G, part);
+      }
       __syncthreads();
       if (step == 0 && tid < TB) cmax = fmaxf(cmax, G[tid][tid]);
-      jg_rounds<TB>(G, Jt, cs, pq, step == 0, p.tol, floor2, rot, tmax);
-      jg_apply<TB>(jg_sm, pitch, pitch, Jt, [&](int j, int r, float v) {
-        p.At[(int64_t)((j < B ? b0 : b1) * B + j % B) * pitch + r] = v;
-      });
-      float* Jo = p.J + ((int64_t)gstep * (nblk / 2) + rank) * TB * TB;
-      for (int e = tid; e < TB * TB / 4; e += JG_THREADS)
-        reinterpret_cast<float4*>(Jo)[e] = reinterpret_cast<const float4*>(&Jt[0][0])[e];
+      jg_rounds<TB>(G, Jt, cs, step == 0, p.tol, floor2, rot, tmax);
+      jg_out<TB>(Jt, Jn, p.J + ((int64_t)gstep * (nblk / 2) + rank) * TB * TB);
+      __syncthreads();
+      jg_apply<TB, 8, 4>(X0, X1, pitch, Jn);
+      for (int e = tid; e < 2 * B * B; e += JG_THREADS) {
+        const int side = e / (B * B), r = e % (B * B);
+        (side ? X1 : X0)[B * pitch + r] = G[side * B + r / B][side * B + r % B];
+      }
+      __syncthreads();
+      {
+        const int rv = region / 4;
+        for (int e = tid; e < 2 * rv; e += JG_THREADS)
+          __stcg(reinterpret_cast<float4*>(p.At + (int64_t)(e < rv ? b0 : b1) * region) + (e < rv ? e : e - rv),
+                 reinterpret_cast<const float4*>(jg_sm)[e]);
+      }
       __syncthreads();
       if (tid == 0) {
         __threadfence();
@@ -474,27 +761,31 @@ __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_grid_kernel(const J
   }
 }
 
-// V = J_1 J_2 ... row by row: a CTA holds `R` rows of V and takes them through the
-// block pairs of every step, the next step's J arriving while one is applied.
-// Out: V (n x n row-major).
+// V = J_1 J_2 ... row by row: a CTA holds `R` rows of V (twice) and takes them
+// through the block pairs of every step, the next step's J arriving while one is
+// applied; a thread forms 4 outputs of one row and pair.  J's rows are padded by
+// 16 bytes (their reads by a quarter warp fall on different banks).  Out: V
+// (n x n row-major).
 template <int TB>
 __global__ void __launch_bounds__(256) jacobi_rows_kernel(const float* __restrict__ J,
                                                           const int* __restrict__ nsteps, int n,
                                                           int nblk, int R, float* __restrict__ V) {
-  constexpr int B = TB / 2, OUT = 4;  // outputs a thread forms at a time
+  constexpr int B = TB / 2, JP = TB + 4, OG = TB / 4;
   extern __shared__ __align__(16) float jr_sm[];
   const int pairs = nblk / 2, steps = nblk - 1, ncol = nblk * B;
-  const int jsz = pairs * TB * TB;       // floats of J per step
+  const int jsz = pairs * TB * JP;       // floats of J per step
   float* jb = jr_sm;                     // [2][jsz]
-  float* v = jr_sm + 2 * (size_t)jsz;    // [R][ncol]
+  const int vp = ncol + 10;              // rows on different banks
+  float* vb = jr_sm + 2 * (size_t)jsz;   // [2][R][vp]
   const int tid = threadIdx.x, r0 = blockIdx.x * R;
   const int total = *nsteps;
-  for (int e = tid; e < R * ncol; e += 256) v[e] = (r0 + e / ncol == e % ncol) ? 1.f : 0.f;
+  for (int e = tid; e < R * ncol; e += 256)
+    vb[(e / ncol) * vp + e % ncol] = (r0 + e / ncol == e % ncol) ? 1.f : 0.f;
   auto fetch = [&](int s, int buf) {
-    const float4* src = reinterpret_cast<const float4*>(J + (int64_t)s * jsz);
+    const float4* src = reinterpret_cast<const float4*>(J + (int64_t)s * pairs * TB * TB);
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(jb + (size_t)buf * jsz);
-    for (int e = tid; e < jsz / 4; e += 256)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + e) : "memory");
+    for (int e = tid; e < pairs * TB * OG; e += 256)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4 * (e / OG * JP + e % OG * 4)), "l"(src + e) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   if (total > 0) fetch(0, 0);
@@ -507,42 +798,43 @@ __global__ void __launch_bounds__(256) jacobi_rows_kernel(const float* __restric
     }
     __syncthreads();
     const float* js = jb + (size_t)(s & 1) * jsz;
-    // a thread takes all TB outputs of one row and pair: rows of a pair's J are
-    // shared by the R threads next to each other
-    for (int it = tid; it < R * pairs; it += 256) {
-      const int k = it / R, r = it % R;
+    const float* vi = vb + (size_t)(s & 1) * R * vp;
+    float* vo = vb + (size_t)((s + 1) & 1) * R * vp;
+    for (int it = tid; it < R * OG * pairs; it += 256) {
+      const int r = it % R, q = it / R, k = q / OG, j = 4 * (q % OG);
       int b0, b1;
       rr_pair(s % steps, k, nblk, b0, b1);
-      float* x0 = v + (size_t)r * ncol + b0 * B;
-      float* x1 = v + (size_t)r * ncol + b1 * B;
-      float x[TB];
+      const float* x0 = vi + (size_t)r * vp + b0 * B;
+      const float* x1 = vi + (size_t)r * vp + b1 * B;
+      const float* jk = js + (size_t)(k * TB + j) * JP;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < B; ++i) {
-        x[i] = x0[i];
-        x[B + i] = x1[i];
-      }
-      const float* jk = js + (size_t)k * TB * TB;
-#pragma unroll 2
-      for (int j = 0; j < TB; j += OUT) {
-        float a[OUT];
+      for (int i = 0; i < TB; i += 4) {
+        float x[4];
 #pragma unroll
-        for (int u = 0; u < OUT; ++u) {
-          a[u] = 0.f;
-#pragma unroll
-          for (int i = 0; i < TB; i += 4) {
-            const float4 c = *reinterpret_cast<const float4*>(jk + (j + u) * TB + i);
-            a[u] = fmaf(x[i], c.x, fmaf(x[i + 1], c.y, fmaf(x[i + 2], c.z, fmaf(x[i + 3], c.w, a[u]))));
-          }
+        for (int u = 0; u < 4; u += 2) {  // (B is even: 8-byte reads)
+          const float2 t = *reinterpret_cast<const float2*>(i + u < B ? x0 + i + u : x1 + i + u - B);
+          x[u] = t.x;
+          x[u + 1] = t.y;
         }
 #pragma unroll
-        for (int u = 0; u < OUT; ++u) (j + u < B ? x0[j + u] : x1[j + u - B]) = a[u];
+        for (int u = 0; u < 4; ++u) {
+          const float4 c = *reinterpret_cast<const float4*>(jk + u * JP + i);
+          a[u] = fmaf(x[0], c.x, fmaf(x[1], c.y, fmaf(x[2], c.z, fmaf(x[3], c.w, a[u]))));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = j + u;
+        vo[(size_t)r * vp + (c < B ? b0 * B + c : b1 * B + c - B)] = a[u];
       }
     }
     __syncthreads();
   }
+  const float* v = vb + (size_t)(total & 1) * R * vp;
   for (int e = tid; e < R * n; e += 256) {
     const int r = e / n, c = e % n;
-    if (r0 + r < n) V[(int64_t)(r0 + r) * n + c] = v[(size_t)r * ncol + c];
+    if (r0 + r < n) V[(int64_t)(r0 + r) * n + c] = v[(size_t)r * vp + c];
   }
 }
 
@@ -568,7 +860,7 @@ static void jg_kernels(JgPlan& pl) {
 // values twice, 131 KiB); beyond, 8-column blocks with one CTA per pair.
 static bool jg_plan(JgPlan& pl, int n) {
   if (n < 1 || n > 1600) return false;
-  pl.pitch = (int)(cdiv(n, 128) * 128);
+  pl.pitch = (int)(cdiv(n, 16) * 16);
   pl.cluster = n <= 512;
   if (pl.cluster) {
     pl.nblk = 2 * JG_CLUSTER;
@@ -581,18 +873,20 @@ static bool jg_plan(JgPlan& pl, int n) {
       case 7: jg_kernels<28>(pl); break;
       default: jg_kernels<32>(pl); break;
     }
-    pl.smem = (size_t)2 * pl.TB * pl.pitch * sizeof(float);
+    pl.smem = (size_t)4 * (pl.TB / 2) * (pl.pitch + pl.TB / 2) * sizeof(float);
   } else {
     const int nb = (int)cdiv(n, 8);
     pl.nblk = std::max(2, nb + (nb & 1));
     jg_kernels<16>(pl);
-    pl.smem = (size_t)16 * pl.pitch * sizeof(float);
+    pl.smem = (size_t)16 * (pl.pitch + 8) * sizeof(float);
     if (pl.nblk / 2 > num_sms()) return false;
   }
-  // rows of V per CTA: two CTAs' worth of rows per SM at most, J twice beside them
-  pl.R = (int)std::max<int64_t>(1, std::min<int64_t>(8, cdiv(n, num_sms())));
-  pl.rows_smem = ((size_t)2 * (pl.nblk / 2) * pl.TB * pl.TB + (size_t)pl.R * pl.nblk * (pl.TB / 2)) *
-                 sizeof(float);
+  // rows of V per CTA: one wave of CTAs, as far as they fit beside two steps' J
+  for (pl.R = (int)std::max<int64_t>(1, std::min<int64_t>(8, cdiv(n, num_sms())));; --pl.R) {
+    pl.rows_smem = ((size_t)2 * (pl.nblk / 2) * pl.TB * (pl.TB + 4) +
+                    (size_t)2 * pl.R * (pl.nblk * (pl.TB / 2) + 10)) * sizeof(float);
+    if (pl.rows_smem <= 220 * 1024 || pl.R == 1) break;
+  }
   return pl.rows_smem <= 220 * 1024;
 }
 
@@ -646,7 +940,7 @@ int jacobi_gram_f32(const double* A, int n, float tol, float floor_rel, float ts
   a.J = ws.take<float>((size_t)JG_MAX_SWEEPS * steps * pairs * pl.TB * pl.TB);
   a.nsteps = ws.take<int>(1);
   if (!pl.cluster) {
-    a.At = ws.take<float>((size_t)pl.nblk * (pl.TB / 2) * pl.pitch);
+    a.At = ws.take<float>((size_t)pl.nblk * (pl.TB / 2) * (pl.pitch + pl.TB / 2));
     a.bflag = ws.take<int>(pl.nblk);
     a.abortf = ws.take<int>(1);
     a.counts = ws.take<int>(JG_MAX_SWEEPS);
