@@ -1,0 +1,548 @@
+// FP64 products of the plain form on the tensor cores.
+//
+// GB300 issues two FP64 FMAs per clock and SM (1.2 TFLOP/s), which bound the Grams
+// and applies of the FP64 form: 16,384 x 200 spent 10.8 of 30 ms in them.  An FP64
+// operand, scaled by the power of two of its column's (or row's) largest element,
+// is a 62-bit integer; it is cut into nine signed 7-bit digits, exact in fp16, and
+// the product is the sum of the 45 digit products of weight 128^8 and above (the
+// splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012), with a
+// fixed radix).  A digit product is an integer of at most 12 bits, and a weight's
+// sum over a stage of 32 rows stays below 2^21: exact in the FP32 accumulators,
+// whatever their rounding.  The sums of all stages are kept in two 64-bit integers
+// per output, so a chunk's sum is exact up to the dropped digit products (below
+// 2^-58 of the two scales per row, 2^-61 typically, and of either sign) and is
+// rounded once: what an FP64 accumulation loses at every addition is not lost.
+// Power-of-two scales per column (and per row in oz_nn) keep graded operands.
+//
+// The digits are cut in the kernels, in shared memory: no planes are written for
+// the tall operand.  mma.sync and not tcgen05: the nine weights have to be drained
+// into integers every 32 rows, in place, by the threads that own the accumulators;
+// mma.sync's own rate bounds both kernels (2,880 instructions a stage: 11.5 of 13.6k
+// cycles).  16,384 x 200, three Grams: 6.3 ms with FP64 FMAs, 0.83 here; three
+// applies 4.0 ms, 1.1 here.  ||Q^T Q - I|| of the QR factors 1.2-2.4e-15 with FP64
+// FMAs, 4-6e-16 here.
+//
+//  oz_gram  G (N x N) = A^T A, A m x N: upper 64 x 64 tiles x row chunks
+//  oz_nn    C (m x k) = A W, A m x N, W N x k: 64 x 64 tiles
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "plom_common.cuh"
+#include "plom_kernels.cuh"
+
+namespace plom {
+
+namespace oz {
+
+constexpr int D = 9;         // digits
+constexpr int TS = 64;       // output tile
+constexpr int KS = 32;       // rows (columns of A in oz_nn) per stage
+constexpr int THREADS = 512; // 16 warps, 16 x 16 outputs each
+constexpr int PK = TS + 8;   // pitch of a [k][64] plane (conflict-free ldmatrix)
+constexpr int PM = KS + 8;   // pitch of a [64][k] plane
+constexpr int PLANE_K = KS * PK, PLANE_M = TS * PM;  // halves
+constexpr int BUF_G = 2 * D * PLANE_K * 2;             // bytes of a Gram stage
+constexpr int BUF_N = D * (PLANE_M + PLANE_K) * 2;     // bytes of an oz_nn stage
+constexpr int64_t MAX_ROWS = 1 << 22;  // of a chunk: 2^38 a row fits the 64-bit sums
+
+constexpr uint64_t bias_of(int s) { return s < 0 ? 0ull : (64ull << (7 * s)) + bias_of(s - 1); }
+constexpr uint64_t BIAS = bias_of(D - 1);
+
+// |x| = mant 2^(e - 1075); e >= 1 (the exponent field of a double), 2047: not finite
+struct Dec {
+  uint64_t mant;
+  int e;
+  bool neg;
+};
+__device__ __forceinline__ Dec decode(double x) {
+  const uint64_t b = (uint64_t)__double_as_longlong(x);
+  const int f = (int)(b >> 52) & 0x7ff;
+  Dec d;
+  d.mant = (b & 0xfffffffffffffull) | (f ? 1ull << 52 : 0ull);
+  d.e = f ? f : 1;
+  d.neg = (b >> 63) != 0;
+  return d;
+}
+__device__ __forceinline__ Dec decode(float x) {
+  const uint32_t b = __float_as_uint(x);
+  const int f = (int)(b >> 23) & 0xff;
+  // m24 2^(f - 150) = (m24 2^29) 2^(f + 896 - 1075)
+  Dec d;
+  d.mant = (uint64_t)((b & 0x7fffffu) | (f ? 0x800000u : 0u)) << 29;
+  d.e = f == 255 ? 2047 : (f ? f : 1) + 896;
+  d.neg = (b >> 31) != 0;
+  return d;
+}
+// exponent for the scale: 0 for a zero
+__device__ __forceinline__ int scale_exp(const Dec& d) { return d.mant ? d.e : 0; }
+
+// the biased digits of +-mant 2^sh (|.| < 2^61), rounded to an integer
+__device__ __forceinline__ uint64_t fix(const Dec& d, int sh) {
+  uint64_t x;
+  if (sh >= 0) {
+    x = sh > 9 ? 0ull : d.mant << sh;  // (more: not finite, flagged elsewhere)
+  } else {
+    const int r = -sh;
+    x = r > 60 ? 0ull : (d.mant + (1ull << (r - 1))) >> r;
+  }
+  return d.neg ? BIAS - x : BIAS + x;
+}
+// digit planes of two neighbours; p: their place in plane 0, stride in halves
+__device__ __forceinline__ void put2(__half* p, int stride, uint64_t y0, uint64_t y1) {
+  const __half2 off = __half2half2(__ushort_as_half(0x6440));  // 1,088
+#pragma unroll
+  for (int s = 0; s < D; ++s) {
+    const uint32_t u = 0x64006400u | ((uint32_t)(y0 >> (7 * s)) & 127u) |
+                       (((uint32_t)(y1 >> (7 * s)) & 127u) << 16);  // 1,024 + digit + 64
+    __half2 h;
+    *reinterpret_cast<uint32_t*>(&h) = u;
+    *reinterpret_cast<__half2*>(p + s * stride) = __hsub2(h, off);
+  }
+}
+
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// an FP32 integer below 2^22
+__device__ __forceinline__ int to_int(float f) {
+  return __float_as_int(f + 12582912.f) - 0x4b400000;
+}
+
+// the digit products of weights G0 .. G0 + NG - 1 (digit indices added) of one stage;
+// a_addr, b_addr: this lane's ldmatrix address in plane 0 for the stage's first 16 rows
+template <int G0, int NG, bool A_TRANS>
+__device__ __forceinline__ void stage_mma(uint32_t a_addr, uint32_t a_plane, uint32_t a_k16,
+                                          uint32_t b_addr, int64_t (&sum)[8]) {
+  constexpr int SMIN = G0 - (D - 1) > 0 ? G0 - (D - 1) : 0;  // least digit that takes part
+  float acc[NG][2][4];
+#pragma unroll
+  for (int g = 0; g < NG; ++g)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[g][h][i] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < KS / 16; ++kk) {
+    uint32_t b[D - SMIN][4];
+#pragma unroll
+    for (int t = SMIN; t < D; ++t)
+      ldm4t(b[t - SMIN], b_addr + (uint32_t)((t * PLANE_K + kk * 16 * PK) * 2));
+#pragma unroll
+    for (int s = D - 1; s >= SMIN; --s) {
+      uint32_t a[4];
+      const uint32_t addr = a_addr + (uint32_t)s * a_plane + (uint32_t)kk * a_k16;
+      if (A_TRANS)
+        ldm4t(a, addr);
+      else
+        ldm4(a, addr);
+#pragma unroll
+      for (int t = SMIN; t < D; ++t) {
+        const int g = s + t - G0;
+        if (g >= 0 && g < NG) {
+          mma(acc[g < 0 ? 0 : g < NG ? g : 0][0], a, b[t - SMIN][0], b[t - SMIN][1]);
+          mma(acc[g < 0 ? 0 : g < NG ? g : 0][1], a, b[t - SMIN][2], b[t - SMIN][3]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int64_t v = 0;
+#pragma unroll
+      for (int g = NG - 1; g >= 0; --g) v = v * 128 + to_int(acc[g][h][i]);
+      sum[4 * h + i] += v;
+    }
+}
+template <bool A_TRANS>
+__device__ __forceinline__ void stage(uint32_t a_addr, uint32_t a_plane, uint32_t a_k16,
+                                      uint32_t b_addr, int64_t (&hi)[8], int64_t (&lo)[8]) {
+  stage_mma<12, 5, A_TRANS>(a_addr, a_plane, a_k16, b_addr, hi);
+  stage_mma<8, 4, A_TRANS>(a_addr, a_plane, a_k16, b_addr, lo);
+}
+// (hi 128^12 + lo 128^8) 2^e, one rounding of the sum
+__device__ __forceinline__ double value(int64_t hi, int64_t lo, int e) {
+  return ldexp(fma((double)hi, 268435456.0, (double)lo), e + 56);
+}
+
+// exponent of each column's largest finite element (0: a zero column), and
+// nf[j] = 1 where an element is not finite.  HBM-bound.
+template <typename T>
+__global__ void __launch_bounds__(256) colexp_kernel(const T* __restrict__ A, int64_t lda, int64_t m,
+                                                     int N, int64_t rows, int* __restrict__ ce,
+                                                     int* __restrict__ nf) {
+  __shared__ int mx[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  const int64_t r0 = (int64_t)blockIdx.y * rows, r1 = min(m, r0 + rows);
+  int e = 0, bad = 0;
+  if (j < N)
+#pragma unroll 4
+    for (int64_t r = r0 + warp; r < r1; r += 8) {
+      const Dec d = decode(A[r * lda + j]);
+      if (d.e == 2047)
+        bad = 1;
+      else
+        e = max(e, scale_exp(d));
+    }
+  if (bad) nf[j] = 1;
+  mx[warp][lane] = e;
+  __syncthreads();
+  if (warp == 0 && j < N) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) e = max(e, mx[w][lane]);
+    atomicMax(ce + j, e);
+  }
+}
+
+// partial[chunk] = A_c^T A_c on the upper tiles.  16 warps of 16 x 16 outputs; two
+// stage buffers, so that the digits of the next stage are cut by warps that are
+// ahead of the others' products; one CTA an SM (166 KB).
+template <typename T>
+__global__ void __launch_bounds__(THREADS, 1)
+    gram_kernel(const T* __restrict__ A, int64_t lda, int64_t m, int N, int tn, int64_t rows,
+                const int* __restrict__ ce, const int* __restrict__ nf, double* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char oz_sm[];
+  int ti = 0, tj = blockIdx.x;
+  while (tj >= tn - ti) {
+    tj -= tn - ti;
+    ++ti;
+  }
+  tj += ti;
+  const bool diag = ti == tj;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r0 = (int64_t)blockIdx.y * rows, r1 = min(m, r0 + rows);
+  const int i0 = ti * TS, j0 = tj * TS;
+  // this thread's column pairs of the two operands
+  const int ca = i0 + 2 * lane, cb = j0 + 2 * lane;
+  const int ea0 = ca < N ? ce[ca] : 0, ea1 = ca + 1 < N ? ce[ca + 1] : 0;
+  const int eb0 = cb < N ? ce[cb] : 0, eb1 = cb + 1 < N ? ce[cb + 1] : 0;
+  auto cut = [&](int64_t k0, int buf) {
+    __half* base = reinterpret_cast<__half*>(oz_sm + (size_t)buf * BUF_G);
+    T xa[KS / 16][2], xb[KS / 16][2];
+#pragma unroll
+    for (int q = 0; q < KS / 16; ++q) {
+      const int64_t r = k0 + warp + 16 * q;
+      const T* src = A + r * lda;
+      xa[q][0] = r < r1 && ca < N ? src[ca] : T(0);
+      xa[q][1] = r < r1 && ca + 1 < N ? src[ca + 1] : T(0);
+      if (!diag) {
+        xb[q][0] = r < r1 && cb < N ? src[cb] : T(0);
+        xb[q][1] = r < r1 && cb + 1 < N ? src[cb + 1] : T(0);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < KS / 16; ++q) {
+      __half* p = base + (warp + 16 * q) * PK + 2 * lane;
+      const Dec d0 = decode(xa[q][0]), d1 = decode(xa[q][1]);
+      put2(p, PLANE_K, fix(d0, d0.e + 8 - ea0), fix(d1, d1.e + 8 - ea1));
+      if (!diag) {
+        const Dec f0 = decode(xb[q][0]), f1 = decode(xb[q][1]);
+        put2(p + D * PLANE_K, PLANE_K, fix(f0, f0.e + 8 - eb0), fix(f1, f1.e + 8 - eb1));
+      }
+    }
+  };
+  const int wi = (warp >> 2) * 16, wj = (warp & 3) * 16;
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(oz_sm);
+  // A fragments (transposed [k][i] blocks): (i0, k0), (i8, k0), (i0, k8), (i8, k8);
+  // B fragments: (k0, j0), (k8, j0), (k0, j8), (k8, j8)
+  const uint32_t a_off =
+      (uint32_t)((((lane & 7) + (lane >> 4) * 8) * PK + wi + ((lane >> 3) & 1) * 8) * 2);
+  const uint32_t b_off =
+      (uint32_t)((((lane & 7) + ((lane >> 3) & 1) * 8) * PK + wj + (lane >> 4) * 8) * 2) +
+      (diag ? 0u : (uint32_t)(D * PLANE_K * 2));
+  int64_t hi[8], lo[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) hi[i] = lo[i] = 0;
+  int buf = 0;
+  cut(r0, 0);
+  __syncthreads();
+  for (int64_t k0 = r0; k0 < r1; k0 += KS) {
+    if (k0 + KS < r1) cut(k0 + KS, buf ^ 1);
+    const uint32_t base = sm0 + (uint32_t)(buf * BUF_G);
+    stage<true>(base + a_off, PLANE_K * 2, 16 * PK * 2, base + b_off, hi, lo);
+    __syncthreads();
+    buf ^= 1;
+  }
+  double* P = part + (int64_t)blockIdx.y * N * N;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + wi + (lane >> 2) + (q >> 1) * 8;
+      const int j = j0 + wj + 8 * h + 2 * (lane & 3) + (q & 1);
+      if (i < N && j < N) {
+        // A = X 2^(ce - 1,022 - 61)
+        double v = value(hi[4 * h + q], lo[4 * h + q], ce[i] + ce[j] - 2 * 1083);
+        if (nf[i] | nf[j]) v = __longlong_as_double(0x7ff8000000000000ll);
+        P[(int64_t)i * N + j] = v;
+      }
+    }
+}
+
+// G = sum over the chunks (in order), mirrored
+__global__ void __launch_bounds__(256) reduce_kernel(const double* __restrict__ part, int N,
+                                                     int chunks, double* __restrict__ G) {
+  const int64_t total = (int64_t)N * N;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+    const int i = (int)(e / N), j = (int)(e % N);
+    const int64_t src = i / TS > j / TS ? (int64_t)j * N + i : e;
+    double s = 0.0;
+    for (int c = 0; c < chunks; ++c) s += part[c * total + src];
+    G[e] = s;
+  }
+}
+
+// digits of W' = diag(2^ce) W, column scales: planes [column tile][k][digit][64],
+// fw[j] = exponent of column j's largest element (4,095: not finite)
+__global__ void __launch_bounds__(256) wsplit_kernel(const double* __restrict__ W, int64_t ldw, int N,
+                                                     int Kp, int k, const int* __restrict__ ce,
+                                                     __half* __restrict__ planes,
+                                                     int* __restrict__ fw) {
+  __shared__ int mx[8][TS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * TS + 2 * lane;
+  int f[2] = {0, 0};
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (c + u < k) {
+      for (int r = warp; r < N; r += 8) {
+        const Dec d = decode(W[(int64_t)r * ldw + c + u]);
+        if (d.e == 2047)
+          f[u] = 1 << 16;
+        else if (d.mant)
+          f[u] = max(f[u], d.e + ce[r]);
+      }
+    }
+  mx[warp][2 * lane] = f[0];
+  mx[warp][2 * lane + 1] = f[1];
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int w = 0; w < 8; ++w) f[u] = max(f[u], mx[w][2 * lane + u]);
+  if (blockIdx.y == 0 && warp == 0) {
+    if (c < k) fw[c] = f[0];
+    if (c + 1 < k) fw[c + 1] = f[1];
+  }
+  for (int r = blockIdx.y * KS + warp; r < min(Kp, (int)(blockIdx.y + 1) * KS); r += 8) {
+    const bool in = r < N;
+    const Dec d0 = decode(in && c < k ? W[(int64_t)r * ldw + c] : 0.0);
+    const Dec d1 = decode(in && c + 1 < k ? W[(int64_t)r * ldw + c + 1] : 0.0);
+    const int e = in ? ce[r] : 0;
+    put2(planes + (((int64_t)blockIdx.x * Kp + r) * D) * TS + 2 * lane, TS,
+         fix(d0, d0.e + e + 8 - f[0]), fix(d1, d1.e + e + 8 - f[1]));
+  }
+}
+
+// C = A W.  Column scales of A are folded into W', the rows have their own besides.
+// upper: W[r][j] = 0 for r > j.
+template <typename T, typename TO>
+__global__ void __launch_bounds__(THREADS, 1)
+    nn_kernel(const T* __restrict__ A, int64_t lda, int64_t m, int N, int Kp, int k,
+              const int* __restrict__ ce, const __half* __restrict__ planes,
+              const int* __restrict__ fw, int upper, TO* __restrict__ C, int64_t ldc) {
+  extern __shared__ __align__(16) unsigned char oz_sm[];
+  __shared__ int rexp[TS], rbad[TS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t i0 = (int64_t)blockIdx.y * TS;
+  const int j0 = blockIdx.x * TS;
+  const int kend = upper ? min(N, j0 + TS) : N;
+  for (int r = warp; r < TS; r += THREADS / 32) {
+    int e = -(1 << 16), bad = 0;
+    if (i0 + r < m)
+#pragma unroll 4
+      for (int c = lane; c < kend; c += 32) {
+        const Dec d = decode(A[(i0 + r) * lda + c]);
+        if (d.e == 2047)
+          bad = 1;
+        else if (d.mant)
+          e = max(e, d.e - ce[c]);
+      }
+    e = warp_max(e);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+      rexp[r] = e == -(1 << 16) ? 0 : e;
+      rbad[r] = bad;
+    }
+  }
+  __syncthreads();
+  const int pr = tid >> 4, pc = 2 * (tid & 15);  // rows pr, pr + 32, columns pc, pc + 1 of a stage
+  const int re0 = rexp[pr], re1 = rexp[pr + 32];
+  const __half* wp = planes + (int64_t)blockIdx.x * Kp * D * TS;
+  auto cut = [&](int k0, int buf) {
+    __half* base = reinterpret_cast<__half*>(oz_sm + (size_t)buf * BUF_N);
+    const uint32_t bw = (uint32_t)__cvta_generic_to_shared(base + D * PLANE_M);
+    for (int e = tid; e < KS * D * (TS / 8); e += THREADS) {  // 16-byte pieces
+      const int kr = e / (D * 8), s = e / 8 % D, q = e % 8;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       bw + (uint32_t)((s * PLANE_K + kr * PK + q * 8) * 2)),
+                   "l"(wp + ((int64_t)(k0 + kr) * D + s) * TS + q * 8));
+    }
+    const int c0 = k0 + pc;
+    const int e0 = c0 < kend ? ce[c0] : 0, e1 = c0 + 1 < kend ? ce[c0 + 1] : 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int64_t r = i0 + pr + 32 * q;
+      const Dec d0 = decode(r < m && c0 < kend ? A[r * lda + c0] : T(0));
+      const Dec d1 = decode(r < m && c0 + 1 < kend ? A[r * lda + c0 + 1] : T(0));
+      const int re = q ? re1 : re0;
+      put2(base + (pr + 32 * q) * PM + pc, PLANE_M, fix(d0, d0.e + 8 - e0 - re),
+           fix(d1, d1.e + 8 - e1 - re));
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  };
+  const int wi = (warp >> 2) * 16, wj = (warp & 3) * 16;
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(oz_sm);
+  // A fragments ([i][k]): (i0, k0), (i8, k0), (i0, k8), (i8, k8)
+  const uint32_t a_off =
+      (uint32_t)(((wi + (lane & 7) + ((lane >> 3) & 1) * 8) * PM + (lane >> 4) * 8) * 2);
+  const uint32_t b_off =
+      (uint32_t)((D * PLANE_M + ((lane & 7) + ((lane >> 3) & 1) * 8) * PK + wj + (lane >> 4) * 8) * 2);
+  int64_t hi[8], lo[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) hi[i] = lo[i] = 0;
+  int buf = 0;
+  cut(0, 0);
+  __syncthreads();
+  for (int k0 = 0; k0 < kend; k0 += KS) {
+    if (k0 + KS < kend) cut(k0 + KS, buf ^ 1);
+    const uint32_t base = sm0 + (uint32_t)(buf * BUF_N);
+    stage<false>(base + a_off, PLANE_M * 2, 16 * 2, base + b_off, hi, lo);
+    __syncthreads();
+    buf ^= 1;
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int il = wi + (lane >> 2) + (q >> 1) * 8;
+      const int j = j0 + wj + 8 * h + 2 * (lane & 3) + (q & 1);
+      if (i0 + il < m && j < k) {
+        // A = X 2^(ce + rexp - 1,022 - 61), W' = Y 2^(fw - 2,044 - 61)
+        double v = value(hi[4 * h + q], lo[4 * h + q], rexp[il] + fw[j] - 2044 - 122);
+        if (rbad[il] || fw[j] >= (1 << 16)) v = __longlong_as_double(0x7ff8000000000000ll);
+        C[(i0 + il) * ldc + j] = (TO)v;
+      }
+    }
+}
+
+}  // namespace oz
+
+template <typename T>
+static int oz_colexp(const T* A, int64_t lda, int64_t m, int N, int* ce, int* nf, cudaStream_t st) {
+  PLOM_CHECK_CUDA(cudaMemsetAsync(ce, 0, (size_t)2 * N * sizeof(int), st));
+  const int64_t cols = cdiv(N, 32);
+  const int64_t rows = std::max<int64_t>(64, cdiv(m, std::max<int64_t>(1, 8 * num_sms() / cols)));
+  const dim3 grid((unsigned)cols, (unsigned)cdiv(m, rows));
+  oz::colexp_kernel<T><<<grid, 256, 0, st>>>(A, lda, m, N, rows, ce, nf);
+  PLOM_CHECK_LAUNCH();
+  return PLOM_OK;
+}
+
+// row chunks of a Gram: the count with the shortest longest CTA (waves of CTAs times
+// stages of a chunk, two for a CTA's start and end), 256 rows at least
+static int64_t oz_chunk_rows(int64_t m, int64_t tiles) {
+  int64_t best = 0, rows = m;
+  for (int64_t c = 1; c <= 64; ++c) {
+    const int64_t r = cdiv(cdiv(m, c), oz::KS) * oz::KS;
+    if (c > 1 && r < 256) break;
+    if (r > oz::MAX_ROWS && c < 64) continue;
+    const int64_t cost = cdiv(tiles * cdiv(m, r), num_sms()) * (r / oz::KS + 2);
+    if (best == 0 || cost < best) {
+      best = cost;
+      rows = r;
+    }
+  }
+  return std::min<int64_t>(rows, oz::MAX_ROWS);
+}
+
+template <typename T>
+int oz_gram(const T* A, int64_t lda, int64_t m, int64_t N, double* G, Arena& ws, cudaStream_t st) {
+  const int64_t tn = cdiv(N, oz::TS), tiles = tn * (tn + 1) / 2;
+  const int64_t rows = oz_chunk_rows(m, tiles), chunks = cdiv(m, rows);
+  int* ce = ws.take<int>((size_t)2 * N);
+  double* part = ws.take<double>((size_t)chunks * N * N);
+  if (ws.measuring()) return PLOM_OK;
+  PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "oz_gram: workspace too small");
+  PLOM_REQUIRE(A && G && m >= 1 && N >= 1 && tiles < (1ll << 31) && chunks <= 65535, PLOM_ERR_ARG,
+               "oz_gram: bad arguments");
+  static bool attr[2] = {false, false};
+  if (!attr[sizeof(T) == 8]) {
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(oz::gram_kernel<T>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * oz::BUF_G));
+    attr[sizeof(T) == 8] = true;
+  }
+  ProfScope prof("gram_oz", st, (double)m * N * N, (double)m * N * sizeof(T) * 2, 4);
+  PLOM_TRY(oz_colexp(A, lda, m, (int)N, ce, ce + N, st));
+  oz::gram_kernel<T><<<dim3((unsigned)tiles, (unsigned)chunks), oz::THREADS, 2 * oz::BUF_G, st>>>(
+      A, lda, m, (int)N, (int)tn, rows, ce, ce + N, part);
+  PLOM_CHECK_LAUNCH();
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(N * N, 256), (int64_t)num_sms() * 8));
+  oz::reduce_kernel<<<blocks, 256, 0, st>>>(part, (int)N, (int)chunks, G);
+  PLOM_CHECK_LAUNCH();
+  return PLOM_OK;
+}
+
+template <typename T, typename TO>
+int oz_nn(const T* A, int64_t lda, int64_t m, int64_t N, const double* W, int64_t ldw, int64_t k,
+          TO* C, int64_t ldc, bool upper, Arena& ws, cudaStream_t st) {
+  const int64_t Kp = cdiv(N, oz::KS) * oz::KS, ct = cdiv(k, oz::TS);
+  int* ce = ws.take<int>((size_t)2 * N);
+  int* fw = ws.take<int>((size_t)k);
+  __half* planes = ws.take<__half>((size_t)ct * Kp * oz::D * oz::TS);
+  if (ws.measuring()) return PLOM_OK;
+  PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "oz_nn: workspace too small");
+  PLOM_REQUIRE(A && W && C && m >= 1 && N >= 1 && k >= 1 && N < (1 << 22) && ct < (1ll << 31),
+               PLOM_ERR_ARG, "oz_nn: bad arguments");
+  constexpr int which = (sizeof(T) == 8 ? 2 : 0) + (sizeof(TO) == 8 ? 1 : 0);
+  static bool attr[4] = {false, false, false, false};
+  if (!attr[which]) {
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(oz::nn_kernel<T, TO>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * oz::BUF_N));
+    attr[which] = true;
+  }
+  const double fl = upper && N == k ? (double)m * N * (N + 1) : 2.0 * m * N * k;
+  ProfScope prof("apply_oz", st, fl, (double)m * N * sizeof(T) * 2 + (double)m * k * sizeof(TO), 4);
+  PLOM_TRY(oz_colexp(A, lda, m, (int)N, ce, ce + N, st));
+  oz::wsplit_kernel<<<dim3((unsigned)ct, (unsigned)(Kp / oz::KS)), 256, 0, st>>>(
+      W, ldw, (int)N, (int)Kp, (int)k, ce, planes, fw);
+  PLOM_CHECK_LAUNCH();
+  for (int64_t i0 = 0; i0 < m; i0 += 65535ll * oz::TS) {  // grid.y
+    const int64_t mi = std::min<int64_t>(m - i0, 65535ll * oz::TS);
+    oz::nn_kernel<T, TO><<<dim3((unsigned)ct, (unsigned)cdiv(mi, oz::TS)), oz::THREADS, 2 * oz::BUF_N,
+                           st>>>(A + i0 * lda, lda, mi, (int)N, (int)Kp, (int)k, ce, planes, fw,
+                                 upper ? 1 : 0, C + i0 * ldc, ldc);
+    PLOM_CHECK_LAUNCH();
+  }
+  return PLOM_OK;
+}
+
+template int oz_gram<double>(const double*, int64_t, int64_t, int64_t, double*, Arena&, cudaStream_t);
+template int oz_gram<float>(const float*, int64_t, int64_t, int64_t, double*, Arena&, cudaStream_t);
+#define OZ_NN(T, TO)                                                                             \
+  template int oz_nn<T, TO>(const T*, int64_t, int64_t, int64_t, const double*, int64_t, int64_t, \
+                            TO*, int64_t, bool, Arena&, cudaStream_t);
+OZ_NN(double, double)
+OZ_NN(double, float)
+OZ_NN(float, double)
+OZ_NN(float, float)
+#undef OZ_NN
+
+}  // namespace plom

@@ -45,9 +45,16 @@ int gemm_tn_in_scratch(const TA* A, int64_t lda, const TB* B, int64_t ldb, TC* C
                        cudaStream_t st);
 size_t gemm_tn_workspace_batched(int64_t M, int64_t N, int64_t K, bool sym, size_t acc_bytes,
                                  int batch);
+// FP64 products on the tensor cores, operands cut into digits (gemm_oz.cu):
+// G (N x N) = A^T A and C (m x k) = A W for a tall A (m x N), W FP64; upper: W is upper
+// triangular.  A row or column with an element that is not finite gives NaN.
+template <typename T>
+int oz_gram(const T* A, int64_t lda, int64_t m, int64_t N, double* G, Arena& ws, cudaStream_t st);
+template <typename T, typename TO>
+int oz_nn(const T* A, int64_t lda, int64_t m, int64_t N, const double* W, int64_t ldw, int64_t k,
+          TO* C, int64_t ldc, bool upper, Arena& ws, cudaStream_t st);
 // C (M x N, FP64, ld ldc) = A^T B for FP32 A (K x M), B (K x N): exact products,
 // compensated double-float sums over row chunks, FP64 chunk reduction.
-// ---- dense.cu ----
 int gemm_tn_df(const float* A, int64_t lda, const float* B, int64_t ldb, double* C, int64_t ldc,
                int64_t M, int64_t N, int64_t K, Arena& ws, cudaStream_t st);
 

@@ -45,8 +45,7 @@ static bool packed_ok(int64_t m) { return m >= 1 && m < (1ll << 31); }
 template <typename TA>
 static int tall_gram(int prec, const TA* A, int64_t lda, int64_t m, int64_t N, double* G,
                      int* err, Arena& ws, cudaStream_t st) {
-  if (prec == PLOM_PREC_FP64)
-    return gemm_tn<TA, TA, double, double>(A, lda, A, lda, G, N, N, N, m, true, ws, st);
+  if (prec == PLOM_PREC_FP64 || sizeof(TA) == 8) return oz_gram<TA>(A, lda, m, N, G, ws, st);
   if constexpr (sizeof(TA) == 4) {
     if (packed_ok(m)) {
       Packed p;
@@ -55,8 +54,6 @@ static int tall_gram(int prec, const TA* A, int64_t lda, int64_t m, int64_t N, d
       return gram_packed(p, G, err, ws, st);
     }
     return gemm_tn<TA, TA, float, double>(A, lda, A, lda, G, N, N, N, m, true, ws, st);
-  } else {
-    return gemm_tn<TA, TA, double, double>(A, lda, A, lda, G, N, N, N, m, true, ws, st);
   }
 }
 
@@ -65,10 +62,8 @@ template <typename TA, typename TO>
 static int tall_apply(int prec, const TA* A, int64_t lda, int64_t m, int64_t N, const double* W,
                       int64_t k, TO* C, int64_t ldc, int* err, Arena& ws, cudaStream_t st,
                       bool upper = false) {
-  if (prec == PLOM_PREC_FP64 || sizeof(TA) == 8) {
-    if (ws.measuring()) return PLOM_OK;  // workspace query: launch nothing
-    return gemm_nn<TA, double, TO, double>(A, lda, W, k, C, ldc, m, k, N, st, upper);
-  }
+  if (prec == PLOM_PREC_FP64 || sizeof(TA) == 8)
+    return oz_nn<TA, TO>(A, lda, m, N, W, k, k, C, ldc, upper, ws, st);
   if constexpr (sizeof(TA) == 4 && sizeof(TO) == 4) {
     if (packed_ok(m)) {
       Packed p;
