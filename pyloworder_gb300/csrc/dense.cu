@@ -2633,6 +2633,63 @@ size_t dense_workspace(int n, int batch, int cplx) {
   return std::max(a.off, b.off) + 256;
 }
 
+// ---- FP32 start of the FP64 sweeps ----------------------------------------
+// A sweep of the FP64 kernel is bound by the FP64 rate and by the latency of its
+// rounds (1.13 ms at n = 200, 15 sweeps); an FP32 sweep takes a tenth of that.  So
+// the FP32 sweeps run first, to their own resolution, and their rotation product is
+// made orthogonal in FP64: two Newton-Schulz steps V <- V (3 I - V^T V) / 2 (the
+// departure squares: 1e-5, 1e-10, below FP64).  The FP64 kernel starts from B = A^T V
+// with V as its rotation product and iterates to its own tolerance as before: a poor
+// start would cost it sweeps, not accuracy (and ten sweeps fewer round fewer times:
+// ||A - U S V|| 5.6e-14 -> 0.9e-14 of ||A|| on modes over a noise floor).  Products by
+// gemm_oz.cu, exact to 2^-58 of their scales.  200 columns of a 16,384-point POD:
+// 15 sweeps, 16.9 ms, before; 13 FP32 and 4 FP64 sweeps, 7.2 ms with the products.
+__global__ void ns_factor_kernel(double* __restrict__ G, int n) {
+  const int64_t nn = (int64_t)n * n;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nn;
+       e += (int64_t)gridDim.x * blockDim.x)
+    G[e] = 0.5 * ((e / n == e % n ? 3.0 : 0.0) - G[e]);
+}
+
+// No floor (every pair is turned): columns left to the FP64 sweeps cost them three
+// more at n = 200 (7.4 ms instead of 4.2).
+constexpr float JAC_START32_TOL = 2e-6f;    // as JAC_PRE32_TOL
+constexpr float JAC_START32_TSTOP = 3e-3f;  // as JAC_PRE32_TSTOP
+
+// V (orthogonal, FP64) and B = At V; J32: n x n FP32 scratch (may be B)
+static int jacobi_start32(const double* A, const double* At, int n, unsigned long long* amax,
+                          float* J32, double* V, double* B, int* info, Arena& ws,
+                          cudaStream_t st) {
+  const size_t nn = (size_t)n * n;
+  const size_t mark = ws.off;
+  PLOM_TRY(jacobi_gram_f32(A, n, JAC_START32_TOL, 0.f, JAC_START32_TSTOP, J32, amax, info, ws, st));
+  size_t need = ws.off;
+  ws.off = mark;
+  double* G = ws.take<double>(nn);
+  double* T = ws.take<double>(nn);
+  const size_t mark2 = ws.off;
+  if (!ws.measuring()) PLOM_TRY((convert<float, double>(J32, V, (int64_t)nn, st)));
+  const int eg = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv((int64_t)nn, 256),
+                                                             (int64_t)num_sms() * 16));
+  double *x = V, *y = T;
+  for (int k = 0; k < 2; ++k) {
+    PLOM_TRY(oz_gram<double>(x, n, n, n, G, ws, st));
+    need = std::max(need, ws.off);
+    ws.off = mark2;
+    if (!ws.measuring()) {
+      ns_factor_kernel<<<eg, 256, 0, st>>>(G, n);
+      PLOM_CHECK_LAUNCH();
+    }
+    PLOM_TRY((oz_nn<double, double>(x, n, n, n, G, n, n, y, n, false, ws, st)));
+    need = std::max(need, ws.off);
+    ws.off = mark2;
+    std::swap(x, y);
+  }
+  PLOM_TRY((oz_nn<double, double>(At, n, n, n, V, n, n, B, n, false, ws, st)));
+  ws.off = std::max(need, ws.off);
+  return PLOM_OK;
+}
+
 // Real n x n SVD through the transpose: one-sided Jacobi on A^T (whose
 // columns are the rows of A) needs fewer sweeps than on A for the
 // triangular factors of the TSQR.  A^T = Ut S Vt^T  ->  A = Vt S Ut^T.
@@ -2643,19 +2700,29 @@ static int jacobi_svd_transposed(const double* A, int n, double tol, double* S, 
   double* Ut = ws.take<double>(nn);
   double* VHt = ws.take<double>(nn);
   const bool pre32 = use_pre32(n, tol);
+  const bool start32 = !pre32 && tol < JAC_DF_TOL && jacobi_gram_plan_ok(n);
   JacState js;
   if (!pre32) carve_jac(ws, js, n, 1, 0);
-  if (ws.measuring())
+  double* V0 = start32 ? ws.take<double>(nn) : nullptr;
+  double* B = start32 ? ws.take<double>(nn) : nullptr;
+  if (ws.measuring()) {
+    if (start32) PLOM_TRY(jacobi_start32(A, At, n, nullptr, nullptr, V0, B, info, ws, st));
     return pre32 ? jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st) : PLOM_OK;
+  }
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
   PLOM_REQUIRE(A && S && U && VH && info, PLOM_ERR_ARG, "jacobi: null pointer");
   if (!pre32 && tol >= JAC_DF_TOL && jacobi_cta_usable(n, 0))
     return jacobi_cta(A, n, 1, 0, 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U, VH, info, st);
   if (!pre32 || !jacobi_gram_usable(n)) PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
-  if (pre32)
+  if (pre32) {
     PLOM_TRY(jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st));
-  else
+  } else if (start32 && jacobi_gram_usable(n)) {
+    PLOM_TRY(jacobi_start32(A, At, n, js.amax, reinterpret_cast<float*>(B), V0, B, info, ws, st));
+    js.V0 = V0;
+    PLOM_TRY(jacobi_launch(B, n, 1, 0, js, tol, S, Ut, VHt, info, st));
+  } else {
     PLOM_TRY(jacobi_launch(At, n, 1, 0, js, tol, S, Ut, VHt, info, st));
+  }
   PLOM_TRY(transpose_f64(VHt, U, n, n, 1, st));   // U of A = Vt (columns)
   PLOM_TRY(transpose_f64(Ut, VH, n, n, 1, st));   // rows of V^T of A = columns of Ut
   return PLOM_OK;

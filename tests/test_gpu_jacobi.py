@@ -77,3 +77,27 @@ def test_tsqr_factors(n, scale):
     assert np.max(np.abs(Q.T @ Q - np.eye(n))) < 2 * TOL
     assert np.linalg.norm(R - Rn) < TOL * s
     assert np.linalg.norm(Q @ R - A) < TOL * s
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 127, 128, 129, 193, 200, 257, 320, 321, 449, 512, 513, 600])
+@pytest.mark.parametrize("kind", ["normal", "floor", "graded", "rank"])
+def test_fp64_from_fp32_start(n, kind):
+    # FP64 sweeps that start from FP32 ones end at their own tolerance, n eps a pair:
+    # ten times that on the factors
+    import pyloworder_gb300 as P
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n + 200, n))
+    if kind == "floor":
+        k = np.arange(n)
+        A = (A[:, :5] * 3.0 ** -np.arange(5)) @ np.cos(0.3 * np.arange(5)[:, None] * k + 1) + 1e-5 * A
+    elif kind == "graded":
+        A = np.linalg.qr(A)[0] * 10.0 ** -np.linspace(0, 11, n) @ np.linalg.qr(rng.standard_normal((n, n)))[0]
+    elif kind == "rank":
+        A = A[:, : n // 2] @ rng.standard_normal((n // 2, n))
+    U, S, V = (x.cpu().numpy() for x in P.math.tsqr_svd(torch.from_numpy(A).cuda()))
+    tol = 10 * n * 2.3e-16
+    r = n // 2 if kind == "rank" else n
+    assert np.max(np.abs(U[:, :r].T @ U[:, :r] - np.eye(r))) < tol
+    assert np.max(np.abs(V @ V.T - np.eye(n))) < tol
+    assert np.linalg.norm((U * S) @ V - A) < tol * np.linalg.norm(A)
+    assert np.max(np.abs(S - np.linalg.svd(A, compute_uv=False))) < tol * S[0]
