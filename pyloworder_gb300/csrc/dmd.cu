@@ -1,5 +1,5 @@
-// DMD reduced stage on the GPU, all in FP64, one CTA (the reduced operator
-// is r x r with r up to a few hundred):
+// DMD reduced stage on the GPU, all in FP64 (the reduced operator is r x r with r
+// up to a few hundred):
 //
 //   Atilde = (U^T Y2) (S^-1 VT)^T                     pyLOM/DMD/wrapper.py:84-87
 //   eig(Atilde) -> mu, W                              wrapper.py:93 (LAPACK dgeev
@@ -52,142 +52,132 @@ struct DmdBufs {
   double* Y;    // N x N complex (eigenvectors of T), interleaved
   double* Pm;   // N x N complex (P, then its Cholesky factor)
   double* qv;   // N complex
-  double* bv;   // N complex
-  double* babs; // N
   int* order;   // N
   double* Vr;   // N x nt complex Vandermonde
   int* flip;    // N conjugate-pair fix-up flags of the ordered modes
 };
 
 // -------------------------------------------------------------------------
-// Hessenberg + Francis QR (one CTA).  A (N x N, row-major) is overwritten
-// with T, Z accumulates the orthogonal transformations.
+// Hessenberg + Francis QR (one CTA).  A (N x N, row-major, pitch ld) is
+// overwritten with T, Z accumulates the orthogonal transformations.  The chain of
+// reflectors is serial: its latency is what counts, so A and Z are in shared
+// memory (see dmd_eig_kernel), one thread forms a reflector, and three barriers
+// separate it from the row and the column updates (r = 32, 802 reflectors: 3,500
+// cycles each, half of them the reflector's own FP64 chain).
 // -------------------------------------------------------------------------
-__device__ void hessenberg(double* A, double* Z, int N, double* sh) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < N * N; e += nt) Z[e] = ((e / N) == (e % N)) ? 1.0 : 0.0;
+__device__ void hessenberg(double* A, double* Z, int N, int ld, double* sh) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
+  for (int e = tid; e < N * N; e += nt) Z[e / N * ld + e % N] = ((e / N) == (e % N)) ? 1.0 : 0.0;
   __syncthreads();
   double* v = sh;        // N
   double* w = sh + N;    // N
   for (int k = 0; k + 2 < N; ++k) {
     // reflector for x = A[k+1:N, k]
-    if (tid == 0) {
+    if (tid < 32) {
       double s = 0.0;
-      for (int i = k + 1; i < N; ++i) s += A[i * N + k] * A[i * N + k];
-      double nrm = sqrt(s);
-      double x0 = A[(k + 1) * N + k];
-      double alpha = (x0 >= 0.0) ? -nrm : nrm;
-      for (int i = 0; i < N; ++i) v[i] = 0.0;
-      double vv = 0.0;
-      if (nrm > 0.0) {
-        v[k + 1] = x0 - alpha;
-        for (int i = k + 2; i < N; ++i) v[i] = A[i * N + k];
-        for (int i = k + 1; i < N; ++i) vv += v[i] * v[i];
+      for (int i = k + 2 + lane; i < N; i += 32) s += A[i * ld + k] * A[i * ld + k];
+      s = warp_sum(s);
+      const double x0 = A[(k + 1) * ld + k];
+      const double nrm = sqrt(s + x0 * x0);
+      const double v0 = x0 - ((x0 >= 0.0) ? -nrm : nrm);
+      for (int i = lane; i < N; i += 32)
+        v[i] = (i <= k || !(nrm > 0.0)) ? 0.0 : (i == k + 1 ? v0 : A[i * ld + k]);
+      if (lane == 0) {
+        const double vv = s + v0 * v0;
+        w[0] = (nrm > 0.0 && vv > 0.0) ? 2.0 / vv : 0.0;  // tau
       }
-      w[0] = (vv > 0.0) ? 2.0 / vv : 0.0;  // tau
     }
     __syncthreads();
     const double tau = w[0];
-    __syncthreads();
     if (tau != 0.0) {
       // A = (I - tau v v^T) A : column j update
       for (int j = tid; j < N; j += nt) {
-        double s = 0.0;
-        for (int i = k + 1; i < N; ++i) s += v[i] * A[i * N + j];
-        s *= tau;
-        for (int i = k + 1; i < N; ++i) A[i * N + j] -= s * v[i];
+        double s0 = 0.0, s1 = 0.0;
+        int i = k + 1;
+        for (; i + 1 < N; i += 2) {
+          s0 += v[i] * A[i * ld + j];
+          s1 += v[i + 1] * A[(i + 1) * ld + j];
+        }
+        if (i < N) s0 += v[i] * A[i * ld + j];
+        const double s = (s0 + s1) * tau;
+        for (i = k + 1; i < N; ++i) A[i * ld + j] -= s * v[i];
       }
       __syncthreads();
       // A = A (I - tau v v^T), Z = Z (I - tau v v^T): row updates
       for (int i = tid; i < 2 * N; i += nt) {
-        double* M = (i < N) ? A : Z;
-        const int r = (i < N) ? i : i - N;
-        double s = 0.0;
-        for (int j = k + 1; j < N; ++j) s += M[r * N + j] * v[j];
-        s *= tau;
-        for (int j = k + 1; j < N; ++j) M[r * N + j] -= s * v[j];
+        double* M = (i < N) ? A + i * ld : Z + (i - N) * ld;
+        double s0 = 0.0, s1 = 0.0;
+        int j = k + 1;
+        for (; j + 1 < N; j += 2) {
+          s0 += M[j] * v[j];
+          s1 += M[j + 1] * v[j + 1];
+        }
+        if (j < N) s0 += M[j] * v[j];
+        const double s = (s0 + s1) * tau;
+        for (j = k + 1; j < N; ++j) M[j] -= s * v[j];
+        if (i >= k + 2 && i < N) M[k] = 0.0;
       }
-      __syncthreads();
-      if (tid == 0)
-        for (int i = k + 2; i < N; ++i) A[i * N + k] = 0.0;
     }
     __syncthreads();
   }
 }
 
-// apply the reflector I - tau v v^T (v of length len at rows/cols k..k+len-1)
-// to rows k.. of A over columns [c0, N), to columns k.. of A over rows
-// [0, r1], and to columns k.. of Z (all rows)
-__device__ void apply_reflector(double* A, double* Z, int N, int k, int len, const double* v,
-                                double tau, int c0, int r1) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int j = c0 + tid; j < N; j += nt) {
-    double s = 0.0;
-    for (int q = 0; q < len; ++q) s += v[q] * A[(k + q) * N + j];
-    s *= tau;
-    for (int q = 0; q < len; ++q) A[(k + q) * N + j] -= s * v[q];
-  }
-  __syncthreads();
-  for (int i = tid; i < (r1 + 1) + N; i += nt) {
-    double* M = (i <= r1) ? A : Z;
-    const int r = (i <= r1) ? i : i - (r1 + 1);
-    double s = 0.0;
-    for (int q = 0; q < len; ++q) s += M[r * N + k + q] * v[q];
-    s *= tau;
-    for (int q = 0; q < len; ++q) M[r * N + k + q] -= s * v[q];
-  }
-  __syncthreads();
-}
-
 // plane rotation [c s; -s c] applied on rows/cols p, p+1
-__device__ void apply_rotation(double* A, double* Z, int N, int p, double c, double s) {
+__device__ void apply_rotation(double* A, double* Z, int N, int ld, int p, double c, double s) {
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int j = p + tid; j < N; j += nt) {  // rows p, p+1 : G^T A
-    double x = A[p * N + j], y = A[(p + 1) * N + j];
-    A[p * N + j] = c * x + s * y;
-    A[(p + 1) * N + j] = -s * x + c * y;
+    double x = A[p * ld + j], y = A[(p + 1) * ld + j];
+    A[p * ld + j] = c * x + s * y;
+    A[(p + 1) * ld + j] = -s * x + c * y;
   }
   __syncthreads();
   for (int i = tid; i < 2 * N; i += nt) {  // cols p, p+1 : A G and Z G
     if (i < N && i > p + 1) continue;
-    double* M = (i < N) ? A : Z;
-    const int r = (i < N) ? i : i - N;
-    double x = M[r * N + p], y = M[r * N + p + 1];
-    M[r * N + p] = c * x + s * y;
-    M[r * N + p + 1] = -s * x + c * y;
+    double* M = (i < N) ? A + i * ld : Z + (i - N) * ld;
+    double x = M[p], y = M[p + 1];
+    M[p] = c * x + s * y;
+    M[p + 1] = -s * x + c * y;
   }
   __syncthreads();
 }
 
 // Francis double-shift QR on the Hessenberg A; returns false on non-convergence
-__device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, double* sh) {
-  const int tid = threadIdx.x;
-  volatile int* ctl = reinterpret_cast<volatile int*>(sh + 8);  // [0]=l, [1]=action
-  double* v = sh;                                                 // 3 + tau at v[3]
+__device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, int ld, double* sh) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
+  volatile int* ctl = reinterpret_cast<volatile int*>(sh + 8);  // [0]=l
+  volatile double* v = sh;                                        // 3, tau at v[3], alpha at v[4]
   const double eps = 2.220446049250313e-16;
   int nn = N - 1;
   int its = 0, total = 0;
   const int max_total = 60 * N + 60;
   while (nn >= 0) {
     if (total > max_total) return false;
-    if (tid == 0) {
-      int l = nn;
-      for (; l > 0; --l) {
-        double s = fabs(A[(l - 1) * N + l - 1]) + fabs(A[l * N + l]);
-        if (s == 0.0) s = 1.0;
-        if (fabs(A[l * N + l - 1]) <= eps * s) {
-          A[l * N + l - 1] = 0.0;
+    if (tid < 32) {  // the last negligible subdiagonal entry: 32 at a time
+      int l = 0;
+      for (int top = nn; top > 0; top -= 32) {
+        const int q = top - lane;
+        bool hit = false;
+        if (q > 0) {
+          double s = fabs(A[(q - 1) * ld + q - 1]) + fabs(A[q * ld + q]);
+          if (s == 0.0) s = 1.0;
+          hit = fabs(A[q * ld + q - 1]) <= eps * s;
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, hit);
+        if (mask) {
+          l = top - (__ffs(mask) - 1);
           break;
         }
       }
-      ctl[0] = l;
+      if (lane == 0) {
+        if (l > 0) A[l * ld + l - 1] = 0.0;
+        ctl[0] = l;
+      }
     }
     __syncthreads();
     const int l = ctl[0];
-    __syncthreads();
     if (l == nn) {  // one real root
       if (tid == 0) {
-        wr[nn] = A[nn * N + nn];
+        wr[nn] = A[nn * ld + nn];
         wi[nn] = 0.0;
       }
       --nn;
@@ -196,8 +186,8 @@ __device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, dou
       continue;
     }
     if (l == nn - 1) {  // 2 x 2 block
-      const double a = A[(nn - 1) * N + nn - 1], b = A[(nn - 1) * N + nn];
-      const double c = A[nn * N + nn - 1], d = A[nn * N + nn];
+      const double a = A[(nn - 1) * ld + nn - 1], b = A[(nn - 1) * ld + nn];
+      const double c = A[nn * ld + nn - 1], d = A[nn * ld + nn];
       const double p = 0.5 * (a - d), q = p * p + b * c;
       __syncthreads();  // every thread has read the block before it is rotated
       if (q >= 0.0) {
@@ -212,11 +202,11 @@ __device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, dou
         }
         const double r = hypot(x0, x1);
         const double cs = (r > 0.0) ? x0 / r : 1.0, sn = (r > 0.0) ? x1 / r : 0.0;
-        apply_rotation(A, Z, N, nn - 1, cs, sn);
+        apply_rotation(A, Z, N, ld, nn - 1, cs, sn);
         if (tid == 0) {
-          A[nn * N + nn - 1] = 0.0;
-          wr[nn - 1] = A[(nn - 1) * N + nn - 1];
-          wr[nn] = A[nn * N + nn];
+          A[nn * ld + nn - 1] = 0.0;
+          wr[nn - 1] = A[(nn - 1) * ld + nn - 1];
+          wr[nn] = A[nn * ld + nn];
           wi[nn - 1] = wi[nn] = 0.0;
         }
       } else if (tid == 0) {
@@ -233,48 +223,70 @@ __device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, dou
     // double-shift QR sweep on the window l..nn
     ++its;
     ++total;
-    double s, t;
-    if (its % 11 == 10) {  // exceptional shift
-      const double e = fabs(A[nn * N + nn - 1]) + fabs(A[(nn - 1) * N + nn - 2]);
-      s = 1.5 * e;
-      t = e * e;
-    } else {
-      s = A[(nn - 1) * N + nn - 1] + A[nn * N + nn];
-      t = A[(nn - 1) * N + nn - 1] * A[nn * N + nn] - A[(nn - 1) * N + nn] * A[nn * N + nn - 1];
-    }
-    double x = A[l * N + l] * A[l * N + l] + A[l * N + l + 1] * A[(l + 1) * N + l] -
-               s * A[l * N + l] + t;
-    double y = A[(l + 1) * N + l] * (A[l * N + l] + A[(l + 1) * N + l + 1] - s);
-    double z = A[(l + 1) * N + l] * A[(l + 2) * N + l + 1];
     for (int k = l; k <= nn - 1; ++k) {
       const int len = (k < nn - 1) ? 3 : 2;
       if (tid == 0) {
-        const double nrm = (len == 3) ? sqrt(x * x + y * y + z * z) : hypot(x, y);
+        double x, y, z;
+        if (k == l) {
+          double s, t;
+          if (its % 11 == 10) {  // exceptional shift
+            const double e = fabs(A[nn * ld + nn - 1]) + fabs(A[(nn - 1) * ld + nn - 2]);
+            s = 1.5 * e;
+            t = e * e;
+          } else {
+            s = A[(nn - 1) * ld + nn - 1] + A[nn * ld + nn];
+            t = A[(nn - 1) * ld + nn - 1] * A[nn * ld + nn] - A[(nn - 1) * ld + nn] * A[nn * ld + nn - 1];
+          }
+          x = A[l * ld + l] * A[l * ld + l] + A[l * ld + l + 1] * A[(l + 1) * ld + l] -
+              s * A[l * ld + l] + t;
+          y = A[(l + 1) * ld + l] * (A[l * ld + l] + A[(l + 1) * ld + l + 1] - s);
+          z = A[(l + 1) * ld + l] * A[(l + 2) * ld + l + 1];
+        } else {
+          x = A[k * ld + k - 1];
+          y = A[(k + 1) * ld + k - 1];
+          z = len == 3 ? A[(k + 2) * ld + k - 1] : 0.0;
+        }
+        // tau = 2 / |v|^2 = 1 / (|x| (|x| + x0)): a reciprocal square root and a
+        // reciprocal (a square root and a division are half of the chain more)
+        const double ss = x * x + y * y + z * z;
+        const double rn = rsqrt(ss), nrm = ss * rn;
         const double alpha = (x >= 0.0) ? -nrm : nrm;
         v[0] = x - alpha;
         v[1] = y;
-        v[2] = (len == 3) ? z : 0.0;
-        const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-        v[3] = (nrm > 0.0 && vv > 0.0) ? 2.0 / vv : 0.0;
+        v[2] = z;
+        v[3] = (ss > 0.0) ? rn * __drcp_rn(nrm + fabs(x)) : 0.0;
         v[4] = alpha;
       }
       __syncthreads();
       const double tau = v[3];
       if (tau != 0.0) {
-        const int c0 = (k > l) ? k - 1 : l;
+        // I - tau v v^T on rows k.. of A, then on columns k.. of A (rows up to r1) and Z
+        const double v0 = v[0], v1 = v[1], v2 = v[2];
+        const double t0 = tau * v0, t1 = tau * v1, t2 = tau * v2;
+        const int c0 = (k > l) ? k : l;  // (column k - 1 is known)
         const int r1 = (k + 3 <= nn) ? k + 3 : nn;
-        apply_reflector(A, Z, N, k, len, v, tau, c0, r1);
-        if (tid == 0 && k > l) {
-          A[k * N + k - 1] = v[4];
-          A[(k + 1) * N + k - 1] = 0.0;
-          if (len == 3) A[(k + 2) * N + k - 1] = 0.0;
+        for (int j = c0 + tid; j < N; j += nt) {
+          double* M = A + k * ld + j;
+          const double x = M[0], y = M[ld], z = len == 3 ? M[2 * ld] : 0.0;
+          const double s = v0 * x + v1 * y + v2 * z;
+          M[0] = x - s * t0;
+          M[ld] = y - s * t1;
+          if (len == 3) M[2 * ld] = z - s * t2;
         }
-      }
-      __syncthreads();
-      if (k < nn - 1) {
-        x = A[(k + 1) * N + k];
-        y = A[(k + 2) * N + k];
-        z = (k < nn - 2) ? A[(k + 3) * N + k] : 0.0;
+        __syncthreads();
+        for (int i = tid; i < (r1 + 1) + N; i += nt) {
+          double* M = (i <= r1 ? A + i * ld : Z + (i - (r1 + 1)) * ld) + k;
+          const double x = M[0], y = M[1], z = len == 3 ? M[2] : 0.0;
+          const double s = x * v0 + y * v1 + z * v2;
+          M[0] = x - s * t0;
+          M[1] = y - s * t1;
+          if (len == 3) M[2] = z - s * t2;
+        }
+        if (tid == 0 && k > l) {
+          A[k * ld + k - 1] = v[4];
+          A[(k + 1) * ld + k - 1] = 0.0;
+          if (len == 3) A[(k + 2) * ld + k - 1] = 0.0;
+        }
       }
       __syncthreads();
     }
@@ -285,11 +297,15 @@ __device__ bool francis(double* A, double* Z, double* wr, double* wi, int N, dou
 // eigenvectors of the quasi-triangular T (complex back substitution), then
 // W = Z Y, normalised like dgeev
 __device__ void schur_vectors(const double* T, const double* Z, const double* wr, const double* wi,
-                              int N, double* Y, double* W, double* sh) {
+                              int N, int ld, double* Y, double* W, double* sh) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const double eps = 2.220446049250313e-16;
   double tnorm = 0.0;
-  for (int e = 0; e < N * N; ++e) tnorm = fmax(tnorm, fabs(T[e]));
+  for (int e = tid; e < N * N; e += nt) tnorm = fmax(tnorm, fabs(T[e / N * ld + e % N]));
+  tnorm = warp_max(tnorm);
+  if ((tid & 31) == 0) sh[tid >> 5] = tnorm;
+  __syncthreads();
+  for (int w = 0; w < nt / 32; ++w) tnorm = fmax(tnorm, sh[w]);
   const double smin = fmax(eps * tnorm, 1e-300);
   // one thread per eigenvalue column k (sequential solve, N^2)
   for (int k = tid; k < N; k += nt) {
@@ -301,27 +317,27 @@ __device__ void schur_vectors(const double* T, const double* Z, const double* wr
       y[k] = {1.0, 0.0};
       top = k;
     } else if (wi[k] > 0.0) {  // block rows k, k+1
-      const double c = T[(k + 1) * N + k];
+      const double c = T[(k + 1) * ld + k];
       y[k + 1] = {1.0, 0.0};
-      y[k] = cdiv({lam.re - T[(k + 1) * N + k + 1], lam.im}, {c, 0.0});
+      y[k] = cdiv({lam.re - T[(k + 1) * ld + k + 1], lam.im}, {c, 0.0});
       top = k;
     } else {  // second of a pair (rows k-1, k)
-      const double c = T[k * N + k - 1];
+      const double c = T[k * ld + k - 1];
       y[k] = {1.0, 0.0};
-      y[k - 1] = cdiv({lam.re - T[k * N + k], lam.im}, {c, 0.0});
+      y[k - 1] = cdiv({lam.re - T[k * ld + k], lam.im}, {c, 0.0});
       top = k - 1;
     }
     const int bottom = (wi[k] > 0.0) ? k + 1 : k;
     int i = top - 1;
     while (i >= 0) {
-      const bool pair = (i > 0) && (T[i * N + i - 1] != 0.0);
+      const bool pair = (i > 0) && (T[i * ld + i - 1] != 0.0);
       if (!pair) {
         cplx r = {0.0, 0.0};
         for (int j = i + 1; j <= bottom; ++j) {
-          r.re += T[i * N + j] * y[j].re;
-          r.im += T[i * N + j] * y[j].im;
+          r.re += T[i * ld + j] * y[j].re;
+          r.im += T[i * ld + j] * y[j].im;
         }
-        cplx den = {T[i * N + i] - lam.re, -lam.im};
+        cplx den = {T[i * ld + i] - lam.re, -lam.im};
         if (cabs2(den) < smin * smin) den = {smin, 0.0};
         y[i] = cdiv({-r.re, -r.im}, den);
         i -= 1;
@@ -329,15 +345,15 @@ __device__ void schur_vectors(const double* T, const double* Z, const double* wr
         // rows i-1, i jointly
         cplx r0 = {0.0, 0.0}, r1 = {0.0, 0.0};
         for (int j = i + 1; j <= bottom; ++j) {
-          r0.re += T[(i - 1) * N + j] * y[j].re;
-          r0.im += T[(i - 1) * N + j] * y[j].im;
-          r1.re += T[i * N + j] * y[j].re;
-          r1.im += T[i * N + j] * y[j].im;
+          r0.re += T[(i - 1) * ld + j] * y[j].re;
+          r0.im += T[(i - 1) * ld + j] * y[j].im;
+          r1.re += T[i * ld + j] * y[j].re;
+          r1.im += T[i * ld + j] * y[j].im;
         }
-        const cplx a11 = {T[(i - 1) * N + i - 1] - lam.re, -lam.im};
-        const cplx a12 = {T[(i - 1) * N + i], 0.0};
-        const cplx a21 = {T[i * N + i - 1], 0.0};
-        const cplx a22 = {T[i * N + i] - lam.re, -lam.im};
+        const cplx a11 = {T[(i - 1) * ld + i - 1] - lam.re, -lam.im};
+        const cplx a12 = {T[(i - 1) * ld + i], 0.0};
+        const cplx a21 = {T[i * ld + i - 1], 0.0};
+        const cplx a22 = {T[i * ld + i] - lam.re, -lam.im};
         cplx det = cmul(a11, a22);
         cplx t2 = cmul(a12, a21);
         det.re -= t2.re;
@@ -362,8 +378,8 @@ __device__ void schur_vectors(const double* T, const double* Z, const double* wr
     const int i = e / N, k = e % N;
     cplx s = {0.0, 0.0};
     for (int j = 0; j < N; ++j) {
-      s.re += Z[i * N + j] * Yc[(size_t)k * N + j].re;
-      s.im += Z[i * N + j] * Yc[(size_t)k * N + j].im;
+      s.re += Z[i * ld + j] * Yc[(size_t)k * N + j].re;
+      s.im += Z[i * ld + j] * Yc[(size_t)k * N + j].im;
     }
     Wc[(size_t)i * N + k] = s;
   }
@@ -394,49 +410,93 @@ __device__ void schur_vectors(const double* T, const double* Z, const double* wr
 }
 
 // -------------------------------------------------------------------------
-// the reduced stage: Atilde, its eigenpairs (Hessenberg + Francis, the Schur
-// vectors) and the Vandermonde rows in one CTA; P, q and the mode matrix in
-// kernels spread over the GPU (their FP64 sums over the snapshots were 57 %
-// of the one-CTA version's cycles); the amplitude solve in one CTA
+// the reduced stage: its sums over the snapshots (Atilde, P, q, the mode matrix)
+// and the Vandermonde rows are spread over the GPU; the eigenpairs (Hessenberg +
+// Francis, the Schur vectors) and the amplitude solve take one CTA each.  r = 32,
+// 511 snapshots: 3.5 ms with Atilde and the Vandermonde rows in the eigen kernel's
+// CTA and all matrices in global memory, 2.0 ms like this.
 // -------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) dmd_eig_kernel(const double* __restrict__ aux1,
-                                                          const double* __restrict__ S,
-                                                          const double* __restrict__ VT, int N,
-                                                          int nt, DmdBufs B, double* muR,
-                                                          double* muI, double* bJov, double* Mphi,
-                                                          int* info) {
-  (void)muR;
-  (void)muI;
-  (void)bJov;
-  (void)Mphi;
-  extern __shared__ double sh[];
+// Atilde[i][j] = sum_t aux1[i][t] VT[j][t] / S[j], one warp per element
+__global__ void __launch_bounds__(256) dmd_atilde_kernel(const double* __restrict__ aux1,
+                                                         const double* __restrict__ S,
+                                                         const double* __restrict__ VT, int N,
+                                                         int nt, double* __restrict__ A) {
+  const int lane = threadIdx.x & 31;
+  const int e = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (e >= N * N) return;
+  const int i = e / N, j = e % N;
+  double s = 0.0;
+  for (int t = lane; t < nt; t += 32) s += aux1[(size_t)i * nt + t] * VT[(size_t)j * nt + t];
+  s = warp_sum(s);
+  if (lane == 0) A[e] = s / S[j];
+}
+
+// shared memory of the eigen kernel: scratch, then A and Z (odd pitch), the
+// eigenvalues and the eigenvectors of T as far as they fit
+constexpr size_t DMD_SMEM_MAX = 200 * 1024;
+static size_t dmd_eig_smem(int N, bool& mats, bool& vecs) {
+  const size_t ld = N | 1;
+  size_t b = sizeof(double) * (2 * (size_t)N + 16);
+  mats = b + sizeof(double) * (2 * N * ld + 2 * N) <= DMD_SMEM_MAX;
+  if (mats) b += sizeof(double) * (2 * N * ld + 2 * N);
+  vecs = mats && b + sizeof(double) * 2 * N * N <= DMD_SMEM_MAX;
+  if (vecs) b += sizeof(double) * 2 * N * N;
+  return b;
+}
+
+__global__ void __launch_bounds__(256) dmd_eig_kernel(int N, DmdBufs B, int mats, int vecs,
+                                                      int* info) {
+  extern __shared__ __align__(16) double sh[];
   const int tid = threadIdx.x, nthr = blockDim.x;
-  // Atilde[i][j] = sum_t aux1[i][t] VT[j][t] / S[j]
-  for (int e = tid; e < N * N; e += nthr) {
-    const int i = e / N, j = e % N;
-    double s = 0.0;
-    for (int t = 0; t < nt; ++t) s += aux1[(size_t)i * nt + t] * VT[(size_t)j * nt + t];
-    B.A[e] = s / S[j];
+  const int ld = mats ? N | 1 : N;
+  double *A = B.A, *Z = B.Z, *wr = B.wr, *wi = B.wi, *Y = B.Y;
+  if (mats) {
+    double* q = sh + 2 * N + 16;
+    if (vecs) {  // (16-byte elements first)
+      Y = q;
+      q += 2 * (size_t)N * N;
+    }
+    A = q;
+    Z = A + (size_t)N * ld;
+    wr = Z + (size_t)N * ld;
+    wi = wr + N;
+    for (int e = tid; e < N * N; e += nthr) A[e / N * ld + e % N] = B.A[e];
   }
   __syncthreads();
-  hessenberg(B.A, B.Z, N, sh);
-  if (!francis(B.A, B.Z, B.wr, B.wi, N, sh)) {
+  hessenberg(A, Z, N, ld, sh);
+  if (!francis(A, Z, wr, wi, N, ld, sh)) {
     if (tid == 0) atomicMax(&info[ST_FAIL], PLOM_NUM_EIG);
     return;
   }
   __syncthreads();
-  schur_vectors(B.A, B.Z, B.wr, B.wi, N, B.Y, B.Wv, sh);
-  cplx* V = reinterpret_cast<cplx*>(B.Vr);
-  // Vandermonde rows mu_i^t by repeated multiplication
-  for (int i = tid; i < N; i += nthr) {
-    const cplx mu = {B.wr[i], B.wi[i]};
-    cplx p = {1.0, 0.0};
-    for (int t = 0; t < nt; ++t) {
-      V[(size_t)i * nt + t] = p;
-      p = cmul(p, mu);
+  schur_vectors(A, Z, wr, wi, N, ld, Y, B.Wv, sh);
+  if (mats)
+    for (int i = tid; i < N; i += nthr) {
+      B.wr[i] = wr[i];
+      B.wi[i] = wi[i];
     }
+}
+
+// Vandermonde rows mu_i^t: a thread multiplies through 16 of them, from a power by
+// squaring
+__global__ void __launch_bounds__(128) dmd_vand_kernel(int N, int nt, DmdBufs B,
+                                                       const int* __restrict__ info) {
+  if (info[ST_FAIL]) return;
+  const int per = (nt + 15) / 16;
+  const int e = blockIdx.x * 128 + threadIdx.x;
+  if (e >= N * per) return;
+  const int i = e / per, t0 = e % per * 16;
+  const cplx mu = {B.wr[i], B.wi[i]};
+  cplx p = {1.0, 0.0}, sq = mu;
+  for (int b = t0; b > 0; b >>= 1) {
+    if (b & 1) p = cmul(p, sq);
+    sq = cmul(sq, sq);
   }
-  __syncthreads();
+  cplx* V = reinterpret_cast<cplx*>(B.Vr) + (size_t)i * nt;
+  for (int t = t0; t < min(nt, t0 + 16); ++t) {
+    V[t] = p;
+    p = cmul(p, mu);
+  }
 }
 
 // P = (W^H W) o conj(Vand Vand^H) (one warp per element) and
@@ -504,85 +564,95 @@ __global__ void __launch_bounds__(256) dmd_pq_kernel(const double* __restrict__ 
   }
 }
 
-// Cholesky solve for the amplitudes, the ordering and the conjugate-pair
-// fix-up flags (one CTA)
-__global__ void __launch_bounds__(256) dmd_amp_kernel(int N, DmdBufs B, double* muR, double* muI,
-                                                      double* bJov, int* info) {
+// Cholesky solve for the amplitudes, the ordering and the conjugate-pair fix-up
+// flags (one CTA; P in shared memory where it fits).  Right-looking: a column, the
+// trailing update by all threads, two barriers.
+__global__ void __launch_bounds__(256) dmd_amp_kernel(int N, DmdBufs B, int psh, double* muR,
+                                                      double* muI, double* bJov, int* info) {
+  extern __shared__ __align__(16) double sh[];
   if (info[ST_FAIL]) return;
-  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+  cplx* b = reinterpret_cast<cplx*>(sh);      // N
+  double* babs = sh + 2 * N;                  // N
   cplx* P = reinterpret_cast<cplx*>(B.Pm);
-  cplx* q = reinterpret_cast<cplx*>(B.qv);
-  // Cholesky P = L L^H (in place, lower), then solve L L^H b = q
-  cplx* b = reinterpret_cast<cplx*>(B.bv);
+  if (psh) {
+    P = reinterpret_cast<cplx*>(sh + 3 * N + (N & 1));
+    const cplx* G = reinterpret_cast<const cplx*>(B.Pm);
+    for (int e = tid; e < N * N; e += nthr) P[e] = G[e];
+  }
+  for (int i = tid; i < N; i += nthr) b[i] = reinterpret_cast<const cplx*>(B.qv)[i];
   __shared__ int bad;
   if (tid == 0) bad = 0;
   __syncthreads();
+  // Cholesky P = L L^H (in place, lower), then solve L L^H b = q
   for (int j = 0; j < N; ++j) {
-    if (tid == 0) {
-      double d = P[(size_t)j * N + j].re;
-      for (int k = 0; k < j; ++k) d -= cabs2(P[(size_t)j * N + k]);
-      if (!(d > 0.0) || !isfinite(d)) {
-        bad = 1;
-        d = 1e-300;
-      }
-      P[(size_t)j * N + j] = {sqrt(d), 0.0};
+    double d = P[(size_t)j * N + j].re;
+    const bool neg = !(d > 0.0) || !isfinite(d);
+    d = neg ? 1e-150 : sqrt(d);
+    if (tid == 0 && neg) bad = 1;
+    for (int i = j + 1 + tid; i < N; i += nthr) {
+      const cplx s = P[(size_t)i * N + j];
+      P[(size_t)i * N + j] = {s.re / d, s.im / d};
     }
     __syncthreads();
-    const double ljj = P[(size_t)j * N + j].re;
-    for (int i = j + 1 + tid; i < N; i += nthr) {
-      cplx s = P[(size_t)i * N + j];
-      for (int k = 0; k < j; ++k) {
-        const cplx ab = cmul(P[(size_t)i * N + k], cconj(P[(size_t)j * N + k]));
-        s.re -= ab.re;
-        s.im -= ab.im;
-      }
-      P[(size_t)i * N + j] = {s.re / ljj, s.im / ljj};
+    if (tid == 0) P[(size_t)j * N + j] = {d, 0.0};
+    const int len = N - 1 - j;
+    for (int e = tid; e < len * len; e += nthr) {
+      const int i = j + 1 + e / len, k = j + 1 + e % len;
+      if (k > i) continue;
+      const cplx ab = cmul(P[(size_t)i * N + j], cconj(P[(size_t)k * N + j]));
+      P[(size_t)i * N + k].re -= ab.re;
+      P[(size_t)i * N + k].im -= ab.im;
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    if (bad) atomicMax(&info[ST_FAIL], PLOM_NUM_CHOLESKY);
+  if (tid < 32) {
+    if (lane == 0 && bad) atomicMax(&info[ST_FAIL], PLOM_NUM_CHOLESKY);
     // forward: L z = q
     for (int i = 0; i < N; ++i) {
-      cplx s = q[i];
-      for (int k = 0; k < i; ++k) {
-        const cplx ab = cmul(P[(size_t)i * N + k], b[k]);
-        s.re -= ab.re;
-        s.im -= ab.im;
+      const double d = P[(size_t)i * N + i].re;
+      const cplx z = {b[i].re / d, b[i].im / d};
+      __syncwarp();
+      if (lane == 0) b[i] = z;
+      for (int r = i + 1 + lane; r < N; r += 32) {
+        const cplx ab = cmul(P[(size_t)r * N + i], z);
+        b[r].re -= ab.re;
+        b[r].im -= ab.im;
       }
-      b[i] = {s.re / P[(size_t)i * N + i].re, s.im / P[(size_t)i * N + i].re};
+      __syncwarp();
     }
     // backward: L^H b = z
     for (int i = N - 1; i >= 0; --i) {
-      cplx s = b[i];
-      for (int k = i + 1; k < N; ++k) {
-        const cplx ab = cmul(cconj(P[(size_t)k * N + i]), b[k]);
-        s.re -= ab.re;
-        s.im -= ab.im;
+      const double d = P[(size_t)i * N + i].re;
+      const cplx z = {b[i].re / d, b[i].im / d};
+      __syncwarp();
+      if (lane == 0) b[i] = z;
+      for (int r = lane; r < i; r += 32) {
+        const cplx ab = cmul(cconj(P[(size_t)i * N + r]), z);
+        b[r].re -= ab.re;
+        b[r].im -= ab.im;
       }
-      b[i] = {s.re / P[(size_t)i * N + i].re, s.im / P[(size_t)i * N + i].re};
-    }
-    // order: |b| descending (ties: larger index first, as flip(argsort))
-    for (int i = 0; i < N; ++i) B.babs[i] = sqrt(cabs2(b[i]));
-    for (int i = 0; i < N; ++i) {
-      int rank = 0;
-      for (int k = 0; k < N; ++k)
-        rank += (B.babs[k] > B.babs[i]) || (B.babs[k] == B.babs[i] && k > i);
-      B.order[rank] = i;
+      __syncwarp();
     }
   }
   __syncthreads();
-  // ordered eigenvalues / amplitudes and the pair fix-up flags
-  int* flip_tab = B.flip;
+  // order: |b| descending (ties: larger index first, as flip(argsort))
+  for (int i = tid; i < N; i += nthr) babs[i] = sqrt(cabs2(b[i]));
+  __syncthreads();
+  for (int i = tid; i < N; i += nthr) {
+    const double bi = babs[i];
+    int rank = 0;
+    for (int k = 0; k < N; ++k) rank += (babs[k] > bi) || (babs[k] == bi && k > i);
+    B.order[rank] = i;
+    muR[rank] = B.wr[i];
+    muI[rank] = B.wi[i];
+    bJov[2 * rank] = b[i].re;
+    bJov[2 * rank + 1] = b[i].im;
+    B.flip[rank] = 0;
+  }
+  __syncthreads();
+  // the pair fix-up flags
   if (tid == 0) {
-    for (int j = 0; j < N; ++j) {
-      const int o = B.order[j];
-      muR[j] = B.wr[o];
-      muI[j] = B.wi[o];
-      bJov[2 * j] = b[o].re;
-      bJov[2 * j + 1] = b[o].im;
-      if (j < 1024) flip_tab[j] = 0;
-    }
     bool skip = false;
     for (int j = 0; j < N; ++j) {
       if (skip) {
@@ -595,14 +665,13 @@ __global__ void __launch_bounds__(256) dmd_amp_kernel(int N, DmdBufs B, double* 
         muI[j + 1] = -muI[j];
         bJov[2 * j + 1] = bJov[2 * (j + 1) + 1];
         bJov[2 * (j + 1) + 1] = -bJov[2 * j + 1];
-        if (j < 1024) flip_tab[j] = 1;
+        B.flip[j] = 1;
         skip = true;
       } else if (muI[j] > 0.0) {
         skip = true;
       }
     }
   }
-  __syncthreads();
 }
 
 // Mphi[t][j] = sum_k VT[k][t] / S_k * W[k][o_j] / mu_{o_j} (one thread per
@@ -654,8 +723,6 @@ size_t dmd_reduced_workspace(int N, int nt) {
   a.take<double>((size_t)2 * N * N);
   a.take<double>((size_t)2 * N * N);
   a.take<double>((size_t)2 * N);
-  a.take<double>((size_t)2 * N);
-  a.take<double>(N);
   a.take<int>(N);
   a.take<double>((size_t)2 * N * nt);
   a.take<int>(N);
@@ -691,23 +758,38 @@ extern "C" int plom_dmd_reduced(const double* aux1, const double* S, const doubl
   B.Y = a.take<double>((size_t)2 * N * N);
   B.Pm = a.take<double>((size_t)2 * N * N);
   B.qv = a.take<double>((size_t)2 * N);
-  B.bv = a.take<double>((size_t)2 * N);
-  B.babs = a.take<double>(N);
   B.order = a.take<int>(N);
   B.Vr = a.take<double>((size_t)2 * N * T);
   B.flip = a.take<int>(N);
   cudaStream_t st = (cudaStream_t)stream;
   PLOM_CHECK_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * PLOM_INFO_WORDS, st));
-  const size_t shbytes = sizeof(double) * (2 * (size_t)N + 16);
-  PLOM_REQUIRE(shbytes <= 48 * 1024, PLOM_ERR_ARG, "dmd_reduced: r too large for one CTA");
-  ProfScope prof("dmd_reduced_fp64", st, 0.0, 0.0, 5);
-  // eigenpairs of Atilde and the Vandermonde rows (one CTA), P and q (spread
-  // over the GPU), the amplitude solve and ordering (one CTA), the mode matrix
-  dmd_eig_kernel<<<1, 256, shbytes, st>>>(aux1, S, VT, N, T, B, muReal, muImag, bJov, Mphi, info);
+  bool mats, vecs;
+  const size_t esm = dmd_eig_smem(N, mats, vecs);
+  const size_t bsm = sizeof(double) * (3 * (size_t)N + (N & 1));
+  const bool psh = bsm + sizeof(double) * 2 * N * N <= DMD_SMEM_MAX;
+  const size_t asm_ = bsm + (psh ? sizeof(double) * 2 * N * N : 0);
+  PLOM_REQUIRE(esm <= DMD_SMEM_MAX && asm_ <= DMD_SMEM_MAX, PLOM_ERR_ARG,
+               "dmd_reduced: r too large for one CTA");
+  static bool attr = false;
+  if (!attr) {
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(dmd_eig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)DMD_SMEM_MAX));
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(dmd_amp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)DMD_SMEM_MAX));
+    attr = true;
+  }
+  ProfScope prof("dmd_reduced_fp64", st, 0.0, 0.0, 7);
+  // Atilde, its eigenpairs (one CTA), the Vandermonde rows, P and q, the amplitude
+  // solve and ordering (one CTA), the mode matrix
+  dmd_atilde_kernel<<<(unsigned)((N * N + 7) / 8), 256, 0, st>>>(aux1, S, VT, N, T, B.A);
+  PLOM_CHECK_LAUNCH();
+  dmd_eig_kernel<<<1, N <= 40 ? 128 : 256, esm, st>>>(N, B, mats, vecs, info);
+  PLOM_CHECK_LAUNCH();
+  dmd_vand_kernel<<<(unsigned)cdiv((int64_t)N * ((T + 15) / 16), 128), 128, 0, st>>>(N, T, B, info);
   PLOM_CHECK_LAUNCH();
   dmd_pq_kernel<<<(unsigned)((N * N + 7) / 8 + N), 256, 0, st>>>(S, VT, N, T, B, info);
   PLOM_CHECK_LAUNCH();
-  dmd_amp_kernel<<<1, 256, 0, st>>>(N, B, muReal, muImag, bJov, info);
+  dmd_amp_kernel<<<1, 256, asm_, st>>>(N, B, psh, muReal, muImag, bJov, info);
   PLOM_CHECK_LAUNCH();
   dmd_mphi_kernel<<<(unsigned)cdiv((int64_t)T * N, 256), 256, 0, st>>>(S, VT, N, T, B, Mphi, info);
   PLOM_CHECK_LAUNCH();
