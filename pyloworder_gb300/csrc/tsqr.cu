@@ -45,16 +45,18 @@ static bool packed_ok(int64_t m) { return m >= 1 && m < (1ll << 31); }
 template <typename TA>
 static int tall_gram(int prec, const TA* A, int64_t lda, int64_t m, int64_t N, double* G,
                      int* err, Arena& ws, cudaStream_t st) {
-  if (prec == PLOM_PREC_FP64 || sizeof(TA) == 8) return oz_gram<TA>(A, lda, m, N, G, ws, st);
   if constexpr (sizeof(TA) == 4) {
-    if (packed_ok(m)) {
-      Packed p;
-      packed_carve(ws, p, m, N);
-      PLOM_TRY(pack_f32(A, lda, m, N, p, ws, st));
-      return gram_packed(p, G, err, ws, st);
+    if (prec != PLOM_PREC_FP64) {
+      if (packed_ok(m)) {
+        Packed p;
+        packed_carve(ws, p, m, N);
+        PLOM_TRY(pack_f32(A, lda, m, N, p, ws, st));
+        return gram_packed(p, G, err, ws, st);
+      }
+      return gemm_tn<TA, TA, float, double>(A, lda, A, lda, G, N, N, N, m, true, ws, st);
     }
-    return gemm_tn<TA, TA, float, double>(A, lda, A, lda, G, N, N, N, m, true, ws, st);
   }
+  return oz_gram<TA>(A, lda, m, N, G, ws, st);
 }
 
 // C(m x k) = A(m x N) W(N x k), W in FP64 (converted for the mixed form)
@@ -639,6 +641,21 @@ static int tsqr_packed(const float* X, int64_t m, int n, int64_t ldx, float* Q, 
   return PLOM_OK;
 }
 
+// Q alone, packed (its planes hold P1 until the last product writes them)
+static int tsqr_packed_q(const float* X, int64_t m, int n, int64_t ldx, Packed& Q, int* info,
+                         Arena& ws, cudaStream_t st) {
+  PackedCore b;
+  carve_packed_core(ws, b, m, n, true, Q.hi);
+  if (!ws.measuring()) PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "tsqr: workspace too small");
+  const size_t mark = ws.off;
+  PLOM_TRY(cholqr3_packed(false, X, m, n, ldx, b, info, ws, st));
+  const size_t need = ws.off;
+  ws.off = mark;
+  PLOM_TRY(apply_packed(b.P2, b.W3, n, n, nullptr, 0, &Q, info, ws, st, 0, 0, true));
+  ws.off = std::max(need, ws.off);
+  return PLOM_OK;
+}
+
 template <typename TI, typename TC>
 static void carve_core(Arena& ws, CoreBufs<TI, TC>& b, int64_t m, int N, bool need_q1) {
   const size_t nn = (size_t)N * N;
@@ -755,7 +772,10 @@ static int tsqr_impl(int prec, const TI* X, int64_t m, int n, int64_t ldx, TI* Q
 // randomized SVD (pyLOM/vmmath/svd.py:121-144, 255-273; svd.c:1267-1519)
 // ---------------------------------------------------------------------------
 // Mixed form on FP32 data: A is packed once; the passes over it (A Omega,
-// A^T Q, A Q2, Q^T A) run on the tensor cores from the packed planes.
+// A^T Q, A Q2, Q^T A) run on the tensor cores from the packed planes.  The range
+// bases Q are written packed by the factorization's last product: they are read
+// only by products (FP32 copies, their column maxima and their packing took
+// 1.3 of 23 ms at 2,097,152 x 512, r = 80).
 // Two modes: randomized_svd (U, S, VT) and, with `qr`, randomized_qr (Q m x r
 // with Householder QR's column signs into Qout (ldq), B = Q^T A r x n into
 // Bout).  omega_in (n x r, or null): the test matrix instead of Philox(seed).
@@ -769,9 +789,7 @@ static int rsvd_packed(const float* A, int64_t m, int64_t n, int64_t lda, int r,
   float* omega = ws.take<float>((size_t)n * r);
   double* om64 = ws.take<double>((size_t)n * r);
   float* Y = ws.take<float>((size_t)m * r);
-  float* Qm = qr ? Qout : ws.take<float>((size_t)m * r);
-  const int64_t ldqm = qr ? ldq : r;
-  float* Rq = ws.take<float>((size_t)r * r);
+  float* Rq = qr ? ws.take<float>((size_t)r * r) : nullptr;
   double* Q2 = ws.take<double>((size_t)n * r);  // A^T Q (n x r); the last one is B^T
   double* Ub = qr ? nullptr : ws.take<double>((size_t)n * r);
   double* Sb = qr ? nullptr : ws.take<double>(r);
@@ -801,10 +819,13 @@ static int rsvd_packed(const float* A, int64_t m, int64_t n, int64_t lda, int r,
   // Y = A Omega
   PLOM_TRY(sub([&] { return apply_packed(Ap, om64, r, r, Y, r, nullptr, info, ws, st); }));
   for (int j = 0; j <= q; ++j) {
-    // only the final range basis needs Householder QR's signs
-    const bool hh = qr && j == q;
-    PLOM_TRY(sub([&] { return tsqr_packed(Y, m, r, r, Qm, ldqm, Rq, info, ws, st, hh); }));
-    PLOM_TRY(sub([&] { return pack_f32(Qm, ldqm, m, r, Qp, ws, st); }));
+    // only randomized_qr's final range basis is a result, with Householder QR's signs
+    if (qr && j == q) {
+      PLOM_TRY(sub([&] { return tsqr_packed(Y, m, r, r, Qout, ldq, Rq, info, ws, st, true); }));
+      PLOM_TRY(sub([&] { return pack_f32(Qout, ldq, m, r, Qp, ws, st); }));
+    } else {
+      PLOM_TRY(sub([&] { return tsqr_packed_q(Y, m, r, r, Qp, info, ws, st); }));
+    }
     // Q2 = A^T Q (n x r); after the last iteration this is B^T = (Q^T A)^T
     PLOM_TRY(sub([&] { return tn_packed(Ap, Qp, Q2, r, info, ws, st); }));
     if (j == q) break;
@@ -830,7 +851,7 @@ static int rsvd_packed(const float* A, int64_t m, int64_t n, int64_t lda, int r,
     PLOM_TRY((convert<double, float>(Vo, VT, (int64_t)r * n, st)));
   }
   // U = Q Ur
-  PLOM_TRY(sub([&] { return tall_apply<float, float>(PLOM_PREC_MIXED, Qm, r, m, r, Ur, r, U, ldu, info, ws, st); }));
+  PLOM_TRY(sub([&] { return apply_packed(Qp, Ur, r, r, U, ldu, nullptr, info, ws, st); }));
   ws.off = need;
   return PLOM_OK;
 }
