@@ -4,9 +4,9 @@
 //
 // GB300 mapping: one warp per row, 16-byte vector loads/stores when the row
 // start and length allow it.  f64 data accumulate in FP64; f32 data in FP32
-// with compensated (Kahan) per-lane sums folded into FP64 across the warp (no
-// per-element FP64 instruction: GB300's FP64 rate is 1/64 of FP32), and the
-// mean is subtracted in FP32 as the reference's float32 path does.
+// with compensated (Kahan) per-lane sums folded across the warp in double-float
+// (no FP64 instruction: GB300's FP64 rate is 1/64 of FP32), and the mean is
+// subtracted in FP32 as the reference's float32 path does.
 // All modes are HBM-bound: algorithmic bytes = read m*n*s (+ write m*n*s when
 // Y is produced).  A row is re-read from L1/L2 for the second and third
 // sweeps (variance, write-out), never from HBM for rows up to ~64 KB.
@@ -14,6 +14,8 @@
 // Reference behaviour (pyLowOrder): pyLOM/vmmath/src/averaging.c:10-157,
 // pyLOM/vmmath/averaging.py:18-75.  Variance is the population variance
 // (np.var, divide by n) and norm_variance divides by the variance itself.
+#include <type_traits>
+
 #include "plom_common.cuh"
 
 namespace plom {
@@ -63,8 +65,29 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
   s = t;
 }
 
-// f32 rows: FP32 compensated sums (see the file comment)
-template <bool VEC>
+// sum over the warp of the lanes' hi + lo, and its mean: TwoSum in FP32 and one
+// corrected FP32 division.  In FP64 the five adds and the division took 320 cycles of
+// the SM's FP64 pipe per row, more than the row's bytes need (2,097,152 x 512 with
+// write-out: 2.14 ms, 1.26 with these: 6.8 TB/s).
+__device__ __forceinline__ float row_mean(float hi, float lo, int64_t n) {
+  const float h0 = hi, l0 = lo;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+    const float t = hi + h2, bb = t - hi;
+    lo += l2 + ((hi - (t - bb)) + (h2 - bb));
+    hi = t;
+  }
+  if (n >= (1 << 24) || !isfinite(hi))  // (the sum of finite lanes may pass FP32's range)
+    return (float)(warp_sum((double)h0 + (double)l0) / (double)n);
+  const float nf = (float)n, q = hi / nf;
+  return q + (fmaf(-q, nf, hi) + lo) / nf;
+}
+
+// f32 rows: FP32 compensated sums (see the file comment).  One warp per row.  NR > 0:
+// the row fits NR registers (vectors when VEC) per lane and is read once, all loads in
+// flight together; NR = 0: any length.
+template <bool VEC, int NR>
 __global__ void __launch_bounds__(256) row_kernel_f32(const float* __restrict__ X, int64_t m,
                                                       int64_t n, int64_t ldx,
                                                       const float* __restrict__ mean_in,
@@ -73,88 +96,91 @@ __global__ void __launch_bounds__(256) row_kernel_f32(const float* __restrict__ 
                                                       float* __restrict__ var_out, int want_var,
                                                       int ymode, float* __restrict__ Y,
                                                       int64_t ldy) {
+  using V = typename std::conditional<VEC, float4, float>::type;
   const int lane = threadIdx.x & 31;
+  const int64_t nv = VEC ? n / 4 : n;
   const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
+  auto sum = [](const V& a) {
+    if constexpr (VEC) return (a.x + a.y) + (a.z + a.w);
+    else return a;
+  };
+  auto squares = [](const V& a, float mu) {
+    if constexpr (VEC) {
+      const float d0 = a.x - mu, d1 = a.y - mu, d2 = a.z - mu, d3 = a.w - mu;
+      return fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3);
+    } else {
+      const float d = a - mu;
+      return d * d;
+    }
+  };
+  auto centred = [](V a, float mu, float inv, bool norm) {
+    if constexpr (VEC) {
+      a.x -= mu;
+      a.y -= mu;
+      a.z -= mu;
+      a.w -= mu;
+      if (norm) {
+        a.x *= inv;
+        a.y *= inv;
+        a.z *= inv;
+        a.w *= inv;
+      }
+    } else {
+      a -= mu;
+      if (norm) a *= inv;
+    }
+    return a;
+  };
   for (int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < m;
        row += warps_total) {
-    const float* x = X + row * ldx;
-    float muf;
+    const V* x = reinterpret_cast<const V*>(X + row * ldx);
+    V r[NR > 0 ? NR : 1];
+    if constexpr (NR > 0) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q)
+        if (lane + 32 * q < nv) r[q] = __ldg(x + lane + 32 * q);
+    }
+    // f(element) over the lane's elements
+    auto each = [&](auto&& f) {
+      if constexpr (NR > 0) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q)
+          if (lane + 32 * q < nv) f(r[q], lane + 32 * q);
+      } else {
+        int64_t j = lane;
+        for (; j + 96 < nv; j += 128) {  // 4 loads in flight per lane
+          const V a = __ldg(x + j), b = __ldg(x + j + 32), c = __ldg(x + j + 64), d = __ldg(x + j + 96);
+          f(a, j);
+          f(b, j + 32);
+          f(c, j + 64);
+          f(d, j + 96);
+        }
+        for (; j < nv; j += 32) f(__ldg(x + j), j);
+      }
+    };
+    float mu;
     if (mean_in) {
-      muf = mean_in[row];
+      mu = mean_in[row];
     } else {
       float s = 0.f, c = 0.f;
-      if (VEC) {
-        const int64_t nv = n / 4;
-        int64_t j = lane;
-        for (; j + 96 < nv; j += 128) {  // 4 vectors in flight per lane
-          const float4 a = __ldg(reinterpret_cast<const float4*>(x + j * 4));
-          const float4 b = __ldg(reinterpret_cast<const float4*>(x + (j + 32) * 4));
-          const float4 d = __ldg(reinterpret_cast<const float4*>(x + (j + 64) * 4));
-          const float4 e = __ldg(reinterpret_cast<const float4*>(x + (j + 96) * 4));
-          kahan_add(s, c, (a.x + a.y) + (a.z + a.w));
-          kahan_add(s, c, (b.x + b.y) + (b.z + b.w));
-          kahan_add(s, c, (d.x + d.y) + (d.z + d.w));
-          kahan_add(s, c, (e.x + e.y) + (e.z + e.w));
-        }
-        for (; j < nv; j += 32) {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(x + j * 4));
-          kahan_add(s, c, (a.x + a.y) + (a.z + a.w));
-        }
-      } else {
-        for (int64_t j = lane; j < n; j += 32) kahan_add(s, c, x[j]);
-      }
-      const double tot = warp_sum((double)s - (double)c);
-      const double mu = tot / (double)n;
-      muf = (float)mu;
-      if (lane == 0 && mean_out) mean_out[row] = muf;
+      each([&](const V& a, int64_t) { kahan_add(s, c, sum(a)); });
+      mu = row_mean(s, -c, n);
+      if (lane == 0 && mean_out) mean_out[row] = mu;
     }
     float var = 1.f;
     if (want_var) {
-      float s2 = 0.f, c2 = 0.f;
-      if (VEC) {
-        const int64_t nv = n / 4;
-        for (int64_t j = lane; j < nv; j += 32) {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(x + j * 4));
-          const float d0 = a.x - muf, d1 = a.y - muf, d2 = a.z - muf, d3 = a.w - muf;
-          kahan_add(s2, c2, fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3));
-        }
-      } else {
-        for (int64_t j = lane; j < n; j += 32) {
-          const float d = x[j] - muf;
-          kahan_add(s2, c2, d * d);
-        }
-      }
-      const double tot = warp_sum((double)s2 - (double)c2);
-      var = (float)(tot / (double)n);
+      float s = 0.f, c = 0.f;
+      each([&](const V& a, int64_t) { kahan_add(s, c, squares(a, mu)); });
+      var = row_mean(s, -c, n);
       if (lane == 0 && var_out) var_out[row] = var;
     } else if (var_in) {
       var = var_in[row];
     }
     if (ymode != Y_NONE) {
-      const float inv = (ymode == Y_NORM) ? 1.f / var : 1.f;
-      float* y = Y + row * ldy;
-      if (VEC) {
-        const int64_t nv = n / 4;
-        for (int64_t j = lane; j < nv; j += 32) {
-          float4 a = __ldg(reinterpret_cast<const float4*>(x + j * 4));
-          a.x -= muf;
-          a.y -= muf;
-          a.z -= muf;
-          a.w -= muf;
-          if (ymode == Y_NORM) {
-            a.x *= inv;
-            a.y *= inv;
-            a.z *= inv;
-            a.w *= inv;
-          }
-          *reinterpret_cast<float4*>(y + j * 4) = a;
-        }
-      } else {
-        for (int64_t j = lane; j < n; j += 32) {
-          const float d = x[j] - muf;
-          y[j] = (ymode == Y_NORM) ? d * inv : d;
-        }
-      }
+      const bool norm = ymode == Y_NORM;
+      const float inv = norm ? 1.f / var : 1.f;
+      V* y = reinterpret_cast<V*>(Y + row * ldy);
+      each([&](const V& a, int64_t j) { y[j] = centred(a, mu, inv, norm); });
     }
   }
 }
@@ -271,14 +297,23 @@ static int launch_rows(const T* X, int64_t m, int64_t n, int64_t ldx, const T* m
   ProfScope prof("rows_mean_subtract", st, 0.0,
                  (double)m * n * sizeof(T) * (ymode == Y_NONE ? 1.0 : 2.0));
   if constexpr (sizeof(T) == 4) {
+    // registers per lane: up to 1,024 values a row in vectors, 512 one by one
+    auto go = [&](auto kern) {
+      kern<<<(unsigned)blocks, threads, 0, st>>>(X, m, n, ldx, mean_in, var_in, mean_out, var_out,
+                                                 want_var, ymode, Y, ldy);
+    };
+    const int64_t per = cdiv(vec ? n / 4 : n, 32);
     if (vec)
-      row_kernel_f32<true><<<(unsigned)blocks, threads, 0, st>>>(X, m, n, ldx, mean_in, var_in,
-                                                                 mean_out, var_out, want_var,
-                                                                 ymode, Y, ldy);
+      per <= 1   ? go(row_kernel_f32<true, 1>)
+      : per <= 2 ? go(row_kernel_f32<true, 2>)
+      : per <= 4 ? go(row_kernel_f32<true, 4>)
+      : per <= 8 ? go(row_kernel_f32<true, 8>)
+                 : go(row_kernel_f32<true, 0>);
     else
-      row_kernel_f32<false><<<(unsigned)blocks, threads, 0, st>>>(X, m, n, ldx, mean_in, var_in,
-                                                                  mean_out, var_out, want_var,
-                                                                  ymode, Y, ldy);
+      per <= 4    ? go(row_kernel_f32<false, 4>)
+      : per <= 8  ? go(row_kernel_f32<false, 8>)
+      : per <= 16 ? go(row_kernel_f32<false, 16>)
+                  : go(row_kernel_f32<false, 0>);
   } else {
     if (vec)
       row_kernel<T, true><<<(unsigned)blocks, threads, 0, st>>>(X, m, n, ldx, mean_in, var_in,

@@ -1,0 +1,45 @@
+"""Row kernels on FP32 rows at the edges of their register forms (32, 64, 128 and
+256 vectors a row, or 128, 256 and 512 single values), strided and misaligned.
+
+The mean and the variance are FP32 roundings of sums that carry twice FP32's
+digits: one unit in the last place (the variance twice, for the rounding of its
+mean)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -23
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 31, 32, 33, 127, 128, 129, 130, 255, 256, 257, 260, 511, 512, 513, 516, 1023,
+                               1024, 1025, 1028, 5000])
+@pytest.mark.parametrize("ld,off", [(0, 0), (4, 4), (3, 1)])
+def test_rows(n, ld, off):
+    import pyloworder_gb300 as P
+    rng = np.random.default_rng(n + ld)
+    W = (rng.standard_normal((77, n + ld)) + 30.0).astype(np.float32)
+    X = torch.from_numpy(W).cuda()[:, off:off + n]
+    A = W[:, off:off + n].astype(np.float64)
+    mean = P.math.temporal_mean(X).cpu().numpy()
+    ex = A.mean(1)
+    assert np.all(np.abs(mean - ex) <= EPS * np.abs(ex))
+    D = A.astype(np.float32) - mean[:, None]
+    Y = P.math.subtract_mean(X, torch.from_numpy(mean).cuda()).cpu().numpy()
+    assert np.array_equal(Y, D)
+    if n > 1:
+        var = P.math.temporal_variance(X, torch.from_numpy(mean).cuda()).cpu().numpy().ravel()
+        ev = ((A - mean[:, None].astype(np.float64)) ** 2).mean(1)
+        # a difference rounds by half a unit, its square by as much again
+        assert np.all(np.abs(var - ev) <= 2 * EPS * ev)
+        Z = P.math.norm_variance(X, torch.from_numpy(mean).cuda(), torch.from_numpy(var).cuda()).cpu().numpy()
+        assert np.all(np.abs(Z - D / var[:, None].astype(np.float64)) <= 2 * EPS * np.abs(Z))
+
+
+def test_range():
+    import pyloworder_gb300 as P
+    for v in (1e37, 1.0, 1e-40, 0.0):
+        X = torch.full((3, 600), v, dtype=torch.float32, device="cuda")
+        m = P.math.temporal_mean(X).cpu().numpy()
+        assert np.all(np.abs(m - np.float32(v)) <= EPS * v)
