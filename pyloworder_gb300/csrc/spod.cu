@@ -120,164 +120,179 @@ __global__ void __launch_bounds__(256) spod_fft_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// Fast path: FP32 data, nDFT = 32 E with E a power of two (1..32).  One warp
-// transforms one window in registers: lane l holds samples l + 32 e; an
-// E-point DIF FFT over its registers, twiddles w_N^(l k1), then a 32-point
-// DIF FFT across the lanes with shuffles.  Lane l, register r ends with bin
-// k1 + E k2, k1 = bitrev_E(r), k2 = bitrev_32(l).  Two real windows share one
-// complex transform (z = x_a + i x_b; X_a[f] = (Z[f] + conj Z[N-f]) / 2,
-// X_b[f] = (Z[f] - conj Z[N-f]) / 2i), which halves the FFT work.  A CTA owns
-// one point (all its Welch blocks); the pair spectra are staged in shared
-// memory in the register layout (one contiguous row per register across the
-// warp) and written per frequency as contiguous runs of nBlks values.
+// Fast path: FP32 data, nDFT = N = P L, a power of two from 32 to 1,024.  L lanes
+// transform one window pair in registers: lane l holds samples l + L e, does a
+// P-point DFT over them and the twiddles w_N^(l k1); the transposition through the
+// pair's shared row gives lane l all L values of k1 = l (+ L q), whose L-point DFT
+// is the bins k1 + P k2.  No stage crosses lanes: a 32-point FFT over the lanes by
+// shuffles took 80 shuffles and as many discarded halves of butterflies a pair, and
+// 5.4 ms at 262,144 points x 31 windows of 256 (3.2 ms with this; reading the points
+// once and writing the spectra takes 1.9).
+// Two real windows share one complex transform (z = x_a + i x_b;
+// X_a[f] = (Z[f] + conj Z[N-f]) / 2, X_b[f] = (Z[f] - conj Z[N-f]) / 2i).  A CTA owns
+// one point (all its Welch blocks); the pair spectra are staged in shared memory and
+// written per frequency as contiguous runs of nBlks values.
 // ---------------------------------------------------------------------------
-template <int E>
-__device__ __forceinline__ void warp_fft(float (&re)[E], float (&im)[E], int lane, int N,
-                                         const float* __restrict__ tc,
-                                         const float* __restrict__ ts) {
-  // E-point DIF over the registers (twiddle w_{2h}^j = w_N^{j N / 2h})
+// cos(2 pi k / 32)
+__device__ constexpr float spod_cos32(int k) {
+  constexpr float c[9] = {1.0f,        0.980785280f, 0.923879533f, 0.831469612f, 0.707106781f,
+                          0.555570233f, 0.382683432f, 0.195090322f, 0.0f};
+  return k <= 8 ? c[k] : -c[16 - k];
+}
+
+// DIF over the registers: register r ends with bin bitrev(r)
+template <int P>
+__device__ __forceinline__ void reg_dft(float (&re)[P], float (&im)[P]) {
 #pragma unroll
-  for (int h = E / 2; h >= 1; h >>= 1) {
+  for (int h = P / 2; h >= 1; h >>= 1) {
 #pragma unroll
-    for (int blk = 0; blk < E; blk += 2 * h) {
+    for (int blk = 0; blk < P; blk += 2 * h) {
 #pragma unroll
       for (int j = 0; j < h; ++j) {
+        const int k = j * (16 / h);  // w_{2h}^j = w_32^k
         const float ur = re[blk + j], ui = im[blk + j];
         const float vr = re[blk + j + h], vi = im[blk + j + h];
         re[blk + j] = ur + vr;
         im[blk + j] = ui + vi;
         const float dr = ur - vr, di = ui - vi;
-        const int ti = j * (N / (2 * h));
-        const float wr = tc[ti], wi = ts[ti];
-        re[blk + j + h] = dr * wr - di * wi;
-        im[blk + j + h] = dr * wi + di * wr;
-      }
-    }
-  }
-  // twiddles w_N^(l k1), k1 = bitrev_E(r)
-#pragma unroll
-  for (int r = 1; r < E; ++r) {
-    const int k1 = (int)(__brev((unsigned)r) >> (32 - __ffs(E) + 1));
-    const int ti = (lane * k1) & (N - 1);
-    const float wr = tc[ti], wi = ts[ti];
-    const float xr = re[r], xi = im[r];
-    re[r] = xr * wr - xi * wi;
-    im[r] = xr * wi + xi * wr;
-  }
-  // 32-point DIF across the lanes
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    const bool upper = (lane & d) != 0;
-    const int ti = (lane & (d - 1)) * (N / (2 * d));
-    const float wr = tc[ti], wi = ts[ti];
-#pragma unroll
-    for (int r = 0; r < E; ++r) {
-      const float pr = __shfl_xor_sync(0xffffffffu, re[r], d);
-      const float pi = __shfl_xor_sync(0xffffffffu, im[r], d);
-      if (!upper) {
-        re[r] += pr;
-        im[r] += pi;
-      } else {
-        const float dr = pr - re[r], di = pi - im[r];
-        re[r] = dr * wr - di * wi;
-        im[r] = dr * wi + di * wr;
+        if (k == 0) {
+          re[blk + j + h] = dr;
+          im[blk + j + h] = di;
+        } else if (k == 8) {
+          re[blk + j + h] = di;
+          im[blk + j + h] = -dr;
+        } else {
+          const float wr = spod_cos32(k), wi = -(k <= 8 ? spod_cos32(8 - k) : spod_cos32(k - 8));
+          re[blk + j + h] = dr * wr - di * wi;
+          im[blk + j + h] = dr * wi + di * wr;
+        }
       }
     }
   }
 }
+__host__ __device__ constexpr int spod_bitrev(int r, int n) {  // of log2(n) bits
+  int v = 0;
+  for (int b = 1; b < n; b <<= 1) v = 2 * v + ((r & b) ? 1 : 0);
+  return v;
+}
 
-template <int E>
-__global__ void __launch_bounds__(256) spod_fft32_kernel(
+template <int P, int L>
+__global__ void __launch_bounds__(256) spod_fft_reg_kernel(
     const float* __restrict__ Y, int64_t M, int64_t ldy, const float* __restrict__ mean, int step,
     int nBlks, int nf, const float* __restrict__ window, const float* __restrict__ twr,
     const float* __restrict__ twi, float scale, float* __restrict__ Q) {
-  constexpr int N = 32 * E;
-  extern __shared__ unsigned char smem_raw[];
-  float* sw = reinterpret_cast<float*>(smem_raw);  // window [N]
-  float* sc = sw + N;                              // cos    [N]
-  float* ss = sc + N;                              // -sin   [N]
-  // spectra of window pairs: [pair][N + 1] complex, bin f of a pair at slot
-  // r(f) 32 + lane(f) (the register layout of warp_fft)
-  float2* zs = reinterpret_cast<float2*>(ss + N);
+  constexpr int N = P * L, KQ = P / L, SUBS = 256 / L;
+  static_assert(P % L == 0 && P <= 32, "a lane owns P / L of the P-point bins");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* tw = reinterpret_cast<float2*>(smem_raw);  // e^(-2 pi i k / N) [N]
+  float* sw = reinterpret_cast<float*>(tw + N);      // window [N]
   constexpr int ZP = N + 1;  // odd pitch: consecutive pairs start 2 banks apart
+  float2* zs = reinterpret_cast<float2*>(sw + N);    // spectra of window pairs: [pair][ZP]
   const int npairs = (nBlks + 1) / 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l = lane % L, sub = tid / L;
   for (int j = tid; j < N; j += blockDim.x) {
     sw[j] = window[j];
-    sc[j] = twr[j];
-    ss[j] = twi[j];
+    tw[j] = make_float2(twr[j], twi[j]);
   }
   __syncthreads();
-  constexpr int LOGE = (E == 1) ? 0 : (E == 2) ? 1 : (E == 4) ? 2 : (E == 8) ? 3 : (E == 16) ? 4 : 5;
-  auto slot = [&](int f) -> int {  // f in [0, N)
-    const int k1 = f % E, k2 = f / E;
-    const int r = LOGE ? (int)(__brev((unsigned)k1) >> (32 - LOGE)) : 0;
-    return r * 32 + (int)(__brev((unsigned)k2) >> 27);
-  };
   for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {
     const float* x = Y + row * ldy;
     const float mu = mean ? mean[row] : 0.f;  // temporal mean removed on load
-    // two real windows per complex FFT: z = x_a + i x_b
-    for (int p = warp; p < npairs; p += 8) {
-      const float* xa = x + (int64_t)(2 * p) * step;
-      const bool has_b = 2 * p + 1 < nBlks;
-      const float* xb = xa + step;
-      float re[E], im[E];
+    for (int p0 = 0; p0 < npairs; p0 += SUBS) {
+      const int p = p0 + sub;
+      const bool live = p < npairs;
+      float2* z = zs + (size_t)(live ? p : 0) * ZP;
+      float re[P], im[P];
+      if (live) {
+        const float* xa = x + (int64_t)(2 * p) * step;
+        const bool has_b = 2 * p + 1 < nBlks;
+        const float* xb = has_b ? xa + step : xa;
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int j = lane + 32 * e;
-        re[e] = (__ldg(xa + j) - mu) * sw[j];
-        im[e] = has_b ? (__ldg(xb + j) - mu) * sw[j] : 0.f;
+        for (int e = 0; e < P; ++e) {
+          re[e] = __ldg(xa + l + L * e);
+          im[e] = __ldg(xb + l + L * e);
+        }
+#pragma unroll
+        for (int e = 0; e < P; ++e) {
+          const float w = sw[l + L * e];
+          re[e] = (re[e] - mu) * w;
+          im[e] = has_b ? (im[e] - mu) * w : 0.f;
+        }
+        reg_dft<P>(re, im);
+        // (columns of a row k1 swapped by k1: neither side of the transposition
+        // has bank conflicts)
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          const int k1 = spod_bitrev(r, P);
+          const float2 t = tw[l * k1];
+          z[k1 * L + (l ^ (k1 & (L - 1)))] =
+              make_float2(re[r] * t.x - im[r] * t.y, re[r] * t.y + im[r] * t.x);
+        }
       }
-      warp_fft<E>(re, im, lane, N, sc, ss);
-      float2* z = zs + (size_t)p * ZP;
+      __syncwarp();
+      if (live) {
 #pragma unroll
-      for (int r = 0; r < E; ++r) z[r * 32 + lane] = make_float2(re[r], im[r]);
+        for (int q = 0; q < KQ; ++q)
+#pragma unroll
+          for (int i = 0; i < L; ++i) {
+            const float2 v = z[(l + L * q) * L + (i ^ l)];
+            re[q * L + i] = v.x;
+            im[q * L + i] = v.y;
+          }
+      }
+      __syncwarp();
+      if (live) {
+#pragma unroll
+        for (int q = 0; q < KQ; ++q) {
+          float yr[L], yi[L];
+#pragma unroll
+          for (int i = 0; i < L; ++i) {
+            yr[i] = re[q * L + i];
+            yi[i] = im[q * L + i];
+          }
+          reg_dft<L>(yr, yi);
+#pragma unroll
+          for (int r = 0; r < L; ++r)
+            z[l + L * q + P * spod_bitrev(r, L)] = make_float2(yr[r], yi[r]);
+        }
+      }
     }
     __syncthreads();
-    // Q[f][row][b]: one contiguous run of nBlks values per frequency, a warp
-    // per frequency (its two spectrum slots and scale computed once), lanes
-    // along the blocks.
+    // Q[f][row][b]: one contiguous run of nBlks values per frequency, a warp per
+    // frequency, lanes along the blocks.
     // X_a[f] = (Z[f] + conj Z[N-f]) / 2,  X_b[f] = (Z[f] - conj Z[N-f]) / (2i)
-    c2<float>* Qc = reinterpret_cast<c2<float>*>(Q);
-    for (int f = warp; f < nf; f += 8) {
-      const int sk = slot(f), sn = slot((N - f) & (N - 1));
-      const float g = 0.5f * ((f >= 1 && f <= nf - 2) ? 2.f * scale : scale);
-      c2<float>* qrow = Qc + ((int64_t)f * M + row) * nBlks;
-      for (int b = lane; b < nBlks; b += 32) {
-        const float2* z = zs + (size_t)(b >> 1) * ZP;
-        const float2 zk = z[sk], zn = z[sn];
+    c2<float>* Qc = reinterpret_cast<c2<float>*>(Q) + row * nBlks;
+    for (int b = lane; b < nBlks; b += 32) {
+      const float2* z = zs + (size_t)(b >> 1) * ZP;
+      const bool odd = b & 1;
+#pragma unroll 4
+      for (int f = warp; f < nf; f += 8) {
+        const float g = 0.5f * ((f >= 1 && f <= nf - 2) ? 2.f * scale : scale);
+        const float2 zk = z[f], zn = z[(N - f) & (N - 1)];
         c2<float> v;
-        if ((b & 1) == 0) {
-          v.re = (zk.x + zn.x) * g;
-          v.im = (zk.y - zn.y) * g;
-        } else {
-          v.re = (zk.y + zn.y) * g;
-          v.im = (zn.x - zk.x) * g;
-        }
-        qrow[b] = v;
+        v.re = (odd ? zk.y + zn.y : zk.x + zn.x) * g;
+        v.im = (odd ? zn.x - zk.x : zk.y - zn.y) * g;
+        Qc[(int64_t)f * M * nBlks + b] = v;
       }
     }
     __syncthreads();
   }
 }
 
-template <int E>
-static int spod_fft32_launch(const float* Y, int64_t M, int64_t ldy, const float* mean, int step,
-                             int nBlks, int nf,
-                             const float* window, const float* twr, const float* twi, double scale,
-                             float* Q, cudaStream_t st) {
-  const size_t smem =
-      sizeof(float) * 3 * 32 * E + sizeof(float2) * (size_t)((nBlks + 1) / 2) * (32 * E + 1);
-  PLOM_CHECK_CUDA(cudaFuncSetAttribute(spod_fft32_kernel<E>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+template <int P, int L>
+static int spod_fft_reg_launch(const float* Y, int64_t M, int64_t ldy, const float* mean, int step,
+                               int nBlks, int nf, const float* window, const float* twr,
+                               const float* twi, double scale, float* Q, cudaStream_t st) {
+  constexpr int N = P * L;
+  const size_t smem = sizeof(float) * 3 * N + sizeof(float2) * (size_t)((nBlks + 1) / 2) * (N + 1);
+  const auto kern = spod_fft_reg_kernel<P, L>;
+  PLOM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  PLOM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spod_fft32_kernel<E>,
-                                                                256, smem));
+  PLOM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
   const int64_t grid = std::min<int64_t>(M, (int64_t)std::max(1, per_sm) * num_sms() * 8);
-  spod_fft32_kernel<E><<<(unsigned)grid, 256, smem, st>>>(Y, M, ldy, mean, step, nBlks, nf, window,
-                                                          twr,
-                                                          twi, (float)scale, Q);
+  kern<<<(unsigned)grid, 256, smem, st>>>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi,
+                                          (float)scale, Q);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
 }
@@ -300,12 +315,12 @@ static int spod_fft_impl(const T* Y, int64_t M, int64_t N, int64_t ldy, const T*
       ProfScope prof("spod_fft", st, 5.0 * (double)M * nBlks * nDFT * log2n,
                      (double)sizeof(T) * ((double)M * N + 2.0 * M * nBlks * nf));
       switch (log2n) {
-        case 5: return spod_fft32_launch<1>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
-        case 6: return spod_fft32_launch<2>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
-        case 7: return spod_fft32_launch<4>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
-        case 8: return spod_fft32_launch<8>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
-        case 9: return spod_fft32_launch<16>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
-        default: return spod_fft32_launch<32>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        case 5: return spod_fft_reg_launch<8, 4>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        case 6: return spod_fft_reg_launch<8, 8>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        case 7: return spod_fft_reg_launch<16, 8>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        case 8: return spod_fft_reg_launch<16, 16>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        case 9: return spod_fft_reg_launch<32, 16>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
+        default: return spod_fft_reg_launch<32, 32>(Y, M, ldy, mean, step, nBlks, nf, window, twr, twi, scale, Q, st);
       }
     }
   }
