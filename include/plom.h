@@ -250,6 +250,12 @@ int plom_spod_modes(int dtype, const void* U, int64_t G, int64_t M, int64_t nBlk
 int plom_spod_assemble(int dtype, const void* T, int64_t rows, int64_t nf, int64_t G,
                        int64_t gstride, const int* order, void* P, void* stream);
 
+/* modes and final column order in one pass: P[b*M + i][c] = Re U_f[i][b], f =
+   order[c], of the nf matrices U_f (M x nBlks complex, row-major, ustride
+   complex elements apart; dtype is the real type). */
+int plom_spod_gather(int dtype, const void* U, int64_t M, int64_t nBlks, int64_t nf,
+                     int64_t ustride, const int* order, void* P, void* stream);
+
 /* ---- packed tall operands (mixed form) --------------------------------- */
 /* No counterpart in the reference.  A caller that multiplies the same FP32
    matrix X (m x N, ldx) several times -- the streaming range finder uses one

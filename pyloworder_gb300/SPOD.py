@@ -19,7 +19,7 @@ from . import vmmath as M
 
 __all__ = ["run"]
 
-SVD_BATCH_MAX = 64  # frequencies per batched SVD
+SVD_BATCH_MAX = 152  # frequencies per batched SVD: one Jacobi CTA per SM
 
 
 def _window(name, n):
@@ -93,6 +93,23 @@ def run_device(x, ld, t_host, nDFT=0, nolap=0, remove_mean=True, window="hamming
     # the per-frequency SVDs run as batches of frequencies (one launch per
     # stage for the whole batch), as many per batch as device memory allows
     group = _svd_batch(Q, nBlks, precision)
+    if x.dtype == t.float32 and L.precision_code(precision, Q) == L.PREC_MIXED and Mrows < 2 ** 31:
+        # the mixed form reads its input once, to pack it: a batch's U takes the
+        # place of its Fourier coefficients, and one pass over all U writes the
+        # real parts in the final column order
+        group = -(-nf // -(-nf // group))
+        for f0 in range(0, nf, group):
+            f1 = min(nf, f0 + group)
+            _, S, _ = M.tsqr_svd_batched_device(Q[f0:f1], precision, U=Q[f0:f1])
+            Lm[f0:f1] = (S * S).to(x.dtype)
+            del S
+        order = np.argsort(Lm[:, 0].cpu().numpy())[::-1].copy()
+        od = t.as_tensor(order, device="cuda")
+        od32 = od.to(t.int32)
+        L.call("plom_spod_gather", L.dtype_code(P), L.ptr(Q), Mrows, nBlks, nf, rows, L.ptr(od32),
+               L.ptr(P), L.stream_ptr())
+        del Q
+        return Lm.index_select(0, od), P, f[order]
     # the mode-layout kernel stages group x nBlks real parts per point
     group = max(1, min(group, (48 * 1024) // (x.element_size() * (nBlks | 1))))
     # a batch's modes are written densely (rows x G_k, G_k frequencies per

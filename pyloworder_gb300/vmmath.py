@@ -222,18 +222,20 @@ def tsqr_svd_device(x, ld, precision=None, info_out=None):
     return U, S, V
 
 
-def tsqr_svd_batched_device(x3, precision=None, info_out=None):
+def tsqr_svd_batched_device(x3, precision=None, info_out=None, U=None):
     """TSQR-SVD of each matrix of a (batch, m, n) CUDA tensor (m >= n, unit
     inner stride, equal strides between matrices) -> U (batch, m, n), S
     (batch, n), V (batch, n, n) holding V^T.  The mixed form on float32 /
-    complex64 data runs every stage as one launch over the batch."""
+    complex64 data runs every stage as one launch over the batch.  U: a dense
+    tensor for the left vectors; in the mixed form it may be x3 itself."""
     t = L.torch()
     b, m, n = x3.shape
     if x3.stride(2) != 1 or (b > 1 and x3.stride(0) < m * x3.stride(1)):
         x3 = x3.contiguous()
     dt = L.dtype_code(x3)
     prec = L.precision_code(precision, x3)
-    U = t.empty((b, m, n), dtype=x3.dtype, device="cuda")
+    if U is None:
+        U = t.empty((b, m, n), dtype=x3.dtype, device="cuda")
     S = t.empty((b, n), dtype=L.real_dtype(x3), device="cuda")
     V = t.empty((b, n, n), dtype=x3.dtype, device="cuda")
     ws = L.workspace(L.load().plom_tsqr_svd_batched_workspace(dt, prec, b, m, n))

@@ -32,3 +32,23 @@ def test_fft(nDFT, nBlks, M):
         F = np.fft.fft(y * win, axis=1)[:, :nf] * 0.25
         F[:, 1:nf - 1] *= 2
         assert np.max(np.abs(Q[:, :, b].T - F)) < 1.2e-6 * np.abs(F).max()
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 9, 1500])
+@pytest.mark.parametrize("nBlks,nf", [(1, 1), (2, 2), (3, 17), (31, 31), (31, 32), (31, 33), (7, 129), (2, 4097), (70, 129)])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_gather(M, nBlks, nf, dt):
+    # a copy: every value exact, whole points and parts of one per tile
+    from pyloworder_gb300 import _lib as L
+    if M * nBlks * nf > 5e6:
+        pytest.skip("small cases")
+    rng = np.random.default_rng(M + nBlks)
+    pad = 3  # matrices need not be back to back
+    U = rng.standard_normal((nf, M * nBlks + pad, 2)).astype(dt)
+    order = rng.permutation(nf).astype(np.int32)
+    Ud, od = torch.from_numpy(U).cuda(), torch.from_numpy(order).cuda()
+    P = torch.zeros((M * nBlks, nf), dtype=Ud.dtype, device="cuda")
+    L.call("plom_spod_gather", L.dtype_code(P), L.ptr(Ud), M, nBlks, nf, M * nBlks + pad, L.ptr(od), L.ptr(P),
+           L.stream_ptr())
+    ex = U[order, :M * nBlks, 0].reshape(nf, M, nBlks).transpose(2, 1, 0).reshape(M * nBlks, nf)
+    assert np.array_equal(P.cpu().numpy(), ex)
