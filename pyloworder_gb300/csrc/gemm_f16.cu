@@ -236,19 +236,25 @@ __device__ __forceinline__ float2 ld_shared_h2f(uint32_t addr) {
 // shared memory and only one value per column and block goes to the global
 // maxima: with one per thread, narrow matrices were bound by the atomics on
 // their few addresses (2,097,152 x 64: 447 us, 80 us with this).
+// A dense matrix of any width is read in vectors: two or four rows of NC columns
+// make one row of N = 2 NC or 4 NC (column c is c mod NC), `tail` rows are left
+// (129 x 262,144 x 62: 2.5 ms one value at a time, 1.3 with this).
 __global__ void __launch_bounds__(256) colmax_kernel(const float* __restrict__ Y, int64_t ld,
-                                                     int64_t m, int N, int vec, int sh,
-                                                     int64_t bstride,
+                                                     int64_t m, int N, int NC, int tail, int vec,
+                                                     int sh, int64_t bstride,
                                                      unsigned* __restrict__ cmax) {
-  extern __shared__ unsigned cm_dyn[];  // N (sh; wider matrices go to the global maxima)
+  extern __shared__ unsigned cm_dyn[];  // NC (sh; wider matrices go to the global maxima)
   // problem blockIdx.y of a batch (matrices bstride elements apart)
   Y += (int64_t)blockIdx.y * bstride;
-  cmax += (int64_t)blockIdx.y * N;
+  cmax += (int64_t)blockIdx.y * NC;
   unsigned* cm_sh = sh ? cm_dyn : cmax;
   if (sh) {
-    for (int c = threadIdx.x; c < N; c += blockDim.x) cm_sh[c] = 0u;
+    for (int c = threadIdx.x; c < NC; c += blockDim.x) cm_sh[c] = 0u;
     __syncthreads();
   }
+  if (tail && blockIdx.x == 0)
+    for (int e = threadIdx.x; e < tail * NC; e += blockDim.x)
+      atomicMax(&cm_sh[e % NC], __float_as_uint(fabsf(Y[m * ld + e])));
   const int64_t rows = (m + gridDim.x - 1) / gridDim.x;
   const int64_t r0b = (int64_t)blockIdx.x * rows;
   const int64_t r1 = (r0b + rows < m) ? r0b + rows : m;
@@ -274,10 +280,10 @@ __global__ void __launch_bounds__(256) colmax_kernel(const float* __restrict__ Y
           mx.z = fmaxf(mx.z, fabsf(v.z));
           mx.w = fmaxf(mx.w, fabsf(v.w));
         }
-        atomicMax(&cm_sh[c], __float_as_uint(mx.x));
-        atomicMax(&cm_sh[c + 1], __float_as_uint(mx.y));
-        atomicMax(&cm_sh[c + 2], __float_as_uint(mx.z));
-        atomicMax(&cm_sh[c + 3], __float_as_uint(mx.w));
+        atomicMax(&cm_sh[c % NC], __float_as_uint(mx.x));
+        atomicMax(&cm_sh[(c + 1) % NC], __float_as_uint(mx.y));
+        atomicMax(&cm_sh[(c + 2) % NC], __float_as_uint(mx.z));
+        atomicMax(&cm_sh[(c + 3) % NC], __float_as_uint(mx.w));
       } else {  // one column, or the last columns of a row
         for (int q = c; q < (vec ? N : c + 1); ++q) {
           float mx = 0.f;
@@ -291,7 +297,7 @@ __global__ void __launch_bounds__(256) colmax_kernel(const float* __restrict__ Y
   }
   if (!sh) return;
   __syncthreads();
-  for (int c = threadIdx.x; c < N; c += blockDim.x)
+  for (int c = threadIdx.x; c < NC; c += blockDim.x)
     if (cm_sh[c]) atomicMax(&cmax[c], cm_sh[c]);
 }
 
@@ -2296,11 +2302,15 @@ int pack_f32(const float* Y, int64_t ld, int64_t m, int64_t N, Packed& p, Arena&
     const int rblocks = (int)std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>(m, cdiv(m * N, 8192)),
                              cdiv((int64_t)num_sms() * 8, batch)));
-    const int cvec = ((ld & 3) == 0) && ((bstride & 3) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(Y) & 15) == 0);
+    const bool al16 = (bstride & 3) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
     const int sh = N <= 8192;
+    // rows side by side so that a row is a whole number of vectors (dense matrices)
+    int64_t k = 1;
+    if (al16 && ld == N && (N & 3)) k = (N & 1) ? 4 : 2;
+    if (m < k) k = 1;
+    const int cvec = al16 && ((k * ld) & 3) == 0;
     hp::colmax_kernel<<<dim3(rblocks, (unsigned)batch), threads, sh ? sizeof(unsigned) * N : 0, st>>>(
-        Y, ld, m, (int)N, cvec, sh, bstride, cmax);
+        Y, k * ld, m / k, (int)(k * N), (int)N, (int)(m % k), cvec, sh, bstride, cmax);
     PLOM_CHECK_LAUNCH();
     hp::colscale_kernel<<<(int)std::min<int64_t>(cdiv(p.ld * batch, 256), 4096), 256, 0, st>>>(
         cmax, (int)N, (int)p.ld, (int)batch, p.scale);

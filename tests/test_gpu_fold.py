@@ -77,3 +77,22 @@ def test_long_products(m, n, r):
     s = P.vmmath.randomized_svd(A, r + 4, 1, seed=1)[1]
     s = torch.as_tensor(np.asarray(s.cpu() if hasattr(s, "cpu") else s)).double()[:r]
     assert float((s - S.cpu()).norm() / S.cpu().norm()) < 4e-6
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 127, 130, 4099])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 6, 30, 31, 61, 62, 129, 301])
+def test_column_scales(m, n):
+    # columns over 40 powers of ten, the largest element in any row (the last ones
+    # included): a missed maximum overflows its fp16 plane
+    import pyloworder_gb300 as P
+    rng = np.random.default_rng(m + n)
+    A = rng.standard_normal((m, n)) * 10.0 ** rng.uniform(-20, 15, n)
+    A[rng.integers(0, m, n), np.arange(n)] *= 1e4
+    A[-1] *= 3
+    A = A.astype(np.float32)
+    B = (rng.standard_normal((n, 7)) / np.abs(A).max(0)[:, None]).astype(np.float32)
+    C = P.math.matmul(A, B).astype(np.float64)
+    A64, B64 = A.astype(np.float64), B.astype(np.float64)
+    # 2^-22 of the column's largest element for the operands, the products' sums besides
+    tol = 2.0 ** -21 * (np.abs(A64).max(0)[None] @ np.abs(B64)) + 1e-6 * (np.abs(A64) @ np.abs(B64))
+    assert np.all(np.abs(C - A64 @ B64) <= tol)
