@@ -1931,7 +1931,7 @@ __global__ void __launch_bounds__(128) jacobi_pair_kernel(const double* __restri
 }
 
 // real matrices from this size on are solved through their transpose
-constexpr int JACOBI_TRANSPOSED_MIN_N = 64;
+constexpr int JACOBI_TRANSPOSED_MIN_N = 17;
 constexpr size_t JAC_BLOCK_SMEM_MAX = 200 * 1024;
 
 static int64_t jac_pitch(int n, int cplx) {
@@ -2653,8 +2653,50 @@ __global__ void ns_factor_kernel(double* __restrict__ G, int n) {
 
 // No floor (every pair is turned): columns left to the FP64 sweeps cost them three
 // more at n = 200 (7.4 ms instead of 4.2).
+// Double-float: 2 or 3 of its sweeps instead of 9, from 41 columns on (32: 260 us
+// without a start, 240 and 40 for the products with one; 64: 926, 537 + 40; 129: 2,954,
+// 1,611 + 45; 255: 6,301, 2,931 + 60) up to the form's own limit.
+constexpr int JAC_START_DF_MIN = 41, JAC_START_DF_MAX = 256;
 constexpr float JAC_START32_TOL = 2e-6f;    // as JAC_PRE32_TOL
 constexpr float JAC_START32_TSTOP = 3e-3f;  // as JAC_PRE32_TSTOP
+
+__global__ void start_df_kernel(const float* __restrict__ J32, double* __restrict__ J,
+                                double* __restrict__ Jt, int n) {
+  const int64_t nn = (int64_t)n * n;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nn;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const double v = (double)J32[e];
+    J[e] = v;
+    Jt[e % n * n + e / n] = v;
+  }
+}
+
+// The same for the double-float sweeps: one step (1e-10 beside their 1e-8), products
+// in double-float.
+static int jacobi_start_df(const double* A, const double* At, int n, unsigned long long* amax,
+                           float* J32, double* V, double* B, int* info, Arena& ws, cudaStream_t st) {
+  const size_t nn = (size_t)n * n;
+  const size_t mark = ws.off;
+  PLOM_TRY(jacobi_gram_f32(A, n, JAC_START32_TOL, JAC_PRE32_FLOOR, JAC_START32_TSTOP, J32, amax, info,
+                           ws, st));
+  const size_t need = ws.off;
+  ws.off = mark;
+  double* J = ws.take<double>(nn);
+  double* Jt = ws.take<double>(nn);
+  double* G = ws.take<double>(nn);
+  ws.off = std::max(ws.off, need);
+  if (ws.measuring()) return PLOM_OK;
+  PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
+  const int eg = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv((int64_t)nn, 256),
+                                                             (int64_t)num_sms() * 16));
+  start_df_kernel<<<eg, 256, 0, st>>>(J32, J, Jt, n);
+  PLOM_CHECK_LAUNCH();
+  PLOM_TRY(gemm_df_nn(Jt, J, G, n, 1, 0, st));
+  ns_factor_kernel<<<eg, 256, 0, st>>>(G, n);
+  PLOM_CHECK_LAUNCH();
+  PLOM_TRY(gemm_df_nn(J, G, V, n, 1, 0, st));
+  return gemm_df_nn(At, V, B, n, 1, 0, st);
+}
 
 // V (orthogonal, FP64) and B = At V; J32: n x n FP32 scratch (may be B)
 static int jacobi_start32(const double* A, const double* At, int n, unsigned long long* amax,
@@ -2699,25 +2741,36 @@ static int jacobi_svd_transposed(const double* A, int n, double tol, double* S, 
   double* At = ws.take<double>(nn);
   double* Ut = ws.take<double>(nn);
   double* VHt = ws.take<double>(nn);
-  const bool pre32 = use_pre32(n, tol);
-  const bool start32 = !pre32 && tol < JAC_DF_TOL && jacobi_gram_plan_ok(n);
+  const bool df = tol >= JAC_DF_TOL;
+  // FP32 sweeps first: for the FP64 sweeps, and for the double-float ones from
+  // JAC_START_DF_MIN columns on
+  const bool start32 = jacobi_gram_plan_ok(n) && (!df || (n >= JAC_START_DF_MIN && n <= JAC_START_DF_MAX));
+  const bool pre32 = use_pre32(n, tol) && !(start32 && jacobi_cta_usable(n, 0));
   JacState js;
   if (!pre32) carve_jac(ws, js, n, 1, 0);
-  double* V0 = start32 ? ws.take<double>(nn) : nullptr;
-  double* B = start32 ? ws.take<double>(nn) : nullptr;
+  double* V0 = start32 && !pre32 ? ws.take<double>(nn) : nullptr;
+  double* B = start32 && !pre32 ? ws.take<double>(nn) : nullptr;
   if (ws.measuring()) {
-    if (start32) PLOM_TRY(jacobi_start32(A, At, n, nullptr, nullptr, V0, B, info, ws, st));
+    if (start32 && !pre32)
+      PLOM_TRY(df ? jacobi_start_df(A, At, n, nullptr, nullptr, V0, B, info, ws, st)
+                  : jacobi_start32(A, At, n, nullptr, nullptr, V0, B, info, ws, st));
     return pre32 ? jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st) : PLOM_OK;
   }
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "jacobi: workspace too small");
   PLOM_REQUIRE(A && S && U && VH && info, PLOM_ERR_ARG, "jacobi: null pointer");
-  if (!pre32 && tol >= JAC_DF_TOL && jacobi_cta_usable(n, 0))
+  const bool cta = !pre32 && df && jacobi_cta_usable(n, 0);
+  const bool start = start32 && !pre32 && jacobi_gram_usable(n);
+  if (cta && !start)
     return jacobi_cta(A, n, 1, 0, 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U, VH, info, st);
   if (!pre32 || !jacobi_gram_usable(n)) PLOM_TRY(transpose_f64(A, At, n, n, 1, st));
   if (pre32) {
     PLOM_TRY(jacobi_pre32(A, At, n, tol, S, Ut, VHt, info, ws, st));
-  } else if (start32 && jacobi_gram_usable(n)) {
-    PLOM_TRY(jacobi_start32(A, At, n, js.amax, reinterpret_cast<float*>(B), V0, B, info, ws, st));
+  } else if (start) {
+    float* J32 = reinterpret_cast<float*>(B);
+    PLOM_TRY(df ? jacobi_start_df(A, At, n, js.amax, J32, V0, B, info, ws, st)
+                : jacobi_start32(A, At, n, js.amax, J32, V0, B, info, ws, st));
+    if (cta)
+      return jacobi_cta(B, n, 1, 0, 1, tol, js.At, js.Vt, js.nrm2, js.amax, S, U, VH, info, st, V0);
     js.V0 = V0;
     PLOM_TRY(jacobi_launch(B, n, 1, 0, js, tol, S, Ut, VHt, info, st));
   } else {

@@ -8,11 +8,10 @@
 // hundred columns are bound by that latency (32 columns: 84 steps, 1,039 us).
 // Here a round costs one CTA barrier: 32 lanes (or 8, 16) hold a column pair
 // in registers from the dot product to the rotation, and the rotation
-// parameters are derived by every lane, in FP32 or double-float arithmetic.
+// parameters are derived by every lane, in double-float arithmetic.
 // Measured, block kernels -> here (4,096-row inputs, to convergence): 32 real
 // columns 1,061 -> 260 us, 64 1,603 -> 953, 128 4,413 -> 1,943; 64 complex
-// problems of 31 columns 3,127 -> 711 us, of 63 12,073 -> 3,590; FP32 sweeps of
-// 301 columns 5,812 -> 4,470.  What bounds it: a round's chain of dependent
+// problems of 31 columns 3,127 -> 711 us, of 63 12,073 -> 3,590.  What bounds it: a round's chain of dependent
 // instructions (1,700 cycles with one warp per scheduler, double-float), from 48
 // columns on the issue rate of one SM, and in a cluster the exchange (8,000 to
 // 11,000 cycles a step).
@@ -26,10 +25,8 @@
 //    move one place round the circle (each CTA reads the ones it needs from
 //    its neighbours' shared memory).
 //
-// Arithmetic: FP32 (c, s) rotations (the pre-sweeps of the refined form), or
-// double-float rows with scaled rotations (column = d x stored row,
-// x' = x - t (dq/dp) e^{-i phi} y, y' = y + t (dp/dq) e^{i phi} x, d' = c d), or
-// the same on FP64 rows.
+// Arithmetic: double-float rows with scaled rotations (column = d x stored row,
+// x' = x - t (dq/dp) e^{-i phi} y, y' = y + t (dp/dq) e^{i phi} x, d' = c d).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -48,38 +45,9 @@ constexpr int JC_MAX_SWEEPS = 40;
 constexpr float JC_FOLD = 9.094947017729282e-13f;  // 2^-40: a smaller scale goes into its row
 
 // ---------------------------------------------------------------------------
-// arithmetic of a column pair.  Rows are vectors of 16 bytes (V): 4 FP32, 2
-// double-float or 2 FP64 values, or 1 complex double-float value.
+// arithmetic of a column pair.  Rows are vectors of 16 bytes (V): 2 double-float
+// values or 1 complex one.
 // ---------------------------------------------------------------------------
-struct ArF32 {
-  using V = float4;
-  using S = float;  // squared norm; < 0: recompute
-  static constexpr int PER = 4;
-  struct Dot { float g, a, b; };
-  struct Rot { float c, s; bool on; float t; };
-  __device__ static V zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ static void clear(Dot& d) { d.g = d.a = d.b = 0.f; }
-  __device__ static void dot(Dot& d, V x, V y) {
-    d.g = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, d.g))));
-  }
-  __device__ static void sq(float& s, V x) {
-    s = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, s))));
-  }
-  template <int L>
-  __device__ static float sum(float v) {
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-  }
-  __device__ static void rotate(V& x, V& y, const Rot& r) {
-    const V a = x, b = y;
-    x = make_float4(fmaf(r.c, a.x, -r.s * b.x), fmaf(r.c, a.y, -r.s * b.y),
-                    fmaf(r.c, a.z, -r.s * b.z), fmaf(r.c, a.w, -r.s * b.w));
-    y = make_float4(fmaf(r.s, a.x, r.c * b.x), fmaf(r.s, a.y, r.c * b.y),
-                    fmaf(r.s, a.z, r.c * b.z), fmaf(r.s, a.w, r.c * b.w));
-  }
-};
-
 // double-float state of a column: squared norm (x < 0: recompute), scale and
 // its inverse
 struct DfState { float2 nrm, d, e; };
@@ -255,10 +223,8 @@ struct JacCtaArgs {
   int rows;          // columns held by a CTA (rows of its A^T and V)
   float tol;
   int trans;         // rotate the rows of A instead of its columns (real)
-  // refined form (FP32): J (n x n row-major) and the stop criterion
-  float* J;
-  float floor, tstop;
-  // otherwise the rotated columns, V and their norms, for jacobi_out_kernel
+  const double* V0;  // n x n starting rotation product (real; null: the identity)
+  // the rotated columns, V and their norms, for jacobi_out_kernel
   double *At, *Vt, *nrm2;
   unsigned long long* amax;  // [batch]
   int* info;
@@ -276,16 +242,13 @@ template <typename Ar, int L, int Q, int T>
 __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
   using V = typename Ar::V;
   using S = typename Ar::S;
-  constexpr bool F32 = std::is_same<Ar, ArF32>::value;
   constexpr int CW = std::is_same<Ar, ArDfC>::value ? 2 : 1;
   constexpr int PV = L * Q;          // vectors per row
   constexpr int GROUPS = T / L;      // column pairs in flight
   extern __shared__ __align__(16) unsigned char jc_smem[];
   __shared__ unsigned long long mx_sh[16];
   __shared__ int cnt_sh[2][16];
-  __shared__ float tmax_sh[2][16], cmax_sh[2][16];
   __shared__ int rot_sh, src_sh[2];
-  __shared__ float tm_sh, cm_sh;
   cg::cluster_group cl = cg::this_cluster();
   const int n = p.n, C = p.C, bs = p.bs, nblk = p.nblk, steps = nblk - 1;
   const int rank = C > 1 ? (int)cl.block_rank() : 0;
@@ -303,10 +266,7 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
   // ---- power-of-two scale: max |a| < 1
   {
     if (tid < 16) mx_sh[tid] = 0ull;
-    if (tid == 0) {
-      rot_sh = 0;
-      tm_sh = cm_sh = 0.f;
-    }
+    if (tid == 0) rot_sh = 0;
     __syncthreads();
     unsigned long long mx = 0ull;
     for (int64_t e = (int64_t)rank * T + tid; e < (int64_t)n * n * CW; e += (int64_t)C * T) {
@@ -346,14 +306,17 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
         const int i = v * Ar::PER + u;
         if (i >= n) continue;
         const int64_t src = p.trans ? (int64_t)col * n + i : (int64_t)i * n + col;
-        if constexpr (F32) {
-          af[u] = (float)ldexp(A[src], -ex);
-          qf[u] = i == col ? 1.f : 0.f;
-        } else if constexpr (CW == 1) {
+        if constexpr (CW == 1) {
           const float2 s = df_split(ldexp(A[src], -ex));
           af[2 * u] = s.x;
           af[2 * u + 1] = s.y;
-          qf[2 * u] = i == col ? 1.f : 0.f;
+          if (p.V0) {
+            const float2 v0 = df_split(p.V0[(int64_t)i * n + col]);
+            qf[2 * u] = v0.x;
+            qf[2 * u + 1] = v0.y;
+          } else {
+            qf[2 * u] = i == col ? 1.f : 0.f;
+          }
         } else {
           const float2 re = df_split(ldexp(A[2 * src], -ex));
           const float2 im = df_split(ldexp(A[2 * src + 1], -ex));
@@ -365,11 +328,9 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
     cA[e] = a;
     cV[e] = q;
   }
-  if constexpr (!F32) {
-    for (int r = tid; r < p.rows; r += T) {
-      st[r].d = st[r].e = make_float2(1.f, 0.f);
-      st[r].nrm = make_float2(-1.f, 0.f);
-    }
+  for (int r = tid; r < p.rows; r += T) {
+    st[r].d = st[r].e = make_float2(1.f, 0.f);
+    st[r].nrm = make_float2(-1.f, 0.f);
   }
   __syncthreads();
 
@@ -378,31 +339,17 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
     for (int r0 = 0; r0 < p.rows; r0 += GROUPS) {  // uniform trip count: warp shuffles inside
       const int r = r0 + grp;
       const V* x = cA + (size_t)(r < p.rows ? r : 0) * PV;
-      if constexpr (F32) {
-        float s = 0.f;
+      float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) Ar::sq(s, x[l + q * L]);
-        s = Ar::template sum<L>(s);
-        if (l == 0 && r < p.rows) {
-          st[r] = s;
-          atomicMax(reinterpret_cast<int*>(&cm_sh), __float_as_int(s));
-        }
-      } else {
-        float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) Ar::sq(s, x[l + q * L]);
-        s = df_lane_sum<L>(s);
-        if (l == 0 && r < p.rows) st[r].nrm = df_mul(df_mul(st[r].d, st[r].d), s);
-      }
+      for (int q = 0; q < Q; ++q) Ar::sq(s, x[l + q * L]);
+      s = df_lane_sum<L>(s);
+      if (l == 0 && r < p.rows) st[r].nrm = df_mul(df_mul(st[r].d, st[r].d), s);
     }
   };
 
-  float cmax_prev = 0.f;
   int sweep = 0;
   for (; sweep < p.max_sweeps; ++sweep) {
     int myrot = 0;
-    float mytmax = 0.f;
-    const float floor2 = (F32 && sweep > 0) ? p.floor * p.floor * cmax_prev : 3.0e38f;
     for (int step = 0; step < steps; ++step) {
       if (C > 1 && (sweep > 0 || step > 0)) {
         // ---- the blocks of this step from the CTAs that held them
@@ -508,7 +455,7 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
           S sp = st[ra], sq = st[rc];
           V* xv = cV + (size_t)ra * PV + l;
           V* yv = cV + (size_t)rc * PV + l;
-          if constexpr (!F32) {
+          {
             // a scale below 2^-40 goes into its row first (rare)
             const bool fa = live && sp.d.x < JC_FOLD, fb = live && sq.d.x < JC_FOLD;
             if (fa || fb) {
@@ -532,35 +479,7 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
 #pragma unroll
           for (int q = 0; q < Q; ++q) Ar::dot(dt, x[q], y[q]);
           typename Ar::Rot r;
-          if constexpr (F32) {
-            const bool need = live && (sp < 0.f || sq < 0.f);
-            if (__any_sync(0xffffffffu, need)) {
-              float a2 = 0.f, b2 = 0.f;
-#pragma unroll
-              for (int q = 0; q < Q; ++q) {
-                Ar::sq(a2, x[q]);
-                Ar::sq(b2, y[q]);
-              }
-              a2 = Ar::template sum<L>(a2);
-              b2 = Ar::template sum<L>(b2);
-              if (sp < 0.f) sp = a2;
-              if (sq < 0.f) sq = b2;
-            }
-            const float g = Ar::template sum<L>(dt.g);
-            const float big = fmaxf(sp, sq);
-            r.on = live && jc_above(sp, sq, fabsf(g), p.tol);
-            if (r.on) {
-              const float t = jc_tan(sq - sp, g);
-              // c and s = c t to FP32 accuracy (an estimate and one Newton step)
-              const float w = fmaf(t, t, 1.0f), c0 = rsqrtf(w);
-              r.c = fmaf(0.5f * c0, fmaf(-w * c0, c0, 1.0f), c0);
-              r.s = r.c * t;
-              const float na = sp - t * g, nb = sq + t * g;
-              sp = na > 0.125f * sp ? na : -1.f;
-              sq = nb > 0.125f * sq ? nb : -1.f;
-              if (big > floor2) mytmax = fmaxf(mytmax, fabsf(t));
-            }
-          } else {
+          {
             const bool need = live && (sp.nrm.x < 0.f || sq.nrm.x < 0.f);
             if (__any_sync(0xffffffffu, need)) {
               float2 a2 = make_float2(0.f, 0.f), b2 = a2;
@@ -601,79 +520,50 @@ __global__ void __launch_bounds__(T, 1) jacobi_cta_kernel(const JacCtaArgs p) {
     // ---- rotations of the sweep over the problem
     if (l == 0) {
       if (myrot) atomicAdd(&rot_sh, myrot);
-      if (F32 && mytmax > 0.f) atomicMax(reinterpret_cast<int*>(&tm_sh), __float_as_int(mytmax));
     }
     __syncthreads();
     const int par = sweep & 1;
     if (tid < C) {
       int* dc = C > 1 ? cl.map_shared_rank(&cnt_sh[par][rank], tid) : &cnt_sh[par][0];
       *dc = rot_sh;
-      if (F32) {
-        float* dtm = C > 1 ? cl.map_shared_rank(&tmax_sh[par][rank], tid) : &tmax_sh[par][0];
-        float* dcm = C > 1 ? cl.map_shared_rank(&cmax_sh[par][rank], tid) : &cmax_sh[par][0];
-        *dtm = tm_sh;
-        *dcm = cm_sh;
-      }
     }
     if (C > 1) cl.sync();
     else __syncthreads();
     int total = 0;
-    float tmax = 0.f, cmax = 0.f;
-    for (int r = 0; r < C; ++r) {
-      total += cnt_sh[par][r];
-      if (F32) {
-        tmax = fmaxf(tmax, tmax_sh[par][r]);
-        cmax = fmaxf(cmax, cmax_sh[par][r]);
-      }
-    }
-    cmax_prev = cmax;
+    for (int r = 0; r < C; ++r) total += cnt_sh[par][r];
     __syncthreads();
-    if (tid == 0) {
-      rot_sh = 0;
-      tm_sh = cm_sh = 0.f;
-    }
+    if (tid == 0) rot_sh = 0;
     __syncthreads();
     if (total == 0) break;
-    if (F32 && sweep > 0 && tmax <= p.tstop) break;
   }
 
   // ---- out (the CTA holds the blocks of the last step)
   if (tid == 0 && rank == 0) {
-    if (F32) {
-      p.info[ST_SWEEPS32] = sweep < p.max_sweeps ? sweep + 1 : sweep;
-    } else {
-      atomicMax(&p.info[ST_SWEEPS], sweep + 1);
-      if (sweep >= p.max_sweeps) atomicMax(&p.info[ST_FAIL], PLOM_NUM_JACOBI);
-    }
+    atomicMax(&p.info[ST_SWEEPS], sweep + 1);
+    if (sweep >= p.max_sweeps) atomicMax(&p.info[ST_FAIL], PLOM_NUM_JACOBI);
   }
-  if constexpr (!F32) {
-    norms();
-    __syncthreads();
-  }
+  norms();
+  __syncthreads();
   const int len = n * CW;
   for (int e = tid; e < p.rows * len; e += T) {
     const int r = e / len, i = e % len;
     const int col = C > 1 ? jc_block(steps - 1, rank, nblk, r / bs) * bs + r % bs : r;
     if (col >= n) continue;
-    if constexpr (F32) {
-      p.J[(int64_t)i * n + col] = reinterpret_cast<const float*>(cV + (size_t)r * PV)[i];
-    } else {
-      const double d = df_val(st[r].d);
-      const float2* a = reinterpret_cast<const float2*>(cA + (size_t)r * PV);
-      const float2* v = reinterpret_cast<const float2*>(cV + (size_t)r * PV);
-      p.At[((int64_t)prob * n + col) * len + i] = df_val(a[i]) * d;
-      p.Vt[((int64_t)prob * n + col) * len + i] = df_val(v[i]) * d;
-      if (i == 0) {
-        double s = df_val(st[r].nrm);
-        if (!(st[r].nrm.x > 1e-28f)) {  // near the end of the FP32 range: in FP64
-          s = 0.0;
-          for (int k = 0; k < len; ++k) {
-            const double x = df_val(a[k]) * d;
-            s = fma(x, x, s);
-          }
+    const double d = df_val(st[r].d);
+    const float2* a = reinterpret_cast<const float2*>(cA + (size_t)r * PV);
+    const float2* v = reinterpret_cast<const float2*>(cV + (size_t)r * PV);
+    p.At[((int64_t)prob * n + col) * len + i] = df_val(a[i]) * d;
+    p.Vt[((int64_t)prob * n + col) * len + i] = df_val(v[i]) * d;
+    if (i == 0) {
+      double s = df_val(st[r].nrm);
+      if (!(st[r].nrm.x > 1e-28f)) {  // near the end of the FP32 range: in FP64
+        s = 0.0;
+        for (int k = 0; k < len; ++k) {
+          const double x = df_val(a[k]) * d;
+          s = fma(x, x, s);
         }
-        p.nrm2[(int64_t)prob * n + col] = s;
       }
+      p.nrm2[(int64_t)prob * n + col] = s;
     }
   }
   if (C > 1) cl.sync();  // no CTA leaves while a neighbour may read it
@@ -873,7 +763,7 @@ bool jacobi_cta_usable(int n, int cplx) {
 
 int jacobi_cta(const double* A, int n, int batch, int cplx, int trans, double tol, double* At,
                double* Vt, double* nrm2, unsigned long long* amax, double* S, double* U,
-               double* VH, int* info, cudaStream_t st) {
+               double* VH, int* info, cudaStream_t st, const double* V0) {
   JcPlan pl;
   PLOM_REQUIRE(jc_plan(pl, n, cplx), PLOM_ERR_UNSUPPORTED, "jacobi: %d columns", n);
   JacCtaArgs a = {};
@@ -884,7 +774,8 @@ int jacobi_cta(const double* A, int n, int batch, int cplx, int trans, double to
   a.nblk = pl.nblk;
   a.rows = pl.rows;
   a.tol = (float)tol;
-  a.trans = trans;
+  a.trans = V0 ? 0 : trans;  // (from V0: A holds the rotated columns)
+  a.V0 = V0;
   a.At = At;
   a.Vt = Vt;
   a.nrm2 = nrm2;

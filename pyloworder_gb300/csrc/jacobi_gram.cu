@@ -453,16 +453,17 @@ __device__ __forceinline__ bool jg_wait(uint32_t bar, uint32_t parity) {
 // before has landed, so the buffers sent from may be written again.
 template <int TB>
 __global__ void __launch_bounds__(JG_THREADS, 1) jacobi_gram_cluster_kernel(const JgArgs p) {
-  constexpr int B = TB / 2, C = JG_CLUSTER, steps = 2 * C - 1;
+  constexpr int B = TB / 2;
+  const int C = p.nblk / 2, steps = p.nblk - 1;
   extern __shared__ __align__(128) float jg_sm[];  // two buffers of two regions
   __shared__ __align__(16) float Jt[TB][TB];
   __shared__ __align__(16) float Jn[TB][TB];
   __shared__ float G[TB][TB + 1];
   __shared__ float part[JG_THREADS / 32 * 16];
   __shared__ float2 cs[B];
-  __shared__ unsigned long long mx_sh[C];
-  __shared__ int cnt_sh[2][C];
-  __shared__ float tm_sh[2][C], cm_sh[2][C];
+  __shared__ unsigned long long mx_sh[JG_CLUSTER];
+  __shared__ int cnt_sh[2][JG_CLUSTER];
+  __shared__ float tm_sh[2][JG_CLUSTER], cm_sh[2][JG_CLUSTER];
   __shared__ int dst_sh[2], abort_sh;
   __shared__ __align__(8) uint64_t bar;
   cg::cluster_group cl = cg::this_cluster();
@@ -856,15 +857,21 @@ static void jg_kernels(JgPlan& pl) {
   pl.rows = (const void*)jacobi_rows_kernel<TB>;
 }
 
-// Up to 512 columns the 16 CTAs of a cluster hold all of them (32 columns of 512
-// values twice, 131 KiB); beyond, 8-column blocks with one CTA per pair.
+// Up to 512 columns the CTAs of a cluster hold all of them (32 columns of 512 values
+// twice, 131 KiB); beyond, 8-column blocks with one CTA per pair.  As few CTAs as
+// hold 32 columns each: a step costs 2,700 cycles of exchange and the latency of its
+// rounds whatever its columns, and 2 C - 1 steps make a sweep (64 columns, with the
+// double-float finish: 537 us on 2 CTAs, 773 on 8, 1,195 on 16; 129: 1,610 on 8, 2,072
+// on 16); from 225 columns 16 CTAs (255: 3,097 us on 8, 2,931 on 16).
 static bool jg_plan(JgPlan& pl, int n) {
   if (n < 1 || n > 1600) return false;
   pl.pitch = (int)(cdiv(n, 16) * 16);
   pl.cluster = n <= 512;
   if (pl.cluster) {
-    pl.nblk = 2 * JG_CLUSTER;
-    switch ((int)std::max<int64_t>(2, cdiv(n, 64))) {
+    int C = n <= 224 ? 1 : JG_CLUSTER;
+    while (n > 32 * C) C *= 2;
+    pl.nblk = 2 * C;
+    switch ((int)std::max<int64_t>(2, cdiv(n, 4 * C))) {
       case 2: jg_kernels<8>(pl); break;
       case 3: jg_kernels<12>(pl); break;
       case 4: jg_kernels<16>(pl); break;
@@ -911,9 +918,9 @@ bool jacobi_gram_usable(int n) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = JG_CLUSTER;
+      at[0].val.clusterDim.x = (unsigned)(pl.nblk / 2);
       at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3(JG_CLUSTER);
+      cfg.gridDim = dim3((unsigned)(pl.nblk / 2));
       cfg.blockDim = dim3(JG_THREADS);
       cfg.dynamicSmemBytes = pl.smem;
       cfg.attrs = at;
@@ -966,9 +973,9 @@ int jacobi_gram_f32(const double* A, int n, float tol, float floor_rel, float ts
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = JG_CLUSTER;
+    at[0].val.clusterDim.x = (unsigned)(pl.nblk / 2);
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(JG_CLUSTER);
+    cfg.gridDim = dim3((unsigned)(pl.nblk / 2));
     cfg.blockDim = dim3(JG_THREADS);
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = st;

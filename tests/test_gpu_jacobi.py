@@ -101,3 +101,22 @@ def test_fp64_from_fp32_start(n, kind):
     assert np.max(np.abs(V @ V.T - np.eye(n))) < tol
     assert np.linalg.norm((U * S) @ V - A) < tol * np.linalg.norm(A)
     assert np.max(np.abs(S - np.linalg.svd(A, compute_uv=False))) < tol * S[0]
+
+
+@pytest.mark.parametrize("n", [17, 18, 24, 31, 32, 33, 40, 41, 47, 63, 127, 224, 225, 254])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_started_sweeps(n, dt):
+    # sizes around the FP32 start's clusters of 1, 2, 4, 8 and 16 CTAs and its first
+    # and last size in either precision
+    import pyloworder_gb300 as P
+    A = field(2 * n + 130, n, 4000 + n).astype(dt)
+    U, S, V = (x.cpu().numpy().astype(np.float64) for x in P.math.tsqr_svd(torch.from_numpy(A).cuda()))
+    A = A.astype(np.float64)
+    if dt == np.float32:
+        check(A, U, S, V)
+        return
+    tol = 10 * n * 2.3e-16  # its own tolerance is n eps a pair
+    assert np.max(np.abs(U.T @ U - np.eye(n))) < tol
+    assert np.max(np.abs(V @ V.T - np.eye(n))) < tol
+    assert np.linalg.norm((U * S) @ V - A) < tol * np.linalg.norm(A)
+    assert np.max(np.abs(S - np.linalg.svd(A, compute_uv=False))) < tol * S[0]
