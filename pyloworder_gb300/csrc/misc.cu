@@ -347,6 +347,44 @@ __global__ void __launch_bounds__(256) hh_update_kernel(float* __restrict__ A, i
   }
 }
 
+// the whole elimination of a matrix that fits shared memory, one barrier a column:
+// a warp takes rows, its lanes their columns.  96 columns: 304 us as three panels and
+// their updates (a chain of global reads per column), 78 us here.
+constexpr int HH_SMALL = 200;
+template <typename T>
+__global__ void __launch_bounds__(1024) hh_small_kernel(const T* __restrict__ Q, int64_t ldq, int n,
+                                                       int square, double* __restrict__ s) {
+  extern __shared__ float hh_sm[];
+  const int pitch = n | 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < n * n; e += 1024)
+    hh_sm[e / n * pitch + e % n] = (float)Q[(int64_t)(e / n) * ldq + e % n];
+  __syncthreads();
+  for (int k = 0; k < n; ++k) {
+    const float* Ak = hh_sm + k * pitch;
+    const float p = Ak[k];
+    const bool last_sq = square && k == n - 1;
+    const float sk = (p >= 0.f) != last_sq ? -1.f : 1.f;
+    const float piv = p - sk;
+    if (threadIdx.x == 0) s[k] = (double)sk;
+    const float rp = 1.f / piv;
+    for (int i = k + 1 + warp; i < n; i += 128) {  // four rows of the warp in flight
+      float l[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) l[u] = i + 32 * u < n ? hh_sm[(i + 32 * u) * pitch + k] * rp : 0.f;
+      for (int j = k + 1 + lane; j < n; j += 32) {
+        const float a = Ak[j];
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i + 32 * u < n ? hh_sm[(i + 32 * u) * pitch + j] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i + 32 * u < n) hh_sm[(i + 32 * u) * pitch + j] = fmaf(-l[u], a, v[u]);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // W (n x n, ld n) <- W diag(s), R (n x n, ld n) <- diag(s) R
 __global__ void sign_fold_kernel(double* __restrict__ W, double* __restrict__ R,
                                  const double* __restrict__ s, int n) {
@@ -367,7 +405,15 @@ int householder_signs(const T* Qtop, int64_t ldq, int n, bool square, double* s,
   PLOM_REQUIRE(!ws.overflow(), PLOM_ERR_WORKSPACE, "householder signs: workspace too small");
   PLOM_REQUIRE(Qtop && s && n >= 1 && ldq >= n, PLOM_ERR_ARG, "householder signs: bad arguments");
   ProfScope prof("hh_signs", st, 2.0 * n * (double)n * n / 3.0, 8.0 * n * (double)n,
-                 1 + 2 * (int)cdiv(n, HH_BW));
+                 n <= HH_SMALL ? 1 : 1 + 2 * (int)cdiv(n, HH_BW));
+  if (n <= HH_SMALL) {
+    const size_t smem = sizeof(float) * (size_t)n * (n | 1);
+    PLOM_CHECK_CUDA(cudaFuncSetAttribute(hh_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(sizeof(float) * HH_SMALL * (HH_SMALL + 1))));
+    hh_small_kernel<T><<<1, 1024, smem, st>>>(Qtop, ldq, n, square ? 1 : 0, s);
+    PLOM_CHECK_LAUNCH();
+    return PLOM_OK;
+  }
   hh_load_kernel<T><<<grid1d((int64_t)n * n), 256, 0, st>>>(Qtop, ldq, n, A);
   PLOM_CHECK_LAUNCH();
   for (int k0 = 0; k0 < n; k0 += HH_BW) {
