@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <type_traits>
 
 namespace plom {
 
@@ -430,73 +431,96 @@ template int gemm_tn_in_scratch<double, double, double>(const double*, int64_t, 
 // 1/64 of its FP32 rate).  Row-chunk partials are summed in FP64 in a fixed
 // order.  Used where a reduction over the points must be FP64-accurate (DMD's
 // projection onto span(U_r)).
-// 128 threads as 8 x 16, 4 x 8 outputs each (rows ty*4.., columns tx*4.. and
-// 64 + tx*4..), operands from shared memory as 16-byte vectors, the next
-// 32-row tile prefetched into registers while the current one is summed.
+// 128 threads: 8 x 16 with 4 x 8 outputs each, or, for tall operands and results wider
+// than 128 columns, 4 x 32 with 8 x 8.  A 16-byte read of shared memory costs four cycles of the SM's
+// return path: 4 x 8 reads 3 vectors for 32 FMAs (12 cycles for the 8 that the SM needs
+// to issue them), 8 x 8 reads 4 for 64.  The next 32-row tiles arrive by asynchronous
+// copies (zero-filled at the edges) while the current ones are summed.
 // ----------------------------------------------------------------------------
-constexpr int DF_BM = 32, DF_BN = 128, DF_BK = 32, DF_THREADS = 128;
+constexpr int DF_BM = 32, DF_BK = 32, DF_THREADS = 128;
 
+template <int TM, int TX>
 __global__ void __launch_bounds__(DF_THREADS) gemm_tn_df_kernel(const float* __restrict__ A,
                                                                 int64_t lda,
                                                                 const float* __restrict__ B,
                                                                 int64_t ldb,
                                                                 double* __restrict__ part,
                                                                 int64_t M, int64_t N, int64_t K,
-                                                                int64_t kchunk, int64_t tm) {
-  constexpr int TM = 4, TN = 8;
-  constexpr int LA = DF_BK * DF_BM / DF_THREADS, LB = DF_BK * DF_BN / DF_THREADS;
-  static_assert(DF_BM == 8 * TM && DF_BN == 16 * TN, "tile / thread layout");
-  __shared__ __align__(16) float As[DF_BK][DF_BM];
-  __shared__ __align__(16) float Bs[DF_BK][DF_BN];
-  const int64_t i0 = (int64_t)(blockIdx.x % tm) * DF_BM, j0 = (int64_t)(blockIdx.x / tm) * DF_BN;
+                                                                int64_t kchunk, int64_t tm, int va,
+                                                                int vb) {
+  constexpr int TN = 8, BN = TX * TN, HB = BN / 2;
+  static_assert(DF_BM / TM * TX == DF_THREADS, "tile / thread layout");
+  extern __shared__ __align__(16) float df_sm[];  // two buffers of [BK][BM], [BK][BN]
+  constexpr int BUF = DF_BK * (DF_BM + BN);
+  const int64_t i0 = (int64_t)(blockIdx.x % tm) * DF_BM, j0 = (int64_t)(blockIdx.x / tm) * BN;
   const int64_t kbeg = (int64_t)blockIdx.y * kchunk;
   const int64_t kend = min(K, kbeg + kchunk);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   float hi[TM][TN], lo[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) hi[i][j] = lo[i][j] = 0.f;
-  float ra[LA], rb[LB];
-  auto load = [&](int64_t k0) {
+  // a [BK][W] tile at rows k0.., columns c0.. of X (n columns) into dst
+  auto tile = [&](auto width, const float* X, int64_t ld, int64_t n, int64_t c0, int64_t k0, int vec,
+                  float* dst) {
+    constexpr int W = decltype(width)::value;
+    if (vec) {
 #pragma unroll
-    for (int q = 0; q < LA; ++q) {
-      const int e = threadIdx.x + q * DF_THREADS;
-      const int64_t gk = k0 + e / DF_BM, gi = i0 + e % DF_BM;
-      ra[q] = (gk < kend && gi < M) ? A[gk * lda + gi] : 0.f;
-    }
-#pragma unroll
-    for (int q = 0; q < LB; ++q) {
-      const int e = threadIdx.x + q * DF_THREADS;
-      const int64_t gk = k0 + e / DF_BN, gj = j0 + e % DF_BN;
-      rb[q] = (gk < kend && gj < N) ? B[gk * ldb + gj] : 0.f;
+      for (int q = 0; q < DF_BK * W / 4 / DF_THREADS; ++q) {
+        const int e = (threadIdx.x + q * DF_THREADS) * 4;
+        const int64_t gk = k0 + e / W, gc = c0 + e % W;
+        const int left = gk < kend ? (int)min((int64_t)4, max((int64_t)0, n - gc)) : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst + e)),
+                     "l"(left ? X + gk * ld + gc : X), "r"(4 * left));
+      }
+    } else {
+#pragma unroll 8
+      for (int q = 0; q < DF_BK * W / DF_THREADS; ++q) {
+        const int e = threadIdx.x + q * DF_THREADS;
+        const int64_t gk = k0 + e / W, gc = c0 + e % W;
+        const bool in = gk < kend && gc < n;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst + e)),
+                     "l"(in ? X + gk * ld + gc : X), "r"(in ? 4 : 0));
+      }
     }
   };
-  if (kbeg < kend) load(kbeg);
+  auto load = [&](int64_t k0, int buf) {
+    if (k0 < kend) {
+      float* d = df_sm + buf * BUF;
+      tile(std::integral_constant<int, DF_BM>(), A, lda, M, i0, k0, va, d);
+      tile(std::integral_constant<int, BN>(), B, ldb, N, j0, k0, vb, d + DF_BK * DF_BM);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int buf = 0;
+  load(kbeg, 0);
   for (int64_t k0 = kbeg; k0 < kend; k0 += DF_BK) {
-#pragma unroll
-    for (int q = 0; q < LA; ++q) {
-      const int e = threadIdx.x + q * DF_THREADS;
-      As[e / DF_BM][e % DF_BM] = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < LB; ++q) {
-      const int e = threadIdx.x + q * DF_THREADS;
-      Bs[e / DF_BN][e % DF_BN] = rb[q];
-    }
+    load(k0 + DF_BK, buf ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    if (k0 + DF_BK < kend) load(k0 + DF_BK);
+    const float* As = df_sm + buf * BUF + ty * TM;
+    const float* Bs = df_sm + buf * BUF + DF_BK * DF_BM + tx * 4;
     float s[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) s[i][j] = 0.f;
-#pragma unroll 8
+#pragma unroll 4
     for (int kk = 0; kk < DF_BK; ++kk) {
-      const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * TM]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[kk][64 + tx * 4]);
-      const float a[TM] = {av.x, av.y, av.z, av.w};
+      float a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(As + kk * DF_BM + i);
+        a[i] = v.x;
+        a[i + 1] = v.y;
+        a[i + 2] = v.z;
+        a[i + 3] = v.w;
+      }
+      const float4 b0 = *reinterpret_cast<const float4*>(Bs + kk * BN);
+      const float4 b1 = *reinterpret_cast<const float4*>(Bs + kk * BN + HB);
       const float b[TN] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
       for (int i = 0; i < TM; ++i)
@@ -514,6 +538,7 @@ __global__ void __launch_bounds__(DF_THREADS) gemm_tn_df_kernel(const float* __r
         hi[i][j] = t;
       }
     __syncthreads();
+    buf ^= 1;
   }
   double* P = part + (int64_t)blockIdx.y * M * N;
 #pragma unroll
@@ -522,11 +547,15 @@ __global__ void __launch_bounds__(DF_THREADS) gemm_tn_df_kernel(const float* __r
     if (gi >= M) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int64_t gj = j0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
+      const int64_t gj = j0 + (j < 4 ? tx * 4 + j : HB + tx * 4 + (j - 4));
       if (gj < N) P[gi * N + gj] = (double)hi[i][j] + (double)lo[i][j];
     }
   }
 }
+
+// wide tiles for tall operands; the n x n products have too few tiles as it is (301 x 301:
+// 25 us on 128-column tiles, 35 on 256)
+static int df_bn(int64_t N, int64_t K) { return N > 128 && K >= 16384 ? 256 : 128; }
 
 struct DfPlan {
   int64_t tm, tn, kchunk;
@@ -535,7 +564,7 @@ struct DfPlan {
 static DfPlan df_plan(int64_t M, int64_t N, int64_t K) {
   DfPlan p;
   p.tm = cdiv(M, DF_BM);
-  p.tn = cdiv(N, DF_BN);
+  p.tn = cdiv(N, df_bn(N, K));
   int c = tn_chunks(p.tm * p.tn, K, DF_BK, 1);
   int64_t kc = cdiv(std::max<int64_t>(K, 1), c);
   kc = cdiv(kc, DF_BK) * DF_BK;
@@ -558,7 +587,21 @@ int gemm_tn_df(const float* A, int64_t lda, const float* B, int64_t ldb, double*
                  K > 0 ? 2 : 1);
   if (K > 0) {
     dim3 grid((unsigned)(p.tm * p.tn), (unsigned)p.chunks, 1u);
-    gemm_tn_df_kernel<<<grid, DF_THREADS, 0, st>>>(A, lda, B, ldb, part, M, N, K, p.kchunk, p.tm);
+    const auto vec = [](const float* X, int64_t ld) {
+      return (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 ? 1 : 0;
+    };
+    const int bn = df_bn(N, K);
+    const auto kern = bn == 256 ? gemm_tn_df_kernel<8, 32> : gemm_tn_df_kernel<4, 16>;
+    const size_t smem = sizeof(float) * 2 * DF_BK * (DF_BM + bn);
+    static bool attr = false;
+    if (!attr) {
+      PLOM_CHECK_CUDA(cudaFuncSetAttribute(gemm_tn_df_kernel<8, 32>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(sizeof(float) * 2 * DF_BK * (DF_BM + 256))));
+      attr = true;
+    }
+    kern<<<grid, DF_THREADS, smem, st>>>(A, lda, B, ldb, part, M, N, K, p.kchunk, p.tm, vec(A, lda),
+                                         vec(B, ldb));
     PLOM_CHECK_LAUNCH();
   } else {
     PLOM_CHECK_CUDA(cudaMemsetAsync(part, 0, sizeof(double) * M * N, st));
@@ -566,7 +609,7 @@ int gemm_tn_df(const float* A, int64_t lda, const float* B, int64_t ldb, double*
   const int64_t total = M * N;
   const int blocks = (int)std::min<int64_t>(cdiv(total, 256), (int64_t)num_sms() * 16);
   reduce_partials_kernel<double, double><<<blocks, 256, 0, st>>>(part, K > 0 ? p.chunks : 1, M, N,
-                                                                 0, DF_BM, DF_BN, C, ldc, 0, 1);
+                                                                 0, DF_BM, df_bn(N, K), C, ldc, 0, 1);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
 }
