@@ -473,12 +473,21 @@ constexpr uint32_t G_BOX = G_BK * 128;         // G_BK rows x 64 fp16
 constexpr uint32_t G_TILE = 2 * G_BOX;         // G_BK rows x 128 columns of one plane
 constexpr uint32_t G_STAGE = 4 * G_TILE;       // A hi, A lo, B hi, B lo
 constexpr int G_STAGES = (3 * 64) / G_BK;      // 192 KiB of stages
-static_assert(G_BK % 16 == 0 && G_BK >= 16 && G_BK <= 64, "stage rows");
+static_assert(G_BK % 32 == 0 && G_BK >= 32 && G_BK <= 64, "stage rows");
 // Rows accumulated in TMEM (FP32) before the FP64 drain (4,096 rows: 256 UMMA
 // of K = 16 per accumulator).
 constexpr int G_KSUB = PLOM_GRAM_KSUB;
-static_assert(G_KSUB % G_BK == 0, "drain on stage boundaries");
+// The one-tile Gram drains every 1,024 rows: the FP32 accumulators cut their sums off,
+// and the error of the singular values follows the length (SPOD energies, 24 seeds of
+// 389,647 points: 4,096 rows at most 2.2e-6, 1.2e-7 to 3.5e-7 typical; 1,024 rows 2.5e-7
+// and 1.1e-7).  Its double-float sums stay in shared memory (upper 32 x 32 blocks,
+// padded rows), not in the slab: through L2 the drains took a fourth of the time.
+constexpr int G_KSUB_SYM = 1024;
+constexpr int G_STAGES_SYM = (4 * 64) / G_BK;
+constexpr int G_SLAB_BLOCK = 32 * 33;          // double-float values
+static_assert(G_KSUB % G_BK == 0 && G_KSUB_SYM % G_BK == 0, "drain on stage boundaries");
 constexpr size_t G_SMEM = (size_t)G_STAGES * G_STAGE + 1024;
+constexpr size_t G_SMEM_SYM = (size_t)G_STAGES_SYM * (G_STAGE / 2) + 10 * G_SLAB_BLOCK * 8 + 1024;
 constexpr uint32_t G_TMEM = 512;               // 2 buffers x (main 128 + correction 128)
 
 // Double-float (unevaluated sum of two FP32 numbers, ~48 bits) for the Gram's
@@ -513,16 +522,20 @@ __device__ __forceinline__ float2 dw_from_double(double d) {
 }
 __device__ __forceinline__ double dw_value(float2 v) { return (double)v.x + (double)v.y; }
 
-// SYM: upper tiles of A^T A (tmB unused) with the exact diagonal on diagonal
-// tiles; otherwise every tile of A^T B (tna x tnb tiles, B from tmB).  The
-// partial of a work item is 128 x 128 double-float values (8 bytes each).
+// SYM: A^T A of up to 128 columns (tmB unused) with the exact diagonal; otherwise every
+// tile of A^T B (tna x tnb tiles, B from tmB).  The partial of a work item is 128 x 128
+// double-float values (8 bytes each).
 template <bool SYM>
 __global__ void __launch_bounds__(320, 1)
     gram16_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmB,
                   int64_t m, int tn, int tnb, int64_t rows_per_chunk, int chunks,
                   double* __restrict__ part, int* err, int64_t mp) {
+  // SYM: one tile (matrices of up to 128 columns), whose stages hold half as much
+  constexpr int NST = SYM ? G_STAGES_SYM : G_STAGES;
+  constexpr uint32_t STB = SYM ? G_STAGE / 2 : G_STAGE;
+  constexpr bool diag = SYM;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t full_bar[G_STAGES], empty_bar[G_STAGES];
+  __shared__ uint64_t full_bar[NST], empty_bar[NST];
   __shared__ uint64_t tfull[2], tempty[2], dfull[2];
   __shared__ double diag_sh[2][2][128];  // [buffer][row half][column]
   __shared__ uint32_t tmem_sh;
@@ -533,36 +546,24 @@ __global__ void __launch_bounds__(320, 1)
   // resident together read the same rows and share them through L2
   // work item -> (problem of the batch, row chunk, tile); the problems' rows
   // are mp apart in the planes
-  const int ntiles = SYM ? tn * (tn + 1) / 2 : tn * tnb;
+  const int ntiles = SYM ? 1 : tn * tnb;
   const int per_problem = ntiles * chunks;
   const int pb = (int)(blockIdx.x / per_problem);
   const int rem_item = (int)(blockIdx.x % per_problem);
   const int chunk = rem_item / ntiles, tile = rem_item % ntiles;
   const int item = (pb * ntiles + tile) * chunks + chunk;  // partial slab index (tile-major)
-  int ti = 0, tj = 0;
-  if (SYM) {
-    int rem = tile;
-    while (rem >= tn - ti) {
-      rem -= tn - ti;
-      ++ti;
-    }
-    tj = ti + rem;
-  } else {
-    ti = tile / tnb;
-    tj = tile % tnb;
-  }
-  const bool diag = SYM && (ti == tj);
+  const int ti = SYM ? 0 : tile / tnb, tj = SYM ? 0 : tile % tnb;
   const int I0 = ti * 128, J0 = tj * 128;
   const int64_t r_beg = (int64_t)chunk * rows_per_chunk;
   const int64_t r_end = (r_beg + rows_per_chunk < m) ? r_beg + rows_per_chunk : m;
   const int64_t nrows = (r_end > r_beg) ? r_end - r_beg : 0;
   const int KB = (int)((nrows + G_BK - 1) / G_BK);
-  constexpr int KB_PER_SUB = G_KSUB / G_BK;
+  constexpr int KB_PER_SUB = (SYM ? G_KSUB_SYM : G_KSUB) / G_BK;
   const int nsub = (KB + KB_PER_SUB - 1) / KB_PER_SUB;
   if (launch_aborted(err)) return;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < G_STAGES; ++s) {
+    for (int s = 0; s < NST; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], diag ? 1 + 128 : 1);  // MMA commit (+ diagonal warps)
     }
@@ -593,10 +594,10 @@ __global__ void __launch_bounds__(320, 1)
     if (lane == 0) {
       const uint32_t bytes = (diag ? 2u : 4u) * G_TILE;
       for (int kb = 0; kb < KB; ++kb) {
-        const int s = kb % G_STAGES;
-        const uint32_t ph = (uint32_t)(kb / G_STAGES) & 1u;
+        const int s = kb % NST;
+        const uint32_t ph = (uint32_t)(kb / NST) & 1u;
         if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_sh, err)) break;
-        const uint32_t st = base + s * G_STAGE;
+        const uint32_t st = base + s * STB;
         const int y = (int)((int64_t)pb * mp + r_beg + (int64_t)kb * G_BK);
         mbar_expect_tx(&full_bar[s], bytes);
 #pragma unroll
@@ -614,9 +615,10 @@ __global__ void __launch_bounds__(320, 1)
   } else if (warp >= 4 && warp < 8) {
     // ---- diagonal tiles: compensated sums of (hi + lo)^2 per column.  A
     // thread takes two adjacent columns (one 32-bit shared load per plane and
-    // row) over one half of each stage's rows, even and odd rows in separate
-    // chains: four independent compensated chains per thread, so the
-    // diagonal keeps pace with the MMA
+    // row) over one half of each stage's rows.  Four rows are summed by FMAs
+    // (one rounding each, as the compensated addition itself has) and added to
+    // one of two compensated sums: row by row, the chains of 128 threads were a
+    // fifth of the kernel's time
     if (diag) {
       const int t = threadIdx.x - 128;
       const int c = 2 * (t & 63);                // first of the two columns
@@ -624,33 +626,42 @@ __global__ void __launch_bounds__(320, 1)
       const uint32_t cb = (uint32_t)(c >> 6) * G_BOX;
       const uint32_t w = (uint32_t)(c & 63);
       const uint32_t ch = w >> 3, within = (w & 7u) * 2u;
-      const uint32_t k0 = (uint32_t)h * (G_BK / 2), k1 = k0 + G_BK / 2;
-      // chains: [column][row parity]
+      const uint32_t k0 = (uint32_t)h * (G_BK / 2);
+      // chains: [column][parity of the group of four rows]
       float sm[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, cp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
       for (int kb = 0; kb < KB; ++kb) {
-        const int s = kb % G_STAGES;
-        const uint32_t ph = (uint32_t)(kb / G_STAGES) & 1u;
+        const int s = kb % NST;
+        const uint32_t ph = (uint32_t)(kb / NST) & 1u;
         if (!mbar_wait(&full_bar[s], ph, &abort_sh, err)) break;
-        const uint32_t st = base + s * G_STAGE + cb;
-#pragma unroll 4
-        for (uint32_t k = k0; k < k1; k += 2) {
+        const uint32_t st = base + s * STB + cb;
+#pragma unroll 1
+        for (uint32_t kg = 0; kg < (uint32_t)G_BK / 2; kg += 16) {
 #pragma unroll
-          for (uint32_t u = 0; u < 2; ++u) {
-            const uint32_t kk = k + u;
-            const uint32_t off = (kk >> 3) * 1024u + (kk & 7u) * 128u + (((ch ^ (kk & 7u)) << 4) | within);
-            const float2 hv = ld_shared_h2f(st + off);
-            const float2 lv = ld_shared_h2f(st + G_TILE + off);
-            const float v[2] = {hv.x + lv.x, hv.y + lv.y};  // exact: 22 bits
+          for (uint32_t k = 0; k < 16; k += 4) {
+            const uint32_t u = (k >> 2) & 1u;
+            float y[2] = {-cp[0][u], -cp[1][u]};
+#pragma unroll
+            for (uint32_t r = 0; r < 4; ++r) {
+              const uint32_t kk = k0 + kg + k + r;
+              const uint32_t off = (kk >> 3) * 1024u + (kk & 7u) * 128u + (((ch ^ (kk & 7u)) << 4) | within);
+              const float2 hv = ld_shared_h2f(st + off);
+              const float2 lv = ld_shared_h2f(st + G_TILE + off);
+              const float v0 = hv.x + lv.x, v1 = hv.y + lv.y;  // exact: 22 bits
+              y[0] = fmaf(v0, v0, y[0]);
+              y[1] = fmaf(v1, v1, y[1]);
+            }
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
-              const float y = fmaf(v[q], v[q], -cp[q][u]);
-              const float tt = sm[q][u] + y;
-              cp[q][u] = (tt - sm[q][u]) - y;
+              const float tt = sm[q][u] + y[q];
+              cp[q][u] = (tt - sm[q][u]) - y[q];
               sm[q][u] = tt;
             }
           }
         }
-        mbar_arrive(&empty_bar[s]);
+        // the stage is given back once its last values have arrived: the sums (never
+        // negative) depend on them.  In straight-line code the arrival overtook reads
+        // that were still under way.
+        if (!(sm[0][1] + sm[1][1] < 0.f)) mbar_arrive(&empty_bar[s]);
         if ((kb % KB_PER_SUB) == KB_PER_SUB - 1 || kb == KB - 1) {
           const int b = (kb / KB_PER_SUB) & 1;
 #pragma unroll
@@ -679,14 +690,14 @@ __global__ void __launch_bounds__(320, 1)
       const uint32_t dcorr = dmain + 128u;
       const int kb_end = (kb + KB_PER_SUB < KB) ? kb + KB_PER_SUB : KB;
       for (int kl = 0; kb < kb_end; ++kb, ++kl) {
-        const int s = kb % G_STAGES;
-        const uint32_t ph = (uint32_t)(kb / G_STAGES) & 1u;
+        const int s = kb % NST;
+        const uint32_t ph = (uint32_t)(kb / NST) & 1u;
         if (!mbar_wait(&full_bar[s], ph, &abort_sh, err)) {
           ok = false;
           break;
         }
         fence_after();
-        const uint32_t st = base + s * G_STAGE;
+        const uint32_t st = base + s * STB;
         const uint32_t aH = st, aL = st + G_TILE;
         const uint32_t bH = diag ? aH : st + 2 * G_TILE, bL = diag ? aL : st + 3 * G_TILE;
 #pragma unroll
@@ -704,8 +715,12 @@ __global__ void __launch_bounds__(320, 1)
       if (ok) mma_commit(&tfull[b]);
     }
   } else if (warp < 4) {
-    // ---- epilogue: drain each finished sub-chunk into the double-float partial
+    // ---- epilogue: drain each finished sub-chunk into the double-float partial (SYM:
+    // the blocks on and above the diagonal, through shared memory)
     const int rloc = warp * 32 + lane;
+    float2* prow = P + (int64_t)rloc * 128;
+    float2* slab = reinterpret_cast<float2*>(smem_raw + (base - smem_u32(smem_raw)) + NST * STB) +
+                   (warp * 4 - warp * (warp - 1) / 2) * G_SLAB_BLOCK + lane * 33;
     for (int sub = 0; sub < nsub; ++sub) {
       const int b = sub & 1;
       const uint32_t par = ((uint32_t)sub >> 1) & 1u;
@@ -716,22 +731,28 @@ __global__ void __launch_bounds__(320, 1)
       fence_after();
       const float2 dval =
           diag ? dw_from_double(diag_sh[b][0][rloc] + diag_sh[b][1][rloc]) : make_float2(0.f, 0.f);
-      float2* prow = P + (int64_t)rloc * 128;
 #pragma unroll 1
-      for (int cc = 0; cc < 4; ++cc) {
+      for (int cc = SYM ? warp : 0; cc < 4; ++cc) {
         uint32_t rm[32], rc[32];
         const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * 256 + cc * 32);
         tmem_ld32(ta, rm);
         tmem_ld32(ta + 128, rc);
         tmem_wait_ld();
-        float2* d = prow + cc * 32;
+        float2* d = SYM ? slab + (cc - warp) * G_SLAB_BLOCK : prow + cc * 32;
+        if (SYM) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            // main + correction exactly, as a double-float pair
+            float2 v = dw_two_sum(__uint_as_float(rm[j]), __uint_as_float(rc[j]));
+            if (cc * 32 + j == rloc) v = dval;
+            d[j] = sub == 0 ? v : dw_add(d[j], v);
+          }
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-          // main + correction exactly, as a double-float pair
-          float2 v0 = dw_two_sum(__uint_as_float(rm[j]), __uint_as_float(rc[j]));
-          float2 v1 = dw_two_sum(__uint_as_float(rm[j + 1]), __uint_as_float(rc[j + 1]));
-          if (diag && cc * 32 + j == rloc) v0 = dval;
-          if (diag && cc * 32 + j + 1 == rloc) v1 = dval;
+          const float2 v0 = dw_two_sum(__uint_as_float(rm[j]), __uint_as_float(rc[j]));
+          const float2 v1 = dw_two_sum(__uint_as_float(rm[j + 1]), __uint_as_float(rc[j + 1]));
           float4* q = reinterpret_cast<float4*>(d + j);
           if (sub == 0) {
             *q = make_float4(v0.x, v0.y, v1.x, v1.y);
@@ -746,8 +767,15 @@ __global__ void __launch_bounds__(320, 1)
       fence_before();
       mbar_arrive(&tempty[b]);
     }
+    if (SYM && nsub > 0)
+      for (int cc = warp; cc < 4; ++cc) {
+        // rows of a block by the warp, 32 values each
+        const float2* d = slab - lane * 33 + (cc - warp) * G_SLAB_BLOCK;
+        __syncwarp();
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) P[(int64_t)(warp * 32 + r) * 128 + cc * 32 + lane] = d[r * 33 + lane];
+      }
     if (nsub == 0) {  // empty chunk: the partial is zero
-      float2* prow = P + (int64_t)rloc * 128;
       for (int j = 0; j < 128; ++j) prow[j] = make_float2(0.f, 0.f);
     }
   }
@@ -2343,22 +2371,25 @@ static int gram16_chunks(int64_t m, int tiles, int bk = hp::G_BK, int wave_mult 
   return (int)std::max<int64_t>(1, std::min<int64_t>(maxc, cdiv(2 * sms, tiles)));
 }
 
-// row chunks of the narrow kernel (tiles: of all problems): whole waves of
-// CTAs, gram_wave_mult of them while a chunk keeps 16 stages or more, else
-// fewer.  A CTA costs ~5 us besides its stages (barriers, TMEM, the drain of
-// its slab), so 17 problems of 10,006 folded rows in 1,343 chunks of two
-// stages took 135 us, in 136 of twenty 40 us.
+// row chunks of the narrow kernel (tiles: of all problems): the count whose longest SM
+// is done first, a chunk costing its stages and seven more (barriers, TMEM, the first
+// loads, the drain of its slab; four waves of chunks for 1,000,003 x 96 cost 22 us
+// besides one's 106), at least four stages a chunk.  17 problems of 10,006 folded rows in
+// 1,343 chunks of two stages took 135 us, in 136 of twenty 40.
 static int gram16_narrow_chunks(int64_t m, int64_t tiles) {
   const int64_t sms = num_sms();
-  int64_t c = 1;
-  for (int64_t mult = std::max(1, tuning().gram_wave_mult);; mult /= 2) {
-    c = std::max<int64_t>(1, sms * mult / tiles);
-    if (mult <= 1 || m / c >= 16 * hp::G_BK) break;
+  const int64_t maxc = std::min<int64_t>(cdiv(m, 4 * hp::G_BK), std::max<int64_t>(1, 16 * sms / tiles));
+  int64_t best = 0, c = 1;
+  for (int64_t k = 1; k <= maxc; ++k) {
+    const int64_t cost = cdiv(tiles * k, sms) * (cdiv(cdiv(m, k), hp::G_BK) + 7);
+    if (best == 0 || cost < best) {
+      best = cost;
+      c = k;
+    }
   }
-  return (int)std::min<int64_t>(c, std::max<int64_t>(1, cdiv(m, 4 * hp::G_BK)));
+  return (int)c;
 }
 
-// Gram of operands wider than 128 columns: 128 x 256 tiles (gram16w_kernel);
 // row chunks are whole 4,096-row sub-chunks, each with its own FP32 slab.
 // Short chunks keep the tiles of one chunk that run at the same time close
 // together in the rows, so that they share its panels in L2 (the slabs do
@@ -2491,7 +2522,7 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
   if (!attr) {
     PLOM_CHECK_CUDA(cudaFuncSetAttribute(hp::gram16_kernel<true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)hp::G_SMEM));
+                                         (int)hp::G_SMEM_SYM));
     PLOM_CHECK_CUDA(cudaFuncSetAttribute(hp::gram16_kernel<false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)hp::G_SMEM));
@@ -2502,7 +2533,7 @@ int gram_packed(const Packed& p, double* G, int* err, Arena& ws, cudaStream_t st
                                hp::G_BK, (uint64_t)p.pstride),
                PLOM_ERR_CUDA, "gram16: tensor map encoding failed");
   ProfScope prof_g("tc_gram_f16x3", st, (double)p.m * N * N * batch, 4.0 * (double)p.m * p.ld * batch);
-  hp::gram16_kernel<true><<<(unsigned)(batch * tiles * chunks_eff), 320, hp::G_SMEM, st>>>(
+  hp::gram16_kernel<true><<<(unsigned)(batch * tiles * chunks_eff), 320, hp::G_SMEM_SYM, st>>>(
       tm, tm, m, tn, tn, rpc, chunks_eff, part, err, mp);
   PLOM_CHECK_LAUNCH();
   const int blocks = (int)std::min<int64_t>(batch * N * cdiv(N, 32), (int64_t)num_sms() * 4);

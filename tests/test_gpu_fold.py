@@ -96,3 +96,21 @@ def test_column_scales(m, n):
     # 2^-22 of the column's largest element for the operands, the products' sums besides
     tol = 2.0 ** -21 * (np.abs(A64).max(0)[None] @ np.abs(B64)) + 1e-6 * (np.abs(A64) @ np.abs(B64))
     assert np.all(np.abs(C - A64 @ B64) <= tol)
+
+
+@pytest.mark.parametrize("m", [1023, 1024, 1025, 2049, 147344, 300001])
+@pytest.mark.parametrize("n", [40, 64, 96, 128])
+def test_narrow_gram_repeats(m, n):
+    # row counts around the drains (1,024 rows of the folded matrix): the same bits from
+    # every run, and Q orthonormal to its FP32 rounding (2^-23 for a column's norm, the
+    # off-diagonal sums far below)
+    import pyloworder_gb300 as P
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n)
+    A = torch.randn(m, n, generator=g, device="cuda")
+    Q0, R0 = P.math.tsqr(A)
+    G = Q0.double().T @ Q0.double()
+    assert float((G - torch.eye(n, device="cuda", dtype=torch.float64)).abs().max()) < 5e-7
+    for _ in range(12):
+        Q, R = P.math.tsqr(A)
+        assert torch.equal(Q, Q0) and torch.equal(R, R0)
