@@ -1953,7 +1953,7 @@ static int jacobi_launch_cw(const double* A, int n, int batch, JacState& js, dou
                  st, 0.0, 8.0 * 3.0 * n * n * batch * CW);
   if (use_df) {
     const void* k = (const void*)jacobi_block_df16_kernel;
-    PLOM_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PLOM_CHECK_CUDA(allow_smem(k, JAC_BLOCK_SMEM_MAX));
     const int nb = (n + 3) / 4;
     const int nbp = std::max(2, nb + (nb & 1));
     const int want = (int)std::max<int64_t>(1, (int64_t)nbp / 2 * batch);
@@ -1967,7 +1967,7 @@ static int jacobi_launch_cw(const double* A, int n, int batch, JacState& js, dou
   if (smem <= JAC_BLOCK_SMEM_MAX) {
     const void* k = block_df ? (const void*)jacobi_block_kernel<CW, true>
                              : (const void*)jacobi_block_kernel<CW, false>;
-    PLOM_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PLOM_CHECK_CUDA(allow_smem(k, JAC_BLOCK_SMEM_MAX));
     const int nb = (n + 3) / 4;
     const int nbp = std::max(2, nb + (nb & 1));
     const int want = (int)std::max<int64_t>(1, (int64_t)nbp / 2 * batch);
@@ -2598,7 +2598,7 @@ static int jacobi_pre32(const double* A, const double* At, int n, double tol, do
   } else {
     const void* k = (const void*)jacobi_block_f32_kernel;
     const size_t smem = (size_t)4 * J32B * j32.pitch * sizeof(float);
-    PLOM_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PLOM_CHECK_CUDA(allow_smem(k, JAC_BLOCK_SMEM_MAX));
     const int nb = (n + J32B - 1) / J32B;
     const int nbp = std::max(2, nb + (nb & 1));
     const int blocks = coop_blocks(k, 512, smem, nbp / 2);

@@ -39,6 +39,7 @@ namespace plom {
 constexpr int JG_THREADS = 512;
 constexpr int JG_MAX_SWEEPS = 16;
 constexpr int JG_CLUSTER = 16;
+constexpr size_t JG_SMEM_MAX = 160 * 1024, JG_ROWS_SMEM_MAX = 220 * 1024;
 constexpr uint64_t JG_WAIT_NS = 2000000000ull;
 
 struct JgArgs {
@@ -892,9 +893,9 @@ static bool jg_plan(JgPlan& pl, int n) {
   for (pl.R = (int)std::max<int64_t>(1, std::min<int64_t>(8, cdiv(n, num_sms())));; --pl.R) {
     pl.rows_smem = ((size_t)2 * (pl.nblk / 2) * pl.TB * (pl.TB + 4) +
                     (size_t)2 * pl.R * (pl.nblk * (pl.TB / 2) + 10)) * sizeof(float);
-    if (pl.rows_smem <= 220 * 1024 || pl.R == 1) break;
+    if (pl.rows_smem <= JG_ROWS_SMEM_MAX || pl.R == 1) break;
   }
-  return pl.rows_smem <= 220 * 1024;
+  return pl.smem <= JG_SMEM_MAX && pl.rows_smem <= JG_ROWS_SMEM_MAX;
 }
 
 bool jacobi_gram_plan_ok(int n) {
@@ -905,10 +906,8 @@ bool jacobi_gram_plan_ok(int n) {
 bool jacobi_gram_usable(int n) {
   JgPlan pl;
   if (!jg_plan(pl, n)) return false;
-  if (cudaFuncSetAttribute(pl.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(pl.rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)pl.rows_smem) != cudaSuccess) {
+  if (allow_smem(pl.kern, JG_SMEM_MAX) != cudaSuccess ||
+      allow_smem(pl.rows, JG_ROWS_SMEM_MAX) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

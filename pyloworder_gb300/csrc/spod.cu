@@ -23,6 +23,8 @@
 
 namespace plom {
 
+constexpr size_t SPOD_SMEM_MAX = 208 * 1024;  // above every kernel's own bound
+
 template <typename T>
 struct c2 {
   T re, im;
@@ -287,7 +289,7 @@ static int spod_fft_reg_launch(const float* Y, int64_t M, int64_t ldy, const flo
   constexpr int N = P * L;
   const size_t smem = sizeof(float) * 3 * N + sizeof(float2) * (size_t)((nBlks + 1) / 2) * (N + 1);
   const auto kern = spod_fft_reg_kernel<P, L>;
-  PLOM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PLOM_CHECK_CUDA(allow_smem(kern, SPOD_SMEM_MAX));
   int per_sm = 0;
   PLOM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
   const int64_t grid = std::min<int64_t>(M, (int64_t)std::max(1, per_sm) * num_sms() * 8);
@@ -332,8 +334,7 @@ static int spod_fft_impl(const T* Y, int64_t M, int64_t N, int64_t ldy, const T*
   int R = (int)std::min<size_t>(8, (cap - fixed) / per_row);
   R = std::max(1, R);
   const size_t smem = fixed + per_row * R;
-  PLOM_CHECK_CUDA(cudaFuncSetAttribute(spod_fft_kernel<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PLOM_CHECK_CUDA(allow_smem(spod_fft_kernel<T>, SPOD_SMEM_MAX));
   const int64_t grid = cdiv(M, R);
   PLOM_REQUIRE(grid < (1ll << 31), PLOM_ERR_ARG, "spod_fft: too many rows");
   ProfScope prof("spod_fft", st, 5.0 * (double)M * nBlks * nDFT * (log2n > 0 ? log2n : nDFT),
@@ -381,8 +382,7 @@ static int spod_modes_impl(const T* U, int64_t G, int64_t M, int64_t nBlks, int6
                "spod_modes: %lld frequencies x %lld blocks do not fit in shared memory",
                (long long)G, (long long)nBlks);
   if (smem > 48 * 1024)
-    PLOM_CHECK_CUDA(cudaFuncSetAttribute(spod_modes_kernel<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PLOM_CHECK_CUDA(allow_smem(spod_modes_kernel<T>, SPOD_SMEM_MAX));
   const int64_t grid = std::min<int64_t>(M, (int64_t)num_sms() * 8);
   ProfScope prof("spod_modes", st, 0.0, (double)sizeof(T) * 3.0 * G * M * nBlks);
   spod_modes_kernel<T><<<(unsigned)grid, 256, smem, st>>>(U, M, (int)nBlks, (int)G, ustride, P, nf,
@@ -479,8 +479,7 @@ static int spod_assemble_impl(const T* Tg, int64_t rows, int nf, int G, int64_t 
   PLOM_REQUIRE(smem <= 200 * 1024, PLOM_ERR_UNSUPPORTED, "spod_assemble: %d frequencies too many",
                nf);
   if (smem > 48 * 1024)
-    PLOM_CHECK_CUDA(cudaFuncSetAttribute(spod_assemble_kernel<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PLOM_CHECK_CUDA(allow_smem(spod_assemble_kernel<T>, SPOD_SMEM_MAX));
   const int64_t grid = std::min<int64_t>((rows + RB - 1) / RB, (int64_t)num_sms() * 8);
   ProfScope prof("spod_assemble", st, 0.0, 2.0 * sizeof(T) * rows * nf);
   spod_assemble_kernel<T><<<(unsigned)grid, 256, smem, st>>>(Tg, rows, nf, G, gstride, order, P,
@@ -568,8 +567,7 @@ static int spod_gather_impl(const T* U, int64_t M, int nBlks, int nf, int64_t us
   const int BT = (int)std::max<size_t>(1, std::min<size_t>(nBlks, cap / row));
   const int R = BT < nBlks ? 1 : (int)std::max<size_t>(1, std::min<size_t>(4, cap / (row * BT)));
   const size_t smem = ob + 2 * row * R * BT;
-  PLOM_CHECK_CUDA(cudaFuncSetAttribute(spod_gather_kernel<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PLOM_CHECK_CUDA(allow_smem(spod_gather_kernel<T>, SPOD_SMEM_MAX));
   const int64_t gx = std::min<int64_t>(cdiv(M, R), (int64_t)num_sms() * 3);
   ProfScope prof("spod_gather", st, 0.0, 3.0 * sizeof(T) * (double)M * nBlks * nf);
   spod_gather_kernel<T><<<dim3((unsigned)gx, (unsigned)cdiv(nBlks, BT)), 256, smem, st>>>(

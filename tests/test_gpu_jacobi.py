@@ -120,3 +120,40 @@ def test_started_sweeps(n, dt):
     assert np.max(np.abs(V @ V.T - np.eye(n))) < tol
     assert np.linalg.norm((U * S) @ V - A) < tol * np.linalg.norm(A)
     assert np.max(np.abs(S - np.linalg.svd(A, compute_uv=False))) < tol * S[0]
+
+
+def test_sizes_on_several_threads():
+    # kernels whose shared memory follows the size: problems of different sizes from
+    # four threads at once, each against its own result alone
+    import threading
+
+    import pyloworder_gb300 as P
+    sizes = [20, 47, 65, 129, 200, 257, 301, 420, 512, 600]
+    data = {n: torch.from_numpy(field(2 * n + 130, n, 7000 + n).astype(np.float32)).cuda() for n in sizes}
+    alone = {n: P.math.tsqr_svd(data[n])[1].cpu() for n in sizes}
+    spod = torch.randn(300, 700, device="cuda")
+    t = np.arange(700) * 1.0
+    ls = {nd: P.SPOD.run(spod, t, nDFT=nd)[0].cpu() for nd in (32, 64, 128)}
+    errors = []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                rng = np.random.default_rng(k)
+                for _ in range(40):
+                    n = int(rng.choice(sizes))
+                    if not torch.equal(P.math.tsqr_svd(data[n])[1].cpu(), alone[n]):
+                        errors.append(("svd", n))
+                    nd = int(rng.choice([32, 64, 128]))
+                    if not torch.allclose(P.SPOD.run(spod, t, nDFT=nd)[0].cpu(), ls[nd], rtol=1e-5):
+                        errors.append(("spod", nd))
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    torch.cuda.synchronize()
+    th = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for x in th:
+        x.start()
+    for x in th:
+        x.join()
+    assert not errors, errors[:5]
