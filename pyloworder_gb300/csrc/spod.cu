@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) spod_fft_kernel(
 // pair's shared row gives lane l all L values of k1 = l (+ L q), whose L-point DFT
 // is the bins k1 + P k2.  No stage crosses lanes: a 32-point FFT over the lanes by
 // shuffles took 80 shuffles and as many discarded halves of butterflies a pair, and
-// 5.4 ms at 262,144 points x 31 windows of 256 (3.2 ms with this; reading the points
+// 5.4 ms at 262,144 points x 31 windows of 256 (3.9 ms with this; reading the points
 // once and writing the spectra takes 1.9).
 // Two real windows share one complex transform (z = x_a + i x_b;
 // X_a[f] = (Z[f] + conj Z[N-f]) / 2, X_b[f] = (Z[f] - conj Z[N-f]) / 2i).  A CTA owns
