@@ -62,7 +62,9 @@ def _svd_batch(Q, nBlks, precision):
            - L.load().plom_tsqr_svd_batched_workspace(dt, prec, 1, Mrows, nBlks))
     per = max(per, 1) + Q[0].numel() * Q.element_size()
     free = t.cuda.mem_get_info()[0] + t.cuda.memory_reserved() - t.cuda.memory_allocated()
-    return int(max(1, min(nf, SVD_BATCH_MAX, (free // 2) // per)))
+    # (the batched form's tall kernels address all problems' rows with 32 bits)
+    rows = -(-Mrows // 128) * 128
+    return int(max(1, min(nf, SVD_BATCH_MAX, (free // 2) // per, (2 ** 31 - 1) // rows)))
 
 
 def run_device(x, ld, t_host, nDFT=0, nolap=0, remove_mean=True, window="hamming", precision=None):
