@@ -61,10 +61,14 @@ def _svd_batch(Q, nBlks, precision):
     per = (L.load().plom_tsqr_svd_batched_workspace(dt, prec, 2, Mrows, nBlks)
            - L.load().plom_tsqr_svd_batched_workspace(dt, prec, 1, Mrows, nBlks))
     per = max(per, 1) + Q[0].numel() * Q.element_size()
-    free = t.cuda.mem_get_info()[0] + t.cuda.memory_reserved() - t.cuda.memory_allocated()
     # (the batched form's tall kernels address all problems' rows with 32 bits)
-    rows = -(-Mrows // 128) * 128
-    return int(max(1, min(nf, SVD_BATCH_MAX, (free // 2) // per, (2 ** 31 - 1) // rows)))
+    want = max(1, min(nf, SVD_BATCH_MAX, (2 ** 31 - 1) // (-(-Mrows // 128) * 128)))
+    free = t.cuda.mem_get_info()[0]
+    # torch's statistics cost 0.2 ms to gather: only where the driver's free memory
+    # alone does not cover the largest batch
+    if free // 2 < want * per:
+        free += t.cuda.memory_reserved() - t.cuda.memory_allocated()
+    return int(max(1, min(want, (free // 2) // per)))
 
 
 def run_device(x, ld, t_host, nDFT=0, nolap=0, remove_mean=True, window="hamming", precision=None):
