@@ -573,7 +573,8 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
 // double-float arithmetic (R3 R2 R1, R3^-1 Ur); F32 = true: C = A B or Cin - A B
 // with FP32 products (corrections at the 1e-7 level of C).  tri bit 0: A upper
 // triangular, bit 1: B upper triangular (zero blocks are skipped).  D (or null):
-// s is the power of two that brings D's largest diagonal entry next to 1; A is
+// s is the power of two that brings D's largest diagonal entry (or the double in
+// amax, its bits) next to 1; A is
 // scaled by s^ea and B by s^eb, so that factors of data of any FP32 magnitude
 // fit.  An FP64 multiply-add issues at 2 lanes a clock and SM: one 32 x 32 x 32
 // block took 14 us on the FP64 pipe, 3 us in double-float arithmetic.
@@ -597,7 +598,8 @@ __global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __res
                                                              const double* __restrict__ Cin,
                                                              double* __restrict__ C, int n, int tri,
                                                              const double* __restrict__ D, int ea,
-                                                             int eb) {
+                                                             int eb,
+                                                             const unsigned long long* __restrict__ amax) {
   __shared__ __align__(16) float2 As[CB][CPITCH];  // [k][row of A]
   __shared__ __align__(16) float2 Bs[CB][CPITCH];
   __shared__ int ex_sh;
@@ -607,7 +609,11 @@ __global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __res
   B += off;
   C += off;
   const int bi = blockIdx.y, bj = blockIdx.x;
-  const int s = D ? cd_diag_exponent(D + off, n, &ex_sh) : 0;
+  int s = D ? cd_diag_exponent(D + off, n, &ex_sh) : 0;
+  if (amax) {
+    const int e = (int)(*amax >> 52) & 0x7ff;
+    s = (e > 0 && e < 0x7ff) ? 1023 - e : 0;
+  }
   const int T = (n + CB - 1) / CB;
   const int k0 = (tri & 1) ? bi : 0, k1 = (tri & 2) ? bj : T - 1;
   const int c = tid & 31, r = tid >> 5;  // rows r, r + 8, ...
@@ -667,16 +673,16 @@ __global__ void __launch_bounds__(CD_THREADS) gemm_df_kernel(const double* __res
 
 static int gemm_df_launch(bool f32, const double* A, const double* B, const double* Cin, double* C,
                           int n, int batch, int tri, const double* D, int ea, int eb,
-                          cudaStream_t st) {
+                          cudaStream_t st, const unsigned long long* amax = nullptr) {
   if (n <= 0 || batch <= 0) return PLOM_OK;
   PLOM_REQUIRE(A && B && C && batch <= 65535, PLOM_ERR_ARG, "gemm_df: bad arguments");
   ProfScope prof("gemm_df", st, 2.0 * n * n * n * batch, 24.0 * n * n * batch);
   const unsigned T = (unsigned)cdiv(n, CB);
   const dim3 grid(T, T, (unsigned)batch);
   if (f32)
-    gemm_df_kernel<true><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb);
+    gemm_df_kernel<true><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb, amax);
   else
-    gemm_df_kernel<false><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb);
+    gemm_df_kernel<false><<<grid, CD_THREADS, 0, st>>>(A, B, Cin, C, n, tri, D, ea, eb, amax);
   PLOM_CHECK_LAUNCH();
   return PLOM_OK;
 }
@@ -684,6 +690,11 @@ static int gemm_df_launch(bool f32, const double* A, const double* B, const doub
 int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
                cudaStream_t st) {
   return gemm_df_launch(false, A, B, nullptr, C, n, batch, tri, (tri & 2) ? B : nullptr, 0, 1, st);
+}
+
+int gemm_df_nn_scaled(const double* A, const double* B, double* C, int n,
+                      const unsigned long long* amax, cudaStream_t st) {
+  return gemm_df_launch(false, A, B, nullptr, C, n, 1, 0, nullptr, 1, 0, st, amax);
 }
 
 // Re = R3 R2' R1' for at most 64 columns in one launch, one CTA per problem:

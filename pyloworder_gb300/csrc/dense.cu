@@ -2695,7 +2695,7 @@ static int jacobi_start_df(const double* A, const double* At, int n, unsigned lo
   ns_factor_kernel<<<eg, 256, 0, st>>>(G, n);
   PLOM_CHECK_LAUNCH();
   PLOM_TRY(gemm_df_nn(J, G, V, n, 1, 0, st));
-  return gemm_df_nn(At, V, B, n, 1, 0, st);
+  return gemm_df_nn_scaled(At, V, B, n, amax, st);
 }
 
 // V (orthogonal, FP64) and B = At V; J32: n x n FP32 scratch (may be B)

@@ -81,6 +81,9 @@ int chol_inverse_df(const double* G, double* R, double* W, int n, int batch, dou
 // as in gemm_sq.
 int gemm_df_nn(const double* A, const double* B, double* C, int n, int batch, int tri,
                cudaStream_t st);
+// The same for one A of any magnitude, B next to 1; amax: the bits of A's largest |a|.
+int gemm_df_nn_scaled(const double* A, const double* B, double* C, int n,
+                      const unsigned long long* amax, cudaStream_t st);
 // Re = R3 R2' R1' with R' = R - R dW R, the factor of X Q W' = Q for the rounded
 // W' = W + dW that the tall product used in the place of W = R^-1: R' is the
 // inverse of W' up to (dW R)^2.  T1, T2: n x n scratch per problem.

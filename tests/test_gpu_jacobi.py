@@ -157,3 +157,17 @@ def test_sizes_on_several_threads():
     for x in th:
         x.join()
     assert not errors, errors[:5]
+
+
+@pytest.mark.parametrize("n", [20, 45, 64, 130, 224, 256, 300])
+@pytest.mark.parametrize("scale", [1e-32, 1e-30, 1e30, 1e35])
+def test_magnitudes(n, scale):
+    # every product of the SVD stage is scaled: data at both ends of the FP32 range
+    # has the singular values of the same data next to 1
+    import pyloworder_gb300 as P
+    A = field(2 * n + 130, n, 9000 + n).astype(np.float32)
+    U, S, V = (x.cpu().numpy().astype(np.float64) for x in P.math.tsqr_svd(torch.from_numpy(A * np.float32(scale)).cuda()))
+    ex = np.linalg.svd((A * np.float32(scale)).astype(np.float64), compute_uv=False)
+    assert np.max(np.abs(S - ex) / ex) < TOL
+    assert np.max(np.abs(U.T @ U - np.eye(n))) < 2 * TOL
+    assert np.max(np.abs(V @ V.T - np.eye(n))) < TOL
